@@ -9,7 +9,7 @@
 //    (kernel_gen_49_turn_matrices, honest_multistreet_solver.cu:56-86, as
 //    integer counts).  Each (completion, hand) is evaluated ONCE into a
 //    16-bit key; pairs are then counted two completions per 32-bit word with
-//    SIMD half-word compares (__vcmpgtu2 / __vcmpeq2) on shared-memory tiles.
+//    one packed add-and-clamp per count on shared-memory tiles.
 //  * mtt_flop_ev / mtt_ev_dump: the reference dumper (mtt_ev_dumper.cu:85-168)
 //    with the same subsampled runouts, villain stride, ½ tie weight, FMA
 //    accumulation order and host aggregation, reproduced bit-exactly.
@@ -178,8 +178,37 @@ k_enumerate7(unsigned long long* __restrict__ hist, unsigned long long* __restri
 }
 
 // ============================================================ board counts
-// keys[w][h] packs the 16-bit keys of completions 2w (low) and 2w+1 (high)
-// for hand h; 0 marks a completion that uses one of h's cards (or padding).
+// Packed comparisons.  A hero word holds key + 1 of two completions as signed
+// halves, a villain word -key, so their half-wise sum is key_h - key_v + 1 and
+// one saturating __viaddmin_s16x2_relu gives, per half,
+//   clamp(sum, 0, 2) = 2 for a win, 1 for a tie, 0 for a loss   (2W + T summed)
+//   clamp(sum - 1, 0, 1) = 1 for a win                          (W summed).
+// A completion that uses one of the hand's cards (or padding) is KEY_H_DEAD in
+// a hero word and KEY_V_DEAD in a villain word.  Keys are 1..16,972, so a sum
+// with one dead side is below 0 and one with both (-17,001) does not wrap:
+// dead completions count 0.  Two packed compares and their mask, before, were
+// about 30 instructions a word (no half-word compare instruction exists); the
+// clamps are one each, which is what makes the pair counts cheap.
+constexpr uint32_t KEY_H_DEAD = 0xFFFFu;            // -1
+constexpr uint32_t KEY_V_DEAD = 0x10000u - 17000u;  // -17,000
+static_assert(KEY_SFLUSH + 12 + 1 < 17000, "a live key never reaches a dead villain's offset");
+
+__device__ __forceinline__ uint32_t villain_half(uint32_t h) {
+    return h == KEY_H_DEAD ? KEY_V_DEAD : ((1u - h) & 0xFFFFu);
+}
+__device__ __forceinline__ uint32_t villain_word(uint32_t hero) {
+    return villain_half(hero & 0xFFFFu) | (villain_half(hero >> 16) << 16);
+}
+__device__ __forceinline__ uint32_t pair_2w_t(uint32_t hero, uint32_t villain) {
+    return __viaddmin_s16x2_relu(hero, villain, 0x00020002u);
+}
+// hero_m1: the hero word with 1 taken from each half (a dead half becomes -2).
+__device__ __forceinline__ uint32_t pair_w(uint32_t hero_m1, uint32_t villain) {
+    return __viaddmin_s16x2_relu(hero_m1, villain, 0x00010001u);
+}
+
+// keys[w][h] packs the hero halves of completions 2w (low) and 2w+1 (high)
+// for hand h.
 __device__ __forceinline__ void pair_unrank(int k, int n, int& a, int& b) {
     // lexicographic (a<b) over n items
     a = 0;
@@ -204,7 +233,7 @@ __global__ void k_completion_keys(const uint8_t* __restrict__ board, int nboard,
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     const int w = blockIdx.y;
     if (h >= Hp) return;
-    uint32_t word = 0u;
+    uint32_t word = KEY_H_DEAD | (KEY_H_DEAD << 16);
     if (h < H) {
         const int hc1 = hands[2 * h], hc2 = hands[2 * h + 1];
         uint64_t bm = 0;
@@ -231,7 +260,7 @@ __global__ void k_completion_keys(const uint8_t* __restrict__ board, int nboard,
                     planes_add(p, rest[a]); planes_add(p, rest[b]);
                 }
                 if (cm & hm) continue;
-                word |= key_planes(p) << (16 * half);
+                word ^= (KEY_H_DEAD ^ (key_planes(p) + 1u)) << (16 * half);
             }
         }
     }
@@ -240,6 +269,10 @@ __global__ void k_completion_keys(const uint8_t* __restrict__ board, int nboard,
 
 constexpr int BC_TILE = 64, BC_WCHUNK = 32;
 
+// Bound by the packed clamps (4 instructions a word of two completions) and,
+// for few completions, by the three H x H outputs.  Accumulator halves hold at
+// most 2 * 588 (flop boards: 1,176 completions), so plain 32-bit adds do not
+// carry across.
 __global__ void __launch_bounds__(256)
 k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
                const uint8_t* __restrict__ hands, const uint8_t* __restrict__ board, int nboard,
@@ -248,59 +281,72 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
     __shared__ alignas(16) uint32_t vk[BC_WCHUNK][BC_TILE];
     const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
     const int i0 = blockIdx.x * BC_TILE, j0 = blockIdx.y * BC_TILE;
-    uint32_t wc[4][4], tc[4][4];
+    uint32_t wc[4][4], sc[4][4];   // wins; 2 wins + ties
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) { wc[a][b] = 0u; tc[a][b] = 0u; }
+        for (int b = 0; b < 4; ++b) { wc[a][b] = 0u; sc[a][b] = 0u; }
     for (int w0 = 0; w0 < ncw; w0 += BC_WCHUNK) {
-        for (int e = tid; e < BC_WCHUNK * BC_TILE; e += 256) {
-            const int w = e / BC_TILE, x = e % BC_TILE;
-            uint32_t hv = 0u, vv = 0xFFFFFFFFu;
-            if (w0 + w < ncw) {
-                if (i0 + x < Hp) hv = keys[(size_t)(w0 + w) * Hp + i0 + x];
-                if (j0 + x < Hp) { vv = keys[(size_t)(w0 + w) * Hp + j0 + x]; vv |= __vcmpeq2(vv, 0u); }
-            }
-            hk[w][x] = hv;
-            vk[w][x] = vv;
+        const int nw = min(BC_WCHUNK, ncw - w0);
+        for (int e = tid; e < nw * BC_TILE; e += 256) {
+            const int w = e / BC_TILE, x = e % BC_TILE;   // Hp is a multiple of the tile
+            hk[w][x] = keys[(size_t)(w0 + w) * Hp + i0 + x];
+            vk[w][x] = villain_word(keys[(size_t)(w0 + w) * Hp + j0 + x]);
         }
         __syncthreads();
 #pragma unroll 4
-        for (int w = 0; w < BC_WCHUNK; ++w) {
-            const uint4 h4 = *reinterpret_cast<const uint4*>(&hk[w][ti * 4]);
-            const uint4 v4 = *reinterpret_cast<const uint4*>(&vk[w][tj * 4]);
+        for (int w = 0; w < nw; ++w) {
+            const uint4 h4 = *reinterpret_cast<const uint4*>(&hk[w][tj * 4]);
+            const uint4 v4 = *reinterpret_cast<const uint4*>(&vk[w][ti * 4]);
             const uint32_t hv[4] = {h4.x, h4.y, h4.z, h4.w};
             const uint32_t vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a) {
+                const uint32_t hm = hv[a] - 0x00010001u;   // no half is 0, so nothing borrows
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    wc[a][b] += __vcmpgtu2(hv[a], vv[b]) & 0x00010001u;
-                    tc[a][b] += __vcmpeq2(hv[a], vv[b]) & 0x00010001u;
+                    sc[a][b] += pair_2w_t(hv[a], vv[b]);
+                    wc[a][b] += pair_w(hm, vv[b]);
                 }
+            }
         }
         __syncthreads();
     }
+    // a thread's villains are 4 consecutive columns, so with H a multiple of 4
+    // each output row part is one 16-byte store
     uint64_t bm = 0;
     for (int k = 0; k < nboard; ++k) bm |= 1ull << board[k];
+    const int j0t = j0 + ti * 4;
+    uint64_t mj[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int j = min(j0t + b, H - 1);
+        mj[b] = (1ull << hands[2 * j]) | (1ull << hands[2 * j + 1]);
+    }
+    const bool vec = (H & 3) == 0 && j0t + 3 < H &&
+                     ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(T) | reinterpret_cast<uintptr_t>(L)) & 15u) == 0;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const int i = i0 + ti * 4 + a;
+        const int i = i0 + tj * 4 + a;
         if (i >= H) continue;
         const uint64_t mi = (1ull << hands[2 * i]) | (1ull << hands[2 * i + 1]);
+        int32_t wv[4], tv[4], lv[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int j = j0 + tj * 4 + b;
-            if (j >= H) continue;
-            const uint64_t mj = (1ull << hands[2 * j]) | (1ull << hands[2 * j + 1]);
-            int32_t wv = 0, tv = 0, lv = 0;
-            if (!(mi & mj) && !(mi & bm) && !(mj & bm)) {
-                wv = (int32_t)((wc[a][b] & 0xFFFFu) + (wc[a][b] >> 16));
-                tv = (int32_t)((tc[a][b] & 0xFFFFu) + (tc[a][b] >> 16));
-                lv = n_const - wv - tv;
-            }
-            const size_t o = (size_t)i * H + j;
-            W[o] = wv; T[o] = tv; L[o] = lv;
+            const bool ok = !(mi & mj[b]) && !(mi & bm) && !(mj[b] & bm);
+            wv[b] = ok ? (int32_t)((wc[a][b] & 0xFFFFu) + (wc[a][b] >> 16)) : 0;
+            tv[b] = ok ? (int32_t)((sc[a][b] & 0xFFFFu) + (sc[a][b] >> 16)) - 2 * wv[b] : 0;
+            lv[b] = ok ? n_const - wv[b] - tv[b] : 0;
+        }
+        const size_t o = (size_t)i * H + j0t;
+        if (vec) {
+            *reinterpret_cast<int4*>(W + o) = make_int4(wv[0], wv[1], wv[2], wv[3]);
+            *reinterpret_cast<int4*>(T + o) = make_int4(tv[0], tv[1], tv[2], tv[3]);
+            *reinterpret_cast<int4*>(L + o) = make_int4(lv[0], lv[1], lv[2], lv[3]);
+        } else {
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (j0t + b < H) { W[o + b] = wv[b]; T[o + b] = tv[b]; L[o + b] = lv[b]; }
         }
     }
 }
@@ -309,7 +355,7 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
 // Runout subsample of the reference loop (mtt_ev_dumper.cu:98-103): turn
 // index r1 = 0,2,..,46 into the 49-card deck, river index r2 = r1+1, r1+4,
 // .. < 47.  192 (r1, r2) pairs, packed two per key word.
-constexpr int FE_RUNOUTS = 192, FE_WORDS = 96, FE_ALIVE = 1176, FE_VILL = 294, FE_VMASK = 6;
+constexpr int FE_RUNOUTS = 192, FE_WORDS = 96, FE_ALIVE = 1176, FE_VILL = 294;
 __constant__ uint8_t c_runout_r1[FE_RUNOUTS];
 __constant__ uint8_t c_runout_r2[FE_RUNOUTS];
 
@@ -325,9 +371,9 @@ __device__ __forceinline__ void flop_deck(const uint8_t* f, uint8_t* deck) {
     for (int c = 0; c < 52; ++c) if (!((fm >> c) & 1ull)) deck[n++] = (uint8_t)c;
 }
 
-// keys[f][w][i] (hand-minor) and validity bits vmask[f][i][6] (bit k = runout k usable by hand i)
+// keys[f][w][i] (hand-minor): hero halves of runouts 2w and 2w + 1 for hand i
 __global__ void __launch_bounds__(128)
-k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys, uint32_t* __restrict__ vmask) {
+k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys) {
     __shared__ uint8_t deck[52];
     const int f = blockIdx.y;
     const uint8_t* fl = flops + 3 * f;
@@ -342,9 +388,8 @@ k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys, uint
     planes_add(base, fl[0]); planes_add(base, fl[1]); planes_add(base, fl[2]);
     planes_add(base, hc1); planes_add(base, hc2);
     uint32_t* kout = keys + (size_t)f * FE_WORDS * FE_ALIVE + i;
-    uint32_t vm[FE_VMASK] = {0u, 0u, 0u, 0u, 0u, 0u};
     for (int w = 0; w < FE_WORDS; ++w) {
-        uint32_t word = 0u;
+        uint32_t word = KEY_H_DEAD | (KEY_H_DEAD << 16);
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int k = 2 * w + half;
@@ -352,91 +397,101 @@ k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys, uint
             if (t == hc1 || t == hc2 || r == hc1 || r == hc2) continue;
             Planes p = base;
             planes_add(p, t); planes_add(p, r);
-            word |= key_planes(p) << (16 * half);
-            vm[k >> 5] |= 1u << (k & 31);
+            word ^= (KEY_H_DEAD ^ (key_planes(p) + 1u)) << (16 * half);
         }
         kout[(size_t)w * FE_ALIVE] = word;
     }
-    uint32_t* vo = vmask + ((size_t)f * FE_ALIVE + i) * FE_VMASK;
-#pragma unroll
-    for (int q = 0; q < FE_VMASK; ++q) vo[q] = vm[q];
 }
 
 // eqT[f][m][i]: equity of hero i vs villain j = 4m over the usable runouts
 // ((2W+T)/(2N) as in mtt_ev_dumper.cu:105-110), -1 when the pair is skipped.
+// The numerator is the sum of one packed clamp per word; N is counted from the
+// hands' deck positions by inclusion and exclusion over the runout pairs (192
+// less the runouts that hold a card of either hand), so the loop spends
+// nothing on it.  Bound by the clamps and their adds: all 1,755 flops took
+// 48.8 ms with half-word compares and a popcount of usable runouts per pair.
 constexpr int FE_TH = 64, FE_TV = 64, FE_WCH = 32;
 __global__ void __launch_bounds__(256)
-k_flop_pair_eq(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vmask,
-               const uint8_t* __restrict__ flops, float* __restrict__ eqT) {
+k_flop_pair_eq(const uint32_t* __restrict__ keys, float* __restrict__ eqT) {
     __shared__ alignas(16) uint32_t hk[FE_WCH][FE_TH];
     __shared__ alignas(16) uint32_t vk[FE_WCH][FE_TV];
-    __shared__ uint8_t deck[52];
+    __shared__ uint64_t adj[49];             // bit y of adj[x]: deck positions x and y are a runout
+    __shared__ uint8_t pos[2][FE_TH][2];     // deck positions of the tile's heroes and villains
+    __shared__ uint8_t usable[2][FE_TH];     // runouts that avoid each hand's two cards
     const int f = blockIdx.z;
     const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
     const int i0 = blockIdx.x * FE_TH, m0 = blockIdx.y * FE_TV;
-    if (tid == 0) flop_deck(flops + 3 * f, deck);
+    if (tid < 49) {
+        uint64_t m = 0;
+        for (int y = 0; y < 49; ++y) {
+            const int lo = min(tid, y), hi = max(tid, y);
+            if (lo != hi && !(lo & 1) && hi < 47 && (hi - lo - 1) % 3 == 0) m |= 1ull << y;
+        }
+        adj[tid] = m;
+    }
+    __syncthreads();
+    if (tid < 2 * FE_TH) {
+        const int side = tid / FE_TH, x = tid % FE_TH;
+        const int hand = side ? min(4 * (m0 + x), FE_ALIVE - 1) : min(i0 + x, FE_ALIVE - 1);
+        int a, b;
+        pair_unrank(hand, 49, a, b);
+        pos[side][x][0] = (uint8_t)a;
+        pos[side][x][1] = (uint8_t)b;
+        usable[side][x] = (uint8_t)(FE_RUNOUTS - __popcll(adj[a]) - __popcll(adj[b]) + (int)((adj[a] >> b) & 1ull));
+    }
     const uint32_t* kf = keys + (size_t)f * FE_WORDS * FE_ALIVE;
-    uint32_t wc[4][4], tc[4][4];
+    uint32_t sc[4][4];   // 2 wins + ties of each half, at most 2 * 96
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) { wc[a][b] = 0u; tc[a][b] = 0u; }
+        for (int b = 0; b < 4; ++b) sc[a][b] = 0u;
     for (int w0 = 0; w0 < FE_WORDS; w0 += FE_WCH) {
         for (int e = tid; e < FE_WCH * FE_TH; e += 256) {
             const int w = e / FE_TH, x = e % FE_TH;
-            const int i = i0 + x, m = m0 + x;
-            hk[w][x] = (i < FE_ALIVE) ? kf[(size_t)(w0 + w) * FE_ALIVE + i] : 0u;
-            uint32_t vv = 0xFFFFFFFFu;
-            if (m < FE_VILL) { vv = kf[(size_t)(w0 + w) * FE_ALIVE + 4 * m]; vv |= __vcmpeq2(vv, 0u); }
-            vk[w][x] = vv;
+            const int i = min(i0 + x, FE_ALIVE - 1), m = min(m0 + x, FE_VILL - 1);
+            hk[w][x] = kf[(size_t)(w0 + w) * FE_ALIVE + i];
+            vk[w][x] = villain_word(kf[(size_t)(w0 + w) * FE_ALIVE + 4 * m]);
         }
         __syncthreads();
 #pragma unroll 4
-        for (int w = 0; w < FE_WCH; ++w) {
+        for (int w = 0; w < FE_WCH; w += 2) {   // two words a step: their adds fuse into one
             const uint4 h4 = *reinterpret_cast<const uint4*>(&hk[w][ti * 4]);
             const uint4 v4 = *reinterpret_cast<const uint4*>(&vk[w][tj * 4]);
-            const uint32_t hv[4] = {h4.x, h4.y, h4.z, h4.w};
-            const uint32_t vv[4] = {v4.x, v4.y, v4.z, v4.w};
+            const uint4 g4 = *reinterpret_cast<const uint4*>(&hk[w + 1][ti * 4]);
+            const uint4 u4 = *reinterpret_cast<const uint4*>(&vk[w + 1][tj * 4]);
+            const uint32_t hv[4] = {h4.x, h4.y, h4.z, h4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+            const uint32_t gv[4] = {g4.x, g4.y, g4.z, g4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    wc[a][b] += __vcmpgtu2(hv[a], vv[b]) & 0x00010001u;
-                    tc[a][b] += __vcmpeq2(hv[a], vv[b]) & 0x00010001u;
-                }
+                for (int b = 0; b < 4; ++b) sc[a][b] += pair_2w_t(hv[a], vv[b]) + pair_2w_t(gv[a], uv[b]);
         }
         __syncthreads();
     }
-    const uint32_t* vmf = vmask + (size_t)f * FE_ALIVE * FE_VMASK;
+    const int i = i0 + ti * 4;   // FE_ALIVE is a multiple of 4
+    if (i >= FE_ALIVE) return;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int i = i0 + ti * 4 + a;
-        if (i >= FE_ALIVE) continue;
-        int ia, ib;
-        pair_unrank(i, 49, ia, ib);
-        const uint64_t mi = (1ull << deck[ia]) | (1ull << deck[ib]);
+    for (int b = 0; b < 4; ++b) {
+        const int m = m0 + tj * 4 + b;
+        if (m >= FE_VILL) continue;
+        const int x = pos[1][tj * 4 + b][0], y = pos[1][tj * 4 + b][1];
+        float eq[4];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int m = m0 + tj * 4 + b;
-            if (m >= FE_VILL) continue;
-            const int j = 4 * m;
-            int ja, jb;
-            pair_unrank(j, 49, ja, jb);
-            const uint64_t mj = (1ull << deck[ja]) | (1ull << deck[jb]);
-            float eq = -1.0f;
-            if (!(mi & mj)) {
-                int n = 0;
-#pragma unroll
-                for (int q = 0; q < FE_VMASK; ++q)
-                    n += __popc(vmf[(size_t)i * FE_VMASK + q] & vmf[(size_t)j * FE_VMASK + q]);
+        for (int a = 0; a < 4; ++a) {
+            const int c = pos[0][ti * 4 + a][0], d = pos[0][ti * 4 + a][1];
+            eq[a] = -1.0f;
+            if (c != x && c != y && d != x && d != y) {
+                const uint64_t ac = adj[c], ad = adj[d];
+                const int shared = (int)((ac >> x) & 1ull) + (int)((ac >> y) & 1ull) + (int)((ad >> x) & 1ull) +
+                                   (int)((ad >> y) & 1ull);
+                const int n = (int)usable[0][ti * 4 + a] + (int)usable[1][tj * 4 + b] - FE_RUNOUTS + shared;
                 if (n > 0) {
-                    const int wins = 2 * (int)((wc[a][b] & 0xFFFFu) + (wc[a][b] >> 16));
-                    const int ties = (int)((tc[a][b] & 0xFFFFu) + (tc[a][b] >> 16));
-                    eq = __fdiv_rn((float)(wins + ties), (float)(2 * n));
+                    const int num = (int)((sc[a][b] & 0xFFFFu) + (sc[a][b] >> 16));
+                    eq[a] = __fdiv_rn((float)num, (float)(2 * n));
                 }
             }
-            eqT[((size_t)f * FE_VILL + m) * FE_ALIVE + i] = eq;
         }
+        *reinterpret_cast<float4*>(eqT + ((size_t)f * FE_VILL + m) * FE_ALIVE + i) = make_float4(eq[0], eq[1], eq[2], eq[3]);
     }
 }
 
@@ -509,29 +564,27 @@ static int upload_runouts(cudaStream_t st) {
     return MTT_OK;
 }
 
-constexpr int FE_BATCH = 256;   // flops per scratch batch (~470 MB of scratch)
+constexpr int FE_BATCH = 64;    // flops per scratch batch: keys and equities (117 MB) stay in the 126 MB L2
 
 static int flop_ev_batched(const uint8_t* d_flops, int nflops, const float* d_reach0,
                            const float* d_reach1, float* d_ev0, float* d_ev1, cudaStream_t st) {
     MTT_TRY(upload_runouts(st));
     const int nb = nflops < FE_BATCH ? nflops : FE_BATCH;
-    uint32_t *keys = nullptr, *vm = nullptr;
+    uint32_t* keys = nullptr;
     float* eqT = nullptr;
     MTT_TRY_CUDA(cudaMallocAsync(&keys, (size_t)nb * FE_WORDS * FE_ALIVE * 4, st));
-    int s = cuda_status(cudaMallocAsync(&vm, (size_t)nb * FE_ALIVE * FE_VMASK * 4, st));
-    if (s == MTT_OK) s = cuda_status(cudaMallocAsync(&eqT, (size_t)nb * FE_VILL * FE_ALIVE * 4, st));
+    int s = cuda_status(cudaMallocAsync(&eqT, (size_t)nb * FE_VILL * FE_ALIVE * 4, st));
     for (int f0 = 0; s == MTT_OK && f0 < nflops; f0 += nb) {
         const int n = (nflops - f0) < nb ? (nflops - f0) : nb;
         const uint8_t* fl = d_flops + 3 * (size_t)f0;
-        k_flop_keys<<<dim3(ceil_div(FE_ALIVE, 128), n), 128, 0, st>>>(fl, keys, vm);
+        k_flop_keys<<<dim3(ceil_div(FE_ALIVE, 128), n), 128, 0, st>>>(fl, keys);
         k_flop_pair_eq<<<dim3(ceil_div(FE_ALIVE, FE_TH), ceil_div(FE_VILL, FE_TV), n), 256, 0, st>>>(
-            keys, vm, fl, eqT);
+            keys, eqT);
         k_flop_accumulate<<<dim3(ceil_div(FE_ALIVE, 128), n), 128, 0, st>>>(
             eqT, d_reach0, d_reach1, n, d_ev0 + (size_t)f0 * FE_ALIVE, d_ev1 + (size_t)f0 * FE_ALIVE);
         s = cuda_status(cudaGetLastError());
     }
     if (eqT) cudaFreeAsync(eqT, st);
-    if (vm) cudaFreeAsync(vm, st);
     cudaFreeAsync(keys, st);
     return s;
 }
