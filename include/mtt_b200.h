@@ -316,8 +316,10 @@ int mtt_batch_check(mtt_batch* b, void* stream);
 int mtt_batch_launch_count(mtt_batch* b, int64_t* launches);
 /* Batches allocate device memory from a library-owned stream-ordered pool
  * per device that keeps what destroyed batches free, so the next batch of a
- * similar size allocates without mapping new pages.  mtt_trim_pool waits for
- * the current device and returns the kept memory to the driver. */
+ * similar size allocates without mapping new pages.  Calls that need scratch
+ * take it from a second such pool, which keeps at most 256 MB between calls.
+ * mtt_trim_pool waits for the current device and returns the kept memory of
+ * both to the driver. */
 int mtt_trim_pool(void);
 /* Depth-limit leaves (MTT_NODE_LEAF, turn subgames): every pass of every
  * iteration values them by the leaf network `net` (whose batch capacity must

@@ -13,7 +13,6 @@
 //  * mtt_flop_ev / mtt_ev_dump: the reference dumper (mtt_ev_dumper.cu:85-168)
 //    with the same subsampled runouts, villain stride, ½ tie weight, FMA
 //    accumulation order and host aggregation, reproduced bit-exactly.
-#include <cuda.h>   // CUcontext / CUresult types only: the driver entry points are resolved at run time
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -572,8 +571,8 @@ static int flop_ev_batched(const uint8_t* d_flops, int nflops, const float* d_re
     const int nb = nflops < FE_BATCH ? nflops : FE_BATCH;
     uint32_t* keys = nullptr;
     float* eqT = nullptr;
-    MTT_TRY_CUDA(cudaMallocAsync(&keys, (size_t)nb * FE_WORDS * FE_ALIVE * 4, st));
-    int s = cuda_status(cudaMallocAsync(&eqT, (size_t)nb * FE_VILL * FE_ALIVE * 4, st));
+    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&keys), (size_t)nb * FE_WORDS * FE_ALIVE * 4, st));
+    int s = scratch_alloc(reinterpret_cast<void**>(&eqT), (size_t)nb * FE_VILL * FE_ALIVE * 4, st);
     for (int f0 = 0; s == MTT_OK && f0 < nflops; f0 += nb) {
         const int n = (nflops - f0) < nb ? (nflops - f0) : nb;
         const uint8_t* fl = d_flops + 3 * (size_t)f0;
@@ -605,7 +604,7 @@ extern "C" int mtt_eval7(const uint8_t* d_cards7, uint32_t* d_out, int64_t n, vo
         MTT_TRY(sm_count(&sms));
         long long grid = (long long)sms * 4;
         if (grid > n_tiles) grid = n_tiles;
-        MTT_TRY_CUDA(cudaMallocAsync(&d_err, sizeof(int), st));
+        MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&d_err), sizeof(int), st));
         MTT_TRY_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
         k_eval7_bulk<<<(unsigned)grid, EV_THREADS, 0, st>>>(d_cards7, d_out, n_tiles, d_err);
         MTT_CHECK_LAUNCH();
@@ -658,7 +657,7 @@ extern "C" int mtt_board_showdown_counts(const uint8_t* d_board, int32_t nboard,
     const int free_cards = nrest - 4;
     const int n_const = nboard == 5 ? 1 : nboard == 4 ? free_cards : free_cards * (free_cards - 1) / 2;
     uint32_t* keys = nullptr;
-    MTT_TRY_CUDA(cudaMallocAsync(&keys, (size_t)ncw * Hp * sizeof(uint32_t), st));
+    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&keys), (size_t)ncw * Hp * sizeof(uint32_t), st));
     k_completion_keys<<<dim3(Hp / 64, ncw), 64, 0, st>>>(d_board, nboard, d_hands, H, Hp, ncomp, keys);
     int s = cuda_status(cudaGetLastError());
     if (s == MTT_OK) {
@@ -680,34 +679,6 @@ constexpr int kMaxDevices = 64;
 static std::mutex g_counts_scratch_mu;
 static uint32_t* g_counts_scratch_ptr[kMaxDevices] = {};
 static unsigned long long g_counts_scratch_ctx[kMaxDevices] = {};
-
-// Unique id of the calling thread's current context (0 if none or if the
-// driver does not offer the query).  Ids are never reused within a process,
-// so a context created after a cudaDeviceReset always has a new one.  The two
-// driver functions are resolved at run time, so the library does not link the
-// driver and still loads on machines without one.
-static unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        f = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-    });
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (get_current && get_id && get_current(&c) == CUDA_SUCCESS && c && get_id(c, &id) == CUDA_SUCCESS) return id;
-    return 0;
-}
 
 // Address of this device's scratch in the current context.  It is looked up
 // with the device current on the first call in each context (the first call
@@ -800,8 +771,8 @@ extern "C" int mtt_ev_dump(const uint8_t* d_flops, int32_t nflops, float* d_out,
     if (!d_flops || !d_out) return MTT_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
     float *ev0 = nullptr, *ev1 = nullptr;
-    MTT_TRY_CUDA(cudaMallocAsync(&ev0, (size_t)nflops * FE_ALIVE * 4, st));
-    int s = cuda_status(cudaMallocAsync(&ev1, (size_t)nflops * FE_ALIVE * 4, st));
+    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&ev0), (size_t)nflops * FE_ALIVE * 4, st));
+    int s = scratch_alloc(reinterpret_cast<void**>(&ev1), (size_t)nflops * FE_ALIVE * 4, st);
     if (s == MTT_OK) s = flop_ev_batched(d_flops, nflops, nullptr, nullptr, ev0, ev1, st);
     if (s == MTT_OK) {
         const int total = nflops * 1352;

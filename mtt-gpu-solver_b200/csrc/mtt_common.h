@@ -16,6 +16,20 @@ inline int cuda_status(cudaError_t e) {
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Scratch of one call, allocated and freed in stream order (cudaFreeAsync).
+// It comes from a library-owned pool per device that keeps up to
+// SCRATCH_KEEP bytes between calls (mtt_trim_pool gives them back): the
+// device's default pool returns its memory to the driver at the next
+// synchronisation, and mapping it again cost 0.4 ms to several ms a call.
+// While the stream is being captured the allocation is a plain graph node.
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+template <typename T>
+inline int scratch_alloc(T** p, size_t count, cudaStream_t st) {
+    return scratch_alloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T), st);
+}
+unsigned long long current_context_id();
+int scratch_trim();   // returns what the current device's scratch pool keeps; the caller has synchronised
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 

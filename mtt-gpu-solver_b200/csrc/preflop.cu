@@ -371,12 +371,12 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
     uint16_t* d_KT = nullptr;
     float* d_E = nullptr;
     int s = MTT_OK;
-    if (!s) s = cuda_status(cudaMallocAsync(&d_cc, sizeof(uint16_t) * L.cc.size(), st));
-    if (!s) s = cuda_status(cudaMallocAsync(&d_cidx, sizeof(int) * L.cidx.size(), st));
-    if (!s) s = cuda_status(cudaMallocAsync(&d_lists, sizeof(int) * L.lists.size(), st));
-    if (!s) s = cuda_status(cudaMallocAsync(&d_counts, sizeof(int) * L.counts.size(), st));
-    if (!s) s = cuda_status(cudaMallocAsync(&d_KT, sizeof(uint16_t) * (size_t)CHUNK * NPAIR * ld, st));
-    if (!s) s = cuda_status(cudaMallocAsync(&d_E, sizeof(float) * (size_t)CHUNK * ld * ld, st));
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_cc), sizeof(uint16_t) * L.cc.size(), st);
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_cidx), sizeof(int) * L.cidx.size(), st);
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_lists), sizeof(int) * L.lists.size(), st);
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_counts), sizeof(int) * L.counts.size(), st);
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_KT), sizeof(uint16_t) * (size_t)CHUNK * NPAIR * ld, st);
+    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_E), sizeof(float) * (size_t)CHUNK * ld * ld, st);
     if (!s) s = cuda_status(cudaMemcpyAsync(d_cc, L.cc.data(), sizeof(uint16_t) * L.cc.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_cidx, L.cidx.data(), sizeof(int) * L.cidx.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_lists, L.lists.data(), sizeof(int) * L.lists.size(), cudaMemcpyHostToDevice, st));
@@ -631,8 +631,8 @@ extern "C" int mtt_pf_dcfr(const float* d_flop_weights, const float* d_class_mat
     float* buf = nullptr;
     int* d_iter = nullptr;
     const size_t nbuf = 2 * (size_t)iters + 4 * (size_t)STATE + 5 * (size_t)PAD;
-    MTT_TRY_CUDA(cudaMallocAsync(&buf, sizeof(float) * nbuf, st));
-    int s = cuda_status(cudaMallocAsync(&d_iter, sizeof(int), st));
+    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&buf), sizeof(float) * nbuf, st));
+    int s = scratch_alloc(reinterpret_cast<void**>(&d_iter), sizeof(int), st);
     PfDev d{};
     d.fw = d_flop_weights; d.mats = d_class_mats; d.allin = d_allin;
     d.tab = buf;

@@ -2778,7 +2778,7 @@ extern "C" int mtt_trim_pool(void) {
     if (!pool) return MTT_ERR_CUDA;
     MTT_TRY_CUDA(cudaDeviceSynchronize());
     MTT_TRY_CUDA(cudaMemPoolTrimTo(pool, 0));
-    return MTT_OK;
+    return mtt::scratch_trim();
 }
 
 extern "C" int mtt_batch_set_leafnet(mtt_batch* b, mtt_leafnet* net, int32_t flags) {

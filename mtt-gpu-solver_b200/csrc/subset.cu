@@ -619,7 +619,7 @@ extern "C" int mtt_subset_nnomp(const float* d_cols, int32_t ncols, int32_t nfea
     const size_t ni = (size_t)d.ncorr + (size_t)nselect + 4;
     const size_t bytes = sizeof(double) * nd + sizeof(int) * ni + (size_t)ncols;
     unsigned char* ws = nullptr;
-    MTT_TRY_CUDA(cudaMallocAsync(&ws, bytes, st));
+    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&ws), bytes, st));
     double* p = reinterpret_cast<double*>(ws);
     d.b = p; p += nfeat;
     d.r = p; p += nfeat;
