@@ -21,6 +21,7 @@
 #include "mtt_bulk.cuh"
 #include "mtt_common.h"
 #include "mtt_device.cuh"
+#include "mtt_pairs.cuh"
 
 namespace mtt {
 
@@ -177,35 +178,6 @@ k_enumerate7(unsigned long long* __restrict__ hist, unsigned long long* __restri
 }
 
 // ============================================================ board counts
-// Packed comparisons.  A hero word holds key + 1 of two completions as signed
-// halves, a villain word -key, so their half-wise sum is key_h - key_v + 1 and
-// one saturating __viaddmin_s16x2_relu gives, per half,
-//   clamp(sum, 0, 2) = 2 for a win, 1 for a tie, 0 for a loss   (2W + T summed)
-//   clamp(sum - 1, 0, 1) = 1 for a win                          (W summed).
-// A completion that uses one of the hand's cards (or padding) is KEY_H_DEAD in
-// a hero word and KEY_V_DEAD in a villain word.  Keys are 1..16,972, so a sum
-// with one dead side is below 0 and one with both (-17,001) does not wrap:
-// dead completions count 0.  Two packed compares and their mask, before, were
-// about 30 instructions a word (no half-word compare instruction exists); the
-// clamps are one each, which is what makes the pair counts cheap.
-constexpr uint32_t KEY_H_DEAD = 0xFFFFu;            // -1
-constexpr uint32_t KEY_V_DEAD = 0x10000u - 17000u;  // -17,000
-static_assert(KEY_SFLUSH + 12 + 1 < 17000, "a live key never reaches a dead villain's offset");
-
-__device__ __forceinline__ uint32_t villain_half(uint32_t h) {
-    return h == KEY_H_DEAD ? KEY_V_DEAD : ((1u - h) & 0xFFFFu);
-}
-__device__ __forceinline__ uint32_t villain_word(uint32_t hero) {
-    return villain_half(hero & 0xFFFFu) | (villain_half(hero >> 16) << 16);
-}
-__device__ __forceinline__ uint32_t pair_2w_t(uint32_t hero, uint32_t villain) {
-    return __viaddmin_s16x2_relu(hero, villain, 0x00020002u);
-}
-// hero_m1: the hero word with 1 taken from each half (a dead half becomes -2).
-__device__ __forceinline__ uint32_t pair_w(uint32_t hero_m1, uint32_t villain) {
-    return __viaddmin_s16x2_relu(hero_m1, villain, 0x00010001u);
-}
-
 // keys[w][h] packs the hero halves of completions 2w (low) and 2w+1 (high)
 // for hand h.
 __device__ __forceinline__ void pair_unrank(int k, int n, int& a, int& b) {
@@ -280,7 +252,7 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
     __shared__ alignas(16) uint32_t vk[BC_WCHUNK][BC_TILE];
     const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
     const int i0 = blockIdx.x * BC_TILE, j0 = blockIdx.y * BC_TILE;
-    uint32_t wc[4][4], sc[4][4];   // wins; 2 wins + ties
+    uint32_t wc[4][4], sc[4][4];   // 2 wins; 2 wins + ties
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -300,14 +272,13 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
             const uint32_t hv[4] = {h4.x, h4.y, h4.z, h4.w};
             const uint32_t vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const uint32_t hm = hv[a] - 0x00010001u;   // no half is 0, so nothing borrows
+            for (int a = 0; a < 4; ++a)
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    sc[a][b] += pair_2w_t(hv[a], vv[b]);
-                    wc[a][b] += pair_w(hm, vv[b]);
+                    const uint32_t t = pair_2w_t(hv[a], vv[b]);
+                    sc[a][b] += t;
+                    wc[a][b] += t & 0x00020002u;
                 }
-            }
         }
         __syncthreads();
     }
@@ -333,7 +304,7 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const bool ok = !(mi & mj[b]) && !(mi & bm) && !(mj[b] & bm);
-            wv[b] = ok ? (int32_t)((wc[a][b] & 0xFFFFu) + (wc[a][b] >> 16)) : 0;
+            wv[b] = ok ? (int32_t)((wc[a][b] & 0xFFFFu) + (wc[a][b] >> 16)) / 2 : 0;
             tv[b] = ok ? (int32_t)((sc[a][b] & 0xFFFFu) + (sc[a][b] >> 16)) - 2 * wv[b] : 0;
             lv[b] = ok ? n_const - wv[b] - tv[b] : 0;
         }

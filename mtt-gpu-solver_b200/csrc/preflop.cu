@@ -16,19 +16,22 @@
 //
 // Flop matrices: per flop, every combo's 16-bit score key for every
 // (turn, river) pair of the 49-card deck is evaluated once into a
-// pair-major table; a CTA per hero combo then walks the hero's runout list
-// (the reference's subsample: turn index r1 = 0, 2, .. and river r2 = r1+1,
-// r1+4, .. into the hero's 47-card deck) comparing keys against every
-// villain, with coalesced loads of the table.  The combo matrix is reduced
-// to classes in the reference's summation order.
+// pair-major table, and each hero's list of runouts (the reference's
+// subsample: turn index r1 = 0, 2, .. and river r2 = r1+1, r1+4, .. into the
+// hero's 47-card deck) into (pair, key) words.  A CTA then holds 64 villains'
+// part of the table in shared memory and its warps walk the heroes' lists,
+// two villains per 32-bit word and lane.  The combo matrix is reduced to
+// classes in the reference's summation order.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <vector>
 
+#include "mtt_bulk.cuh"
 #include "mtt_common.h"
 #include "mtt_device.cuh"
+#include "mtt_pairs.cuh"
 
 namespace mtt {
 namespace pf {
@@ -95,36 +98,39 @@ __host__ __device__ inline int combo_class(int c1, int c2) {
     return base + (hi - 1 - lo);
 }
 
-// Reference score of 7 cards that may repeat: rank counts are exact (a rank
-// seen 5+ times is neither quads, trips nor a pair, as with the reference's
-// rc[r] == 4 / 3 / 2 tests) and a suit flushes on its card count (sc[s] >= 5)
-// with the ranks it holds (sm[s]), as the reference does.
-__device__ inline uint32_t score_dup(const int* c) {
+// Rank and suit counts of cards that may repeat: rank counts are exact (a
+// rank seen 5+ times is neither quads, trips nor a pair, as with the
+// reference's rc[r] == 4 / 3 / 2 tests) and a suit flushes on its card count
+// (sc[s] >= 5) with the ranks it holds (sm[s]), as the reference does.
+struct DupCards {
     uint32_t one = 0, two = 0, three = 0, four = 0, five = 0;
-    uint32_t sm[4] = {0, 0, 0, 0};
-    int sc[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        const uint32_t b = 1u << (c[i] >> 2);
+    uint32_t cnt = 0;          // byte s: cards of suit s
+    uint32_t sm01 = 0, sm23 = 0;   // 16-bit halves: ranks held of suits 0, 1 and 2, 3
+    __device__ __forceinline__ void add(int card) {
+        const uint32_t b = 1u << (card >> 2);
         five |= four & b; four |= three & b; three |= two & b; two |= one & b; one |= b;
-        sm[c[i] & 3] |= b;
-        sc[c[i] & 3] += 1;
+        cnt += 1u << ((card & 3) * 8);
+        const uint32_t h = b << ((card & 1) * 16);
+        if (card & 2) sm23 |= h; else sm01 |= h;
     }
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        if (sc[s] >= 5) {
-            const int sf = straight_high(sm[s]);
-            if (sf >= 0) return (8u << 24) | (uint32_t)sf;
-            uint32_t m = sm[s], score = 5u << 24;
-            for (int p = 0; p < 5 && m; ++p) {
-                const int r = hi_bit(m);
-                score |= (uint32_t)r << (4 * (4 - p));
-                m ^= 1u << r;
-            }
-            return score;
+};
+
+__device__ __forceinline__ uint32_t score_dup(const DupCards& d) {
+    const uint32_t fl = (d.cnt + 0x7B7B7B7Bu) & 0x80808080u;   // a byte of 5 or more
+    if (fl) {
+        const int s = (31 - __clz(fl & (0u - fl))) >> 3;       // 7 cards: at most one suit
+        const uint32_t ranks = ((s & 2 ? d.sm23 : d.sm01) >> ((s & 1) * 16)) & 0x1FFFu;
+        const int sf = straight_high(ranks);
+        if (sf >= 0) return (8u << 24) | (uint32_t)sf;
+        uint32_t m = ranks, score = 5u << 24;
+        for (int p = 0; p < 5 && m; ++p) {
+            const int r = hi_bit(m);
+            score |= (uint32_t)r << (4 * (4 - p));
+            m ^= 1u << r;
         }
+        return score;
     }
-    const uint32_t quads = four & ~five, trips = three & ~four, pairs = two & ~three;
+    const uint32_t quads = d.four & ~d.five, trips = d.three & ~d.four, pairs = d.two & ~d.three;
     if (quads) return (7u << 24) | ((uint32_t)hi_bit(quads) << 4);
     const int t1 = trips ? hi_bit(trips) : -1;
     const uint32_t trips2 = trips & ~(t1 >= 0 ? (1u << t1) : 0u);
@@ -133,27 +139,46 @@ __device__ inline uint32_t score_dup(const int* c) {
     const uint32_t pairs2 = pairs & ~(p1 >= 0 ? (1u << p1) : 0u);
     const int p2 = pairs2 ? hi_bit(pairs2) : -1;
     if (t1 >= 0 && (t2 >= 0 || p1 >= 0)) return (6u << 24) | ((uint32_t)t1 << 4) | (uint32_t)(t2 >= 0 ? t2 : p1);
-    const int st = straight_high(one);
+    const int st = straight_high(d.one);
     if (st >= 0) return (4u << 24) | (uint32_t)st;
     if (t1 >= 0) return (3u << 24) | ((uint32_t)t1 << 8);
     if (p1 >= 0 && p2 >= 0) return (2u << 24) | ((uint32_t)p1 << 8) | ((uint32_t)p2 << 4);
     if (p1 >= 0) return (1u << 24) | ((uint32_t)p1 << 12);
-    return one;
+    return d.one;
 }
 
-// kernel_gen_preflop_matrix (:95-127): thread per (hero, villain) class pair.
-__global__ void __launch_bounds__(128) k_pf_allin(int mode, float* __restrict__ out, int* __restrict__ wins_out,
-                                                  int* __restrict__ ties_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= NC * NC) return;
+// The all-in sampler (kernel_gen_preflop_matrix, :95-127).  28,561 class
+// pairs are 6 warps an SM, so one thread per pair left the chip waiting on
+// dependent steps (9.3 ms, 3.1 us a sample; 1.8 ms now).  In the reference's mode boards
+// are drawn with replacement, samples depend only on the generator, and
+// AI_SPLIT threads of a pair take a share each, their generators started by
+// the LCG's n-step map; counts add up exactly.  Without replacement the deck's
+// order carries over from sample to sample, so there one thread keeps a pair,
+// its deck in shared memory (AI_DECK words apart by thread: no bank
+// conflicts).  Divisions by the deck size are multiplications by its
+// reciprocal, exact for 16-bit dividends.
+constexpr int AI_SPLIT = 8, AI_THREADS = 128, AI_SHARE = SAMPLES / AI_SPLIT;
+static_assert(AI_SHARE * AI_SPLIT == SAMPLES && AI_THREADS % AI_SPLIT == 0, "equal shares");
+
+template <int MODE>
+__global__ void __launch_bounds__(AI_THREADS) k_pf_allin(float* __restrict__ out, int* __restrict__ wins_out,
+                                                         int* __restrict__ ties_out) {
+    constexpr bool REF = MODE == MTT_PF_REFERENCE;
+    constexpr int SPLIT = REF ? AI_SPLIT : 1;
+    __shared__ uint32_t deck[REF ? 1 : 52][AI_THREADS];
+    const int tid = threadIdx.x;
+    const int i = (blockIdx.x * AI_THREADS + tid) / SPLIT, part = tid % SPLIT;
+    if (i >= NC * NC) return;                 // a pair's threads leave together
     const int hc = i / NC, vc = i % NC;
     if (hc == vc) {
-        out[i] = 0.5f;
-        if (wins_out) { wins_out[i] = 0; ties_out[i] = 0; }
+        if (part == 0) {
+            out[i] = 0.5f;
+            if (wins_out) { wins_out[i] = 0; ties_out[i] = 0; }
+        }
         return;
     }
     int h1, h2, v1, v2;
-    if (mode == MTT_PF_REFERENCE) {
+    if (REF) {
         class_cards_ref(hc, h1, h2);
         class_cards_ref(vc, v1, v2);
         if (h1 == v1 || h1 == v2 || h2 == v1 || h2 == v2) {   // the reference's suit switch (:104-107)
@@ -165,35 +190,73 @@ __global__ void __launch_bounds__(128) k_pf_allin(int mode, float* __restrict__ 
         class_cards_avoid(vc, (1ull << h1) | (1ull << h2), v1, v2);
     }
     const uint64_t dead = (1ull << h1) | (1ull << h2) | (1ull << v1) | (1ull << v2);
-    uint8_t deck[52];
-    int dsz = 0;
-    for (int c = 0; c < 52; ++c) if (!((dead >> c) & 1ull)) deck[dsz++] = (uint8_t)c;
+    const int dsz = 52 - __popcll(dead);
+    int gone[4];                              // dead cards ascending, 52 past the last
+    {
+        uint64_t m = dead;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            gone[k] = m ? __ffsll((long long)m) - 1 : 52;
+            m &= m - 1ull;
+        }
+    }
+    if (!REF)
+        for (int c = 0, n = 0; c < 52; ++c) if (!((dead >> c) & 1ull)) deck[n++][tid] = (uint32_t)c;
+    uint32_t recip[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) recip[k] = 0xFFFFFFFFu / (uint32_t)(dsz - k) + 1u;
     uint32_t rng = (uint32_t)(hc * 169 + vc) * 2654435761u + 0x9E3779B9u;
+    if (REF) {                                // 5 * AI_SHARE * part steps ahead: x -> A x + C, squared bit by bit
+        uint32_t A = 1664525u, C = 1013904223u;
+        for (uint32_t n = 5u * AI_SHARE * (uint32_t)part; n; n >>= 1) {
+            if (n & 1u) rng = rng * A + C;
+            C = C * (A + 1u);
+            A = A * A;
+        }
+    }
+    DupCards hero, vill;
+    hero.add(h1); hero.add(h2);
+    vill.add(v1); vill.add(v2);
     int wins = 0, ties = 0;
-    int a[7] = {h1, h2, 0, 0, 0, 0, 0}, b[7] = {v1, v2, 0, 0, 0, 0, 0};
-    for (int s = 0; s < SAMPLES; ++s) {
+    for (int s = 0; s < SAMPLES / SPLIT; ++s) {
+        DupCards a = hero, b = vill;
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             rng = rng * 1664525u + 1013904223u;
-            const int pick = k + (int)((rng >> 16) % (uint32_t)(dsz - k));
-            int card = deck[pick];
-            if (mode != MTT_PF_REFERENCE) {   // without replacement: partial Fisher-Yates
-                deck[pick] = deck[k];
-                deck[k] = (uint8_t)card;
+            const uint32_t x = rng >> 16;
+            const int pick = k + (int)(x - __umulhi(x, recip[k]) * (uint32_t)(dsz - k));
+            int card;
+            if (REF) {                        // the pick-th live card: step over each dead card below it
+                card = pick;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) card += card >= gone[q];
+            } else {                          // without replacement: partial Fisher-Yates
+                card = (int)deck[pick][tid];
+                deck[pick][tid] = deck[k][tid];
+                deck[k][tid] = (uint32_t)card;
             }
-            a[2 + k] = card;
-            b[2 + k] = card;
+            a.add(card);
+            b.add(card);
         }
         const uint32_t sh = score_dup(a), sv = score_dup(b);
         wins += sh > sv;
         ties += sh == sv;
     }
+    if (SPLIT > 1) {
+        const unsigned mask = (SPLIT == 32 ? 0xFFFFFFFFu : ((1u << SPLIT) - 1u)) << ((tid & 31) / SPLIT * SPLIT);
+#pragma unroll
+        for (int o = SPLIT / 2; o > 0; o >>= 1) {
+            wins += __shfl_down_sync(mask, wins, o, SPLIT);
+            ties += __shfl_down_sync(mask, ties, o, SPLIT);
+        }
+        if (part) return;
+    }
     out[i] = ((float)wins + 0.5f * (float)ties) / (float)SAMPLES;
     if (wins_out) { wins_out[i] = wins; ties_out[i] = ties; }
 }
 
-// Key table of one flop: KT[pair][combo] = 16-bit score key of combo with
-// the flop and the (turn, river) pair (0xFFFF where cards collide).
+// Key table of one flop: KT[pair][combo] = hero half (mtt_pairs.cuh) of combo
+// with the flop and the (turn, river) pair (dead where cards collide).
 __global__ void __launch_bounds__(256) k_pf_keys(const uint8_t* __restrict__ flops, const uint16_t* __restrict__ cc,
                                                  int ncombo, int ld, uint16_t* __restrict__ KT) {
     const int f = blockIdx.y;
@@ -213,7 +276,7 @@ __global__ void __launch_bounds__(256) k_pf_keys(const uint8_t* __restrict__ flo
     }
     uint16_t* out = KT + ((size_t)f * NPAIR + p) * ld;
     for (int j = threadIdx.x; j < ld; j += blockDim.x) {
-        uint16_t key = 0xFFFFu;
+        uint16_t key = (uint16_t)KEY_H_DEAD;
         if (j < ncombo) {
             const int c1 = cc[2 * j], c2 = cc[2 * j + 1];
             const uint64_t m = (1ull << c1) | (1ull << c2);
@@ -221,81 +284,140 @@ __global__ void __launch_bounds__(256) k_pf_keys(const uint8_t* __restrict__ flo
                 Planes pl; planes_clear(pl);
                 planes_add(pl, f0); planes_add(pl, f1); planes_add(pl, f2);
                 planes_add(pl, c1); planes_add(pl, c2); planes_add(pl, ta); planes_add(pl, tb);
-                key = (uint16_t)key_planes(pl);
+                key = (uint16_t)(key_planes(pl) + 1u);
             }
         }
         out[j] = key;
     }
 }
 
-// kernel_gen_100_flop_matrices (:130-183) from the key table: CTA per hero
-// combo; E[f][j][h] = (wins + ties / 2) / total with the mode's tie weight.
-__global__ void __launch_bounds__(256) k_pf_flop_eq(const uint8_t* __restrict__ flops, const uint16_t* __restrict__ cc,
-                                                    const int* __restrict__ cidx, int ncombo, int ld, int mode,
-                                                    const uint16_t* __restrict__ KT, float* __restrict__ E) {
-    __shared__ uint16_t rp[256];     // pair index of each hero runout
-    __shared__ uint16_t rk[256];     // hero key there
-    __shared__ uint64_t rm[256];     // card mask of the runout
-    __shared__ int nr;
-    const int f = blockIdx.y, h = blockIdx.x;
-    if (h >= ncombo) return;
-    const uint8_t f0 = flops[3 * f], f1 = flops[3 * f + 1], f2 = flops[3 * f + 2];
-    const uint64_t fm = (1ull << f0) | (1ull << f1) | (1ull << f2);
-    const int hc1 = cc[2 * h], hc2 = cc[2 * h + 1];
-    const uint64_t hm = (1ull << hc1) | (1ull << hc2);
-    const int hcol = cidx[h];      // column of this hero in the padded matrix
-    float* Ef = E + (size_t)f * ld * ld;
-    if (hm & fm) {
-        // the reference never writes these entries; here they are 0
-        for (int j = threadIdx.x; j < ncombo; j += blockDim.x) Ef[(size_t)cidx[j] * ld + hcol] = 0.0f;
-        return;
+// Runout k of a 47-card deck in the reference's order: r1 = 0, 2, .., r2 =
+// r1 + 1, r1 + 4, ..; 192 of them.
+constexpr int RUNS = 192;
+
+// Position in a 49-card deck of card r of the 47-card deck that lacks
+// positions a < b.
+__device__ __forceinline__ int deck_pos(int r, int a, int b) {
+    r += r >= a;
+    return r + (r >= b);
+}
+__device__ __forceinline__ int flop_deck_pos(uint64_t fm, int card) {
+    return card - __popcll(fm & ((1ull << card) - 1ull));
+}
+
+// Hero lists: HL[f][h][k] = pair index << 16 | hero half of combo h on its
+// runout k.  Not written for combos that touch the flop.
+__global__ void __launch_bounds__(RUNS) k_pf_runs(const uint8_t* __restrict__ flops, const uint16_t* __restrict__ cc,
+                                                  int ncombo, int ld, const uint16_t* __restrict__ KT,
+                                                  uint32_t* __restrict__ HL) {
+    const int f = blockIdx.y, h = blockIdx.x, k = threadIdx.x;
+    const uint64_t fm = (1ull << flops[3 * f]) | (1ull << flops[3 * f + 1]) | (1ull << flops[3 * f + 2]);
+    const int c1 = cc[2 * h], c2 = cc[2 * h + 1];
+    if (((fm >> c1) | (fm >> c2)) & 1ull) return;
+    int r1 = 0, left = k;
+    for (;;) {                                 // runouts with this r1: r2 = r1 + 1, r1 + 4, .. < 47
+        const int n = (47 - r1 - 1 + 2) / 3;
+        if (left < n) break;
+        left -= n;
+        r1 += 2;
     }
-    if (threadIdx.x == 0) {
-        // the hero's 47-card deck and its runout subsample
-        uint8_t deck[52];
-        int dsz = 0;
-        for (int c = 0; c < 52; ++c) if (!(((hm | fm) >> c) & 1ull)) deck[dsz++] = (uint8_t)c;
-        // position of a card in the 49-card flop deck
-        auto fpos = [&](int c) { int n = 0; for (int x = 0; x < c; ++x) n += !((fm >> x) & 1ull); return n; };
-        int n = 0;
-        for (int r1 = 0; r1 < dsz; r1 += 2)
-            for (int r2 = r1 + 1; r2 < dsz; r2 += 3) {
-                const int t = deck[r1], r = deck[r2];
-                const int a = fpos(t), b = fpos(r);     // a < b since the deck is ascending
-                const int p = a * 48 - (a * (a - 1)) / 2 + (b - a - 1);
-                rp[n] = (uint16_t)p;
-                rm[n] = (1ull << t) | (1ull << r);
-                ++n;
-            }
-        nr = n;
-    }
-    __syncthreads();
-    const int n = nr;
-    const uint16_t* KTf = KT + (size_t)f * NPAIR * ld;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) rk[k] = KTf[(size_t)rp[k] * ld + h];
-    __syncthreads();
-    for (int j = threadIdx.x; j < ncombo; j += blockDim.x) {
-        const int v1 = cc[2 * j], v2 = cc[2 * j + 1];
-        const uint64_t vm = (1ull << v1) | (1ull << v2);
-        float eq = 0.0f;
-        if (!(vm & hm) && !(vm & fm)) {
-            int wins = 0, ties = 0, total = 0;
-            for (int k = 0; k < n; ++k) {
-                if (rm[k] & vm) continue;
-                const uint16_t hk = rk[k], vk = KTf[(size_t)rp[k] * ld + j];
-                if (mode == MTT_PF_REFERENCE) {
-                    wins += hk > vk ? 2 : 0;
-                    ties += hk == vk ? 1 : 0;
-                    total += 2;
-                } else {
-                    wins += hk > vk ? 2 : 0;
-                    ties += hk == vk ? 2 : 0;
-                    total += 2;
-                }
-            }
-            eq = total > 0 ? ((float)wins + 0.5f * (float)ties) / (float)total : 0.0f;
+    const int r2 = r1 + 1 + 3 * left;
+    const int a = flop_deck_pos(fm, c1), b = flop_deck_pos(fm, c2);
+    const int x = deck_pos(r1, a, b), y = deck_pos(r2, a, b);
+    const int p = x * 48 - (x * (x - 1)) / 2 + (y - x - 1);
+    HL[((size_t)f * ncombo + h) * RUNS + k] = ((uint32_t)p << 16) | KT[((size_t)f * NPAIR + p) * ld + h];
+}
+
+// kernel_gen_100_flop_matrices (:130-183): E[f][h][j] = (wins + ties / 2) /
+// total of hero h against villain j with the mode's tie weight.  One CTA
+// holds EQ_VILL villains' keys of all 1,176 pairs in shared memory (150 KB, a
+// word per two villains, 32 words a row: conflict-free) and its warps take
+// heroes in turn; a hero's list is staged per warp as (row offset, doubled
+// hero half) and read two runouts a 16-byte broadcast.  Per runout and 64
+// pairs: one broadcast half, one row load, one packed clamp, its win bits and
+// their adds.  Usable runouts are counted by inclusion and exclusion from the
+// villain's positions in the hero's deck, not in the loop.  The kernel
+// before read the table from L2 one 16-bit key at a time and wrote the matrix
+// with a stride of a row: 29.9 ms for 100 flops, 3.5 ms now.
+constexpr int EQ_VILL = 64, EQ_WARPS = 32, EQ_THREADS = 32 * EQ_WARPS;
+constexpr int EQ_TABLE = NPAIR * EQ_VILL / 2;                       // words
+constexpr int EQ_SMEM = 4 * EQ_TABLE + 8 * RUNS * EQ_WARPS;         // 199,680 B
+
+__global__ void __launch_bounds__(EQ_THREADS, 1) k_pf_flop_eq(const uint8_t* __restrict__ flops,
+                                                           const uint16_t* __restrict__ cc, int ncombo, int ld, int mode,
+                                                           const uint16_t* __restrict__ KT,
+                                                           const uint32_t* __restrict__ HL, float* __restrict__ E) {
+    extern __shared__ __align__(16) uint32_t eq_smem[];
+    __shared__ uint64_t adj[47];               // bit y of adj[x]: 47-card deck positions x and y are a runout
+    const int f = blockIdx.y, j0 = blockIdx.x * EQ_VILL;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < 47) {
+        uint64_t m = 0;
+        for (int y = 0; y < 47; ++y) {
+            const int lo = min(tid, y), hi = max(tid, y);
+            if (lo != hi && !(lo & 1) && (hi - lo - 1) % 3 == 0) m |= 1ull << y;
         }
-        Ef[(size_t)cidx[j] * ld + hcol] = eq;
+        adj[tid] = m;
+    }
+    // ld is a multiple of EQ_VILL: every tile's words exist (dead past ncombo)
+    const uint32_t* KTf = reinterpret_cast<const uint32_t*>(KT + (size_t)f * NPAIR * ld + j0);
+    for (int e = tid; e < EQ_TABLE; e += EQ_THREADS)
+        eq_smem[e] = villain_word(KTf[(size_t)(e >> 5) * (ld >> 1) + (e & 31)]);
+    __syncthreads();
+    uint2* list = reinterpret_cast<uint2*>(eq_smem + EQ_TABLE) + warp * RUNS;
+    const char* table = reinterpret_cast<const char*>(eq_smem + lane);
+    const uint64_t fm = (1ull << flops[3 * f]) | (1ull << flops[3 * f + 1]) | (1ull << flops[3 * f + 2]);
+    const int j = j0 + 2 * lane;               // this lane's villains: j and j + 1
+    int pos[2][2];                             // their positions in the flop's deck
+    uint64_t vm[2];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        const int jj = min(j + v, ncombo - 1);
+        const int c1 = cc[2 * jj], c2 = cc[2 * jj + 1];
+        vm[v] = (1ull << c1) | (1ull << c2);
+        pos[v][0] = flop_deck_pos(fm, c1);
+        pos[v][1] = flop_deck_pos(fm, c2);
+    }
+    float* Ef = E + (size_t)f * ld * ld;
+    for (int h = warp; h < ncombo; h += EQ_WARPS) {
+        const int hc1 = cc[2 * h], hc2 = cc[2 * h + 1];
+        const uint64_t hm = (1ull << hc1) | (1ull << hc2);
+        float2 eq = make_float2(0.0f, 0.0f);   // heroes on the flop: the reference never writes these; here 0
+        if (!(hm & fm)) {
+            const uint32_t* src = HL + ((size_t)f * ncombo + h) * RUNS;
+            __syncwarp();
+#pragma unroll
+            for (int k = lane; k < RUNS; k += 32) {
+                const uint32_t w = src[k];
+                list[k] = make_uint2((w >> 16) * (4u * 32u), (w & 0xFFFFu) * 0x00010001u);
+            }
+            __syncwarp();
+            uint32_t sc = 0u, w2 = 0u;         // halves: 2 wins + ties; 2 wins (at most 2 * 192)
+#pragma unroll 8
+            for (int k = 0; k < RUNS; k += 2) {
+                const uint4 l = *reinterpret_cast<const uint4*>(list + k);
+                const uint32_t t0 = pair_2w_t(l.y, *reinterpret_cast<const uint32_t*>(table + l.x));
+                const uint32_t t1 = pair_2w_t(l.w, *reinterpret_cast<const uint32_t*>(table + l.z));
+                sc += t0 + t1;
+                w2 += (t0 & 0x00020002u) + (t1 & 0x00020002u);
+            }
+            const int a = flop_deck_pos(fm, hc1), b = flop_deck_pos(fm, hc2);
+            float r[2];
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                r[v] = 0.0f;
+                if ((vm[v] & hm) || (vm[v] & fm) || j + v >= ncombo) continue;
+                const int x = pos[v][0] - (pos[v][0] > a) - (pos[v][0] > b);
+                const int y = pos[v][1] - (pos[v][1] > a) - (pos[v][1] > b);
+                const int n = RUNS - __popcll(adj[x]) - __popcll(adj[y]) + (int)((adj[x] >> y) & 1ull);
+                const int wins = (int)(v ? w2 >> 16 : w2 & 0xFFFFu);
+                const int t = (int)(v ? sc >> 16 : sc & 0xFFFFu) - wins;
+                const int ties = mode == MTT_PF_REFERENCE ? t : 2 * t;
+                r[v] = n > 0 ? ((float)wins + 0.5f * (float)ties) / (float)(2 * n) : 0.0f;
+            }
+            eq = make_float2(r[0], r[1]);
+        }
+        *reinterpret_cast<float2*>(Ef + (size_t)h * ld + j) = eq;
     }
 }
 
@@ -310,7 +432,7 @@ __global__ void k_pf_reduce(const float* __restrict__ E, int ld, const int* __re
     for (int i = 0; i < counts[hcl]; ++i) {
         const int ch = lists[hcl * 12 + i];
         for (int j = 0; j < counts[vcl]; ++j) {
-            const float eq = Ef[(size_t)lists[vcl * 12 + j] * ld + ch];
+            const float eq = Ef[(size_t)ch * ld + lists[vcl * 12 + j]];
             if (eq > 0.0f) { sum = __fadd_rn(sum, eq); valid++; }
         }
     }
@@ -322,7 +444,6 @@ __global__ void k_pf_reduce(const float* __restrict__ E, int ld, const int* __re
 // per flop by the kernels) and up to `cap` combos per class.
 struct Lists {
     std::vector<uint16_t> cc;     // 2 per combo
-    std::vector<int> cidx;        // padded-matrix column of each combo
     std::vector<int> lists, counts;
     int ncombo = 0;
 };
@@ -339,7 +460,6 @@ static Lists make_lists(int mode) {
             const int cls = combo_class(c1, c2);
             L.cc.push_back((uint16_t)c1);
             L.cc.push_back((uint16_t)c2);
-            L.cidx.push_back(L.ncombo);
             if (L.counts[cls] < cap) L.lists[cls * 12 + L.counts[cls]++] = L.ncombo;
             ++L.ncombo;
         }
@@ -354,7 +474,11 @@ using namespace mtt::pf;
 
 extern "C" int mtt_pf_allin_matrix(int32_t mode, float* d_out, int32_t* d_wins, int32_t* d_ties, void* stream) {
     if (!d_out || (mode != MTT_PF_REFERENCE && mode != MTT_PF_CORRECT) || (!d_wins != !d_ties)) return MTT_ERR_INVALID;
-    k_pf_allin<<<(NC * NC + 127) / 128, 128, 0, as_stream(stream)>>>(mode, d_out, d_wins, d_ties);
+    cudaStream_t st = as_stream(stream);
+    if (mode == MTT_PF_REFERENCE)
+        k_pf_allin<MTT_PF_REFERENCE><<<ceil_div(NC * NC * AI_SPLIT, AI_THREADS), AI_THREADS, 0, st>>>(d_out, d_wins, d_ties);
+    else
+        k_pf_allin<MTT_PF_CORRECT><<<ceil_div(NC * NC, AI_THREADS), AI_THREADS, 0, st>>>(d_out, d_wins, d_ties);
     MTT_CHECK_LAUNCH();
     return MTT_OK;
 }
@@ -365,38 +489,40 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
     cudaStream_t st = as_stream(stream);
     const Lists L = make_lists(mode);
     const int ld = mode == MTT_PF_REFERENCE ? LD_REF : LD_OK;
-    constexpr int CHUNK = 8;   // flops per pass: 8 x (up to 3.2 MB of keys + 7.2 MB of matrix)
+    // flops per pass: one CTA of k_pf_flop_eq per (villain tile, flop) and SM,
+    // as many flops as fit three waves (23 of the reference's 19 tiles, 217 MB)
+    const int tiles = ceil_div(L.ncombo, EQ_VILL);
+    int dev = 0, sms = 0;
+    MTT_TRY_CUDA(cudaGetDevice(&dev));
+    MTT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MTT_TRY_CUDA(cudaFuncSetAttribute(k_pf_flop_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, EQ_SMEM));
+    const int chunk = std::max(1, std::min(n, std::min(3 * sms / tiles, 23)));
     uint16_t* d_cc = nullptr;
-    int *d_cidx = nullptr, *d_lists = nullptr, *d_counts = nullptr;
+    int *d_lists = nullptr, *d_counts = nullptr;
     uint16_t* d_KT = nullptr;
+    uint32_t* d_HL = nullptr;
     float* d_E = nullptr;
     int s = MTT_OK;
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_cc), sizeof(uint16_t) * L.cc.size(), st);
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_cidx), sizeof(int) * L.cidx.size(), st);
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_lists), sizeof(int) * L.lists.size(), st);
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_counts), sizeof(int) * L.counts.size(), st);
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_KT), sizeof(uint16_t) * (size_t)CHUNK * NPAIR * ld, st);
-    if (!s) s = scratch_alloc(reinterpret_cast<void**>(&d_E), sizeof(float) * (size_t)CHUNK * ld * ld, st);
+    if (!s) s = scratch_alloc(&d_cc, L.cc.size(), st);
+    if (!s) s = scratch_alloc(&d_lists, L.lists.size(), st);
+    if (!s) s = scratch_alloc(&d_counts, L.counts.size(), st);
+    if (!s) s = scratch_alloc(&d_KT, (size_t)chunk * NPAIR * ld, st);
+    if (!s) s = scratch_alloc(&d_HL, (size_t)chunk * L.ncombo * RUNS, st);
+    if (!s) s = scratch_alloc(&d_E, (size_t)chunk * ld * ld, st);
     if (!s) s = cuda_status(cudaMemcpyAsync(d_cc, L.cc.data(), sizeof(uint16_t) * L.cc.size(), cudaMemcpyHostToDevice, st));
-    if (!s) s = cuda_status(cudaMemcpyAsync(d_cidx, L.cidx.data(), sizeof(int) * L.cidx.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_lists, L.lists.data(), sizeof(int) * L.lists.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_counts, L.counts.data(), sizeof(int) * L.counts.size(), cudaMemcpyHostToDevice, st));
-    for (int f0 = 0; f0 < n && !s; f0 += CHUNK) {
-        const int nf = std::min(CHUNK, n - f0);
-        k_pf_keys<<<dim3(NPAIR, nf), 256, 0, st>>>(d_flops + 3 * f0, d_cc, L.ncombo, ld, d_KT);
+    for (int f0 = 0; f0 < n && !s; f0 += chunk) {
+        const int nf = std::min(chunk, n - f0);
+        const uint8_t* fl = d_flops + 3 * (size_t)f0;
+        k_pf_keys<<<dim3(NPAIR, nf), 256, 0, st>>>(fl, d_cc, L.ncombo, ld, d_KT);
+        k_pf_runs<<<dim3(L.ncombo, nf), RUNS, 0, st>>>(fl, d_cc, L.ncombo, ld, d_KT, d_HL);
+        k_pf_flop_eq<<<dim3(tiles, nf), EQ_THREADS, EQ_SMEM, st>>>(fl, d_cc, L.ncombo, ld, mode, d_KT, d_HL, d_E);
+        k_pf_reduce<<<dim3(NC, nf), PAD, 0, st>>>(d_E, ld, d_lists, d_counts, d_out + (size_t)f0 * NC * NC);
         s = cuda_status(cudaGetLastError());
-        if (!s) {
-            k_pf_flop_eq<<<dim3(L.ncombo, nf), 256, 0, st>>>(d_flops + 3 * f0, d_cc, d_cidx, L.ncombo, ld, mode, d_KT,
-                                                              d_E);
-            s = cuda_status(cudaGetLastError());
-        }
-        if (!s) {
-            k_pf_reduce<<<dim3(NC, nf), PAD, 0, st>>>(d_E, ld, d_lists, d_counts, d_out + (size_t)f0 * NC * NC);
-            s = cuda_status(cudaGetLastError());
-        }
     }
-    cudaFreeAsync(d_cc, st); cudaFreeAsync(d_cidx, st); cudaFreeAsync(d_lists, st); cudaFreeAsync(d_counts, st);
-    cudaFreeAsync(d_KT, st); cudaFreeAsync(d_E, st);
+    cudaFreeAsync(d_cc, st); cudaFreeAsync(d_lists, st); cudaFreeAsync(d_counts, st);
+    cudaFreeAsync(d_KT, st); cudaFreeAsync(d_HL, st); cudaFreeAsync(d_E, st);
     return s;
 }
 
@@ -417,91 +543,220 @@ constexpr int STATE = 10 * PAD;
 
 struct PfDev {
     const float* fw;        // flop weights [nf]
-    const float* mats;      // class matrices [nf][v][h]
-    const float* allin;     // [h][v]
-    const float* tab;       // per iteration: w_pos, w_strat
-    int* iter;              // 1-based iteration counter
-    float *R, *G, *S, *C;   // regrets, current strategy, strategy sums, action values [STATE]
-    float *root, *rbc, *rbb, *evb, *evbb;
+    const float* mats;      // class matrices [nf][MAT] (v-major, rows of 169)
+    const float* jam;       // all-in equity by step CTA: [tile][2][o][32 classes], as [o][cls] and transposed
+    float *R, *G, *S;       // regrets, current strategy, strategy sums [STATE]
+    float* Gn;              // the next strategy: every CTA of a step reads all classes of G
+    float *root, *evb, *evbb;
+    float *nb, *nbb;        // net flop EVs [nf][PAD]
     int nf;
     float stack, bf, dead;
 };
 
+constexpr int MAT = (NC * NC + 3) / 4 * 4;           // a class matrix padded to 16 bytes
+constexpr int STEP_CLS = 32, STEP_WARPS = 7, STEP_THREADS = STEP_CLS * STEP_WARPS;
+constexpr int STEP_TILES = (NC + STEP_CLS - 1) / STEP_CLS, STEP_JAM = 2 * NC * STEP_CLS;
+
+// Copies of the matrices in the layouts that the iterations stage 16 bytes at
+// a time: class matrices with padded stride, the all-in matrix in step tiles.
+__global__ void __launch_bounds__(256) k_pf_layout(const float* __restrict__ mats, const float* __restrict__ allin, int nf,
+                                                   float* __restrict__ om, float* __restrict__ oj) {
+    const size_t total = (size_t)nf * MAT, stride = (size_t)gridDim.x * blockDim.x;
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (size_t i = i0; i < total; i += stride) {
+        const int e = (int)(i % MAT);
+        om[i] = e < NC * NC ? mats[i / MAT * (NC * NC) + e] : 0.0f;
+    }
+    for (size_t i = i0; i < (size_t)STEP_TILES * STEP_JAM; i += stride) {
+        const int e = (int)(i % STEP_JAM), o = e / STEP_CLS % NC;
+        const int col = min((int)(i / STEP_JAM) * STEP_CLS + e % STEP_CLS, NC - 1);
+        oj[i] = e < NC * STEP_CLS ? allin[o * NC + col] : allin[col * NC + o];
+    }
+}
+
 __global__ void k_pf_init(PfDev d) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *d.iter = 1;
     if (i < STATE) {
         d.R[i] = 0.0f;
         d.S[i] = 0.0f;
-        d.C[i] = 0.0f;
-        d.G[i] = i < 6 * PAD ? 1.0f / 3.0f : 0.5f;
+        d.G[i] = d.Gn[i] = i < 6 * PAD ? 1.0f / 3.0f : 0.5f;
     }
-    if (i < PAD) d.root[i] = i < NC ? (i < 13 ? 6.0f : i < 91 ? 4.0f : 12.0f) / 1326.0f : 0.0f;
+    if (i < PAD) {
+        d.root[i] = i < NC ? (i < 13 ? 6.0f : i < 91 ? 4.0f : 12.0f) / 1326.0f : 0.0f;
+        d.evb[i] = 0.0f;
+        d.evbb[i] = 0.0f;
+    }
 }
 
-// kernel_update_dynamic_reaches (:412-421)
-__global__ void k_pf_reach(PfDev d) {
-    const int c = threadIdx.x;
-    if (c >= NC) return;
-    d.rbc[c] = __fmul_rn(d.root[c], d.G[node_off(0) + 1 * PAD + c]);
-    d.rbb[c] = __fmul_rn(d.root[c], d.G[node_off(1) + 1 * PAD + c]);
-}
+// One DCFR iteration is two launches, chained by programmatic dependent
+// launch: the reference's float sums run in a fixed order, so what can be
+// spread is the independent sums, and what bounds each launch is one chain of
+// 169 adds.  k_pf_cosolve: CTA per flop, thread per class and player;
+// k_pf_step: warp per sum over 32 classes.  Both stage the matrices they read,
+// which no iteration writes, in shared memory before they wait for the
+// launch ahead, so those loads run under its tail: an iteration over 100 flops
+// takes 11.5 us (most of it the two launches' hand-over), against 29 us with
+// the loads left in the chains.  The five launches before (thread per flop
+// over one class's strided column, all classes' sums in one CTA) took 80 us.
 
-// kernel_cosolve_100_board_matrices (:228-285): CTA per class; threads
-// evaluate the flops' net EVs in parallel, thread 0 accumulates them in flop
-// order, so the float sums follow the reference's loop exactly.
-__global__ void __launch_bounds__(128) k_pf_cosolve(PfDev d) {
-    __shared__ float nb_s[128], nbb_s[128];
-    __shared__ float acc[3];
-    const int cls = blockIdx.x, tid = threadIdx.x;
-    const float pot_flop = __fadd_rn(d.dead, 3.1f);
-    if (tid == 0) { acc[0] = 0.0f; acc[1] = 0.0f; acc[2] = 0.0f; }
-    for (int f0 = 0; f0 < d.nf; f0 += 128) {
-        const int f = f0 + tid;
-        if (f < d.nf) {
-            const float* eq = d.mats + (size_t)f * NC * NC;
-            float s1 = 0.0f, e0 = 0.0f, s0 = 0.0f, e1 = 0.0f;
-            for (int o = 0; o < NC; ++o) {
-                const float r = d.rbb[o];
-                s1 = __fadd_rn(s1, r);
-                e0 = __fadd_rn(e0, __fmul_rn(r, eq[o * NC + cls]));
-            }
-            if (s1 > 1e-7f) e0 = __fdiv_rn(e0, s1);
-            for (int o = 0; o < NC; ++o) {
-                const float r = d.rbc[o];
-                s0 = __fadd_rn(s0, r);
-                e1 = __fadd_rn(e1, __fmul_rn(r, __fsub_rn(1.0f, eq[cls * NC + o])));
-            }
-            if (s0 > 1e-7f) e1 = __fdiv_rn(e1, s0);
-            const float shb = __fmul_rn(__fmul_rn(e0, 1.06f), pot_flop);
-            const float shbb = __fmul_rn(__fmul_rn(e1, 0.94f), pot_flop);
-            nb_s[tid] = shb >= 2.1f ? __fsub_rn(shb, 2.1f) : -__fmul_rn(__fsub_rn(2.1f, shb), d.bf);
-            nbb_s[tid] = shbb >= 2.1f ? __fsub_rn(shbb, 2.1f) : -__fmul_rn(__fsub_rn(2.1f, shbb), d.bf);
+// Asynchronous copies of 16 and 4 bytes to shared memory; copies_done waits
+// for this thread's copies (a barrier must follow).
+__device__ __forceinline__ void copy16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Net flop EVs of the reached classes (kernel_update_dynamic_reaches,
+// :412-421, and the per-flop part of kernel_cosolve_100_board_matrices,
+// :228-285).
+constexpr int COSOLVE_SMEM = 4 * MAT;
+__global__ void __launch_bounds__(2 * PAD) k_pf_cosolve(PfDev d) {
+    extern __shared__ __align__(16) float eqm[];   // the flop's matrix: 169 is odd, so rows and columns are conflict-free
+    __shared__ float rb[2][PAD];              // reach: BB's classes, BTN's classes
+    __shared__ float rsum[2];
+    const int f = blockIdx.x, tid = threadIdx.x;
+    const int side = tid / PAD, cls = tid % PAD;   // side 0: BTN's EV, 1: BB's
+    for (int i = tid; i < MAT / 4; i += 2 * PAD) copy16(eqm + 4 * i, d.mats + (size_t)f * MAT + 4 * i);
+    grid_dep_wait();
+    grid_dep_trigger();
+    if (cls < NC)                             // side 0 sums over BB's reach, side 1 over BTN's
+        rb[side][cls] = __fmul_rn(d.root[cls], d.G[node_off(1 - side) + PAD + cls]);
+    copies_done();
+    __syncthreads();
+    float e = 0.0f;
+    if (cls < NC) {
+        const float* eq = eqm + (side ? cls * NC : cls);
+        const float* r = rb[side];
+        if (side) {
+#pragma unroll 13
+            for (int o = 0; o < NC; ++o) e = __fadd_rn(e, __fmul_rn(r[o], __fsub_rn(1.0f, eq[o])));
+        } else {
+#pragma unroll 13
+            for (int o = 0; o < NC; ++o) e = __fadd_rn(e, __fmul_rn(r[o], eq[o * NC]));
         }
-        __syncthreads();
-        if (tid == 0) {
-            const int n = min(128, d.nf - f0);
-            for (int k = 0; k < n; ++k) {
-                const float w = d.fw[f0 + k];
-                acc[2] = __fadd_rn(acc[2], w);
-                acc[0] = __fadd_rn(acc[0], __fmul_rn(w, nb_s[k]));
-                acc[1] = __fadd_rn(acc[1], __fmul_rn(w, nbb_s[k]));
-            }
-        }
-        __syncthreads();
+    } else if (cls == PAD - 1) {              // an idle thread of each side adds the reach up
+        float sum = 0.0f;
+#pragma unroll 13
+        for (int o = 0; o < NC; ++o) sum = __fadd_rn(sum, rb[side][o]);
+        rsum[side] = sum;
     }
-    if (tid == 0 && acc[2] > 0.0f) {
-        d.evb[cls] = __fdiv_rn(acc[0], acc[2]);
-        d.evbb[cls] = __fdiv_rn(acc[1], acc[2]);
-    }
-}
-
-// kernel_build_closed_preflop_cfvs (:290-385)
-__global__ void k_pf_cfvs(PfDev d) {
-    const int cls = threadIdx.x;
+    __syncthreads();
     if (cls >= NC) return;
-    const float *sbr = d.G + node_off(0), *sbd = d.G + node_off(1), *s3b = d.G + node_off(2), *sbj = d.G + node_off(3);
-    float *cbr = d.C + node_off(0), *cbd = d.C + node_off(1), *c3b = d.C + node_off(2), *cbj = d.C + node_off(3);
+    const float pot_flop = __fadd_rn(d.dead, 3.1f);
+    if (rsum[side] > 1e-7f) e = __fdiv_rn(e, rsum[side]);
+    const float sh = __fmul_rn(__fmul_rn(e, side ? 0.94f : 1.06f), pot_flop);
+    (side ? d.nbb : d.nb)[(size_t)f * PAD + cls] =
+        sh >= 2.1f ? __fsub_rn(sh, 2.1f) : -__fmul_rn(__fsub_rn(2.1f, sh), d.bf);
+}
+
+// The weighted flop average (:270-285), the action values of the four nodes
+// (kernel_build_closed_preflop_cfvs, :290-385) and their regret and strategy
+// update (kernel_dcfr_step, :387-410) for 32 classes per CTA.  The masses
+// behind the action values are the same for every class: one warp forms the
+// nine of them, a lane each.  Four warps form one equity sum each over their
+// 32 classes and two the flop averages; then warp k updates node k.
+constexpr int STEP_FLOPS = 128;           // flops staged at a time
+constexpr int STEP_SMEM = 4 * (STEP_JAM + STEP_FLOPS * (2 * STEP_CLS + 1));
+enum { M_M3, M_BF3, M_BC3, M_MJ, M_CJ, M_FM, M_CM, M_JM, M_FJ, N_MASS };   // mass order; the first of each equity sum's too
+__global__ void __launch_bounds__(STEP_THREADS) k_pf_step(PfDev d, float wp, float ws) {
+    extern __shared__ __align__(16) float step_smem[];
+    __shared__ float G[STATE], root[PAD];
+    __shared__ float reach[N_MASS][PAD];                     // summands of the masses
+    __shared__ float mass[N_MASS];
+    __shared__ float sums[6][STEP_CLS];                      // equity sums of warps 0..3, flop sums of warps 4, 5
+    __shared__ float wsum;                                   // flop weights
+    float* const Ac = step_smem;                             // all-in equity [o][cls] of this CTA's classes
+    float* const Ar = Ac + NC * STEP_CLS;                    // [o][cls] of the transpose
+    float* const nbs = Ar + NC * STEP_CLS;                   // net flop EVs [player][flop][cls]
+    float* const fws = nbs + STEP_FLOPS * 2 * STEP_CLS;      // flop weights
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cls = blockIdx.x * STEP_CLS + lane;
+    const int col = min(cls, NC - 1);
+    for (int i = tid; i < STEP_JAM / 4; i += STEP_THREADS)
+        copy16(step_smem + 4 * i, d.jam + (size_t)blockIdx.x * STEP_JAM + 4 * i);
+    auto stage_flops = [&](int f0) {                         // flops [f0, f0 + STEP_FLOPS)
+        const int n = min(STEP_FLOPS, d.nf - f0);
+        for (int k = warp; k < n; k += STEP_WARPS) {
+            copy4(nbs + k * STEP_CLS + lane, d.nb + (size_t)(f0 + k) * PAD + col);
+            copy4(nbs + (STEP_FLOPS + k) * STEP_CLS + lane, d.nbb + (size_t)(f0 + k) * PAD + col);
+        }
+        for (int k = tid; k < n; k += STEP_THREADS) copy4(fws + k, d.fw + f0 + k);
+    };
+    grid_dep_wait();
+    grid_dep_trigger();
+    for (int i = tid; i < STATE / 4; i += STEP_THREADS) copy16(G + 4 * i, d.G + 4 * i);
+    for (int i = tid; i < PAD / 4; i += STEP_THREADS) copy16(root + 4 * i, d.root + 4 * i);
+    stage_flops(0);
+    float Rc[3] = {0.0f, 0.0f, 0.0f}, Sc[3] = {0.0f, 0.0f, 0.0f};   // the updated node's rows of this class
+    if (warp < 4 && cls < NC)
+        for (int a = 0; a < node_actions(warp); ++a) {
+            Rc[a] = d.R[node_off(warp) + a * PAD + cls];
+            Sc[a] = d.S[node_off(warp) + a * PAD + cls];
+        }
+    copies_done();
+    __syncthreads();
+    const float *sbr = G + node_off(0), *sbd = G + node_off(1), *s3b = G + node_off(2), *sbj = G + node_off(3);
+    for (int o = tid; o < NC; o += STEP_THREADS) {
+        const float r = root[o], ro = __fmul_rn(r, sbr[PAD + o]);
+        reach[M_M3][o] = __fmul_rn(r, sbd[2 * PAD + o]);
+        reach[M_BF3][o] = __fmul_rn(ro, s3b[o]);
+        reach[M_BC3][o] = __fmul_rn(ro, s3b[PAD + o]);
+        reach[M_MJ][o] = __fmul_rn(r, sbr[2 * PAD + o]);
+        reach[M_CJ][o] = __fmul_rn(r, sbj[PAD + o]);
+        reach[M_FM][o] = __fmul_rn(r, sbd[o]);
+        reach[M_CM][o] = __fmul_rn(r, sbd[PAD + o]);
+        reach[M_JM][o] = reach[M_M3][o];
+        reach[M_FJ][o] = __fmul_rn(r, sbj[o]);
+    }
+    __syncthreads();
+    // equity sums: warp 0 BTN vs 3-bet jam (eqc), 1 BB's jam over the min-raise (eqj), 2 BB vs open jam (eqo),
+    // 3 BTN's open jam (eo)
+    if (warp < 4) {
+        const float* r = reach[warp == 0 ? M_M3 : warp == 1 ? M_BC3 : warp == 2 ? M_MJ : M_CJ];
+        float y = 0.0f;
+        if (warp == 0 || warp == 3) {
+            const float* A = Ar + lane;
+#pragma unroll 13
+            for (int o = 0; o < NC; ++o) y = __fadd_rn(y, __fmul_rn(r[o], A[o * STEP_CLS]));
+        } else {
+            const float* A = Ac + lane;
+#pragma unroll 13
+            for (int o = 0; o < NC; ++o) y = __fadd_rn(y, __fmul_rn(r[o], __fsub_rn(1.0f, A[o * STEP_CLS])));
+        }
+        sums[warp][lane] = y;
+    } else if (warp == 6 && lane < N_MASS) {
+        float x = 0.0f;
+#pragma unroll 13
+        for (int o = 0; o < NC; ++o) x = __fadd_rn(x, reach[lane][o]);
+        mass[lane] = x;
+    }
+    float tw = 0.0f, fe = 0.0f;
+    for (int f0 = 0; f0 < d.nf; f0 += STEP_FLOPS) {          // flop sums, in flop order: BTN (4) and BB (5)
+        if (f0) {                                            // further flops of a large subset
+            __syncthreads();
+            stage_flops(f0);
+            copies_done();
+            __syncthreads();
+        }
+        if (warp != 4 && warp != 5) continue;
+        const float* n = nbs + (warp == 4 ? 0 : STEP_FLOPS * STEP_CLS) + lane;
+        const int nf = min(STEP_FLOPS, d.nf - f0);
+#pragma unroll 4
+        for (int f = 0; f < nf; ++f) {
+            const float w = fws[f];
+            tw = __fadd_rn(tw, w);
+            fe = __fadd_rn(fe, __fmul_rn(w, n[f * STEP_CLS]));
+        }
+    }
+    if (warp == 4 || warp == 5) {
+        sums[warp][lane] = fe;
+        if (warp == 4 && lane == 0) wsum = tw;
+    }
+    __syncthreads();
+    if (warp >= 4 || cls >= NC) return;
     const float stack = d.stack, bf = d.bf, dead = d.dead;
     const float jam_pot = __fadd_rn(__fmul_rn(2.0f, stack), dead);
     const float jam_net = __fsub_rn(jam_pot, stack);
@@ -509,108 +764,60 @@ __global__ void k_pf_cfvs(PfDev d) {
     auto jam_value = [&](float eq) {
         return __fsub_rn(__fmul_rn(eq, jam_net), __fmul_rn(__fmul_rn(__fsub_rn(1.0f, eq), bf), stack));
     };
-    const float* root = d.root;
-    const float* A = d.allin;
-    // BTN vs 3-bet jam
-    c3b[cls] = __fmul_rn(-2.1f, bf);
-    float m3 = 0.0f, eqc = 0.0f;
-    for (int o = 0; o < NC; ++o) {
-        const float r = __fmul_rn(root[o], sbd[2 * PAD + o]);
-        m3 = __fadd_rn(m3, r);
-        eqc = __fadd_rn(eqc, __fmul_rn(r, A[cls * NC + o]));
+    auto share = [&](int k, int m) {   // equity sum k over its mass
+        return mass[m] > 1e-7f ? __fdiv_rn(sums[k][lane], mass[m]) : sums[k][lane];
+    };
+    // the flop EV of player k, kept from before when no flop has weight
+    auto flop_ev = [&](int k, float* ev) {
+        const float v = wsum > 0.0f ? __fdiv_rn(sums[4 + k][lane], wsum) : ev[cls];
+        if (wsum > 0.0f) ev[cls] = v;
+        return v;
+    };
+    float C[3];
+    if (warp == 0) {            // BTN root
+        const float c30 = __fmul_rn(-2.1f, bf), c31 = jam_value(share(0, M_M3));
+        const float v3 = __fadd_rn(__fmul_rn(s3b[cls], c30), __fmul_rn(s3b[PAD + cls], c31));
+        const float tb = __fadd_rn(__fadd_rn(__fadd_rn(mass[M_FM], mass[M_CM]), mass[M_JM]), 1e-9f);
+        const float toj = __fadd_rn(__fadd_rn(mass[M_FJ], mass[M_CJ]), 1e-9f);
+        const float evj = jam_value(share(3, M_CJ));
+        C[0] = 0.0f;
+        C[1] = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(mass[M_FM], dead), __fmul_rn(mass[M_CM], flop_ev(0, d.evb))),
+                                   __fmul_rn(mass[M_JM], v3)), tb);
+        C[2] = __fdiv_rn(__fadd_rn(__fmul_rn(mass[M_FJ], dead), __fmul_rn(mass[M_CJ], evj)), toj);
+    } else if (warp == 1) {     // BB vs min-raise
+        const float tot3 = __fadd_rn(__fadd_rn(mass[M_BF3], mass[M_BC3]), 1e-9f);
+        const float evsh = jam_value(share(1, M_BC3));
+        C[0] = __fmul_rn(-1.0f, bf);
+        C[1] = flop_ev(1, d.evbb);
+        C[2] = __fdiv_rn(__fadd_rn(__fmul_rn(mass[M_BF3], __fadd_rn(dead, 2.1f)), __fmul_rn(mass[M_BC3], evsh)), tot3);
+    } else if (warp == 2) {     // BTN vs 3-bet jam
+        C[0] = __fmul_rn(-2.1f, bf);
+        C[1] = jam_value(share(0, M_M3));
+        C[2] = 0.0f;
+    } else {                    // BB vs open jam
+        C[0] = __fmul_rn(-1.0f, bf);
+        C[1] = jam_value(share(2, M_MJ));
+        C[2] = 0.0f;
     }
-    if (m3 > 1e-7f) eqc = __fdiv_rn(eqc, m3);
-    c3b[PAD + cls] = jam_value(eqc);
-    const float v3 = __fadd_rn(__fmul_rn(s3b[cls], c3b[cls]), __fmul_rn(s3b[PAD + cls], c3b[PAD + cls]));
-    // BB vs min-raise
-    cbd[cls] = __fmul_rn(-1.0f, bf);
-    cbd[PAD + cls] = d.evbb[cls];
-    float bf3 = 0.0f, bc3 = 0.0f, eqj = 0.0f;
-    for (int o = 0; o < NC; ++o) {
-        const float ro = __fmul_rn(root[o], sbr[PAD + o]);
-        bf3 = __fadd_rn(bf3, __fmul_rn(ro, s3b[o]));
-        bc3 = __fadd_rn(bc3, __fmul_rn(ro, s3b[PAD + o]));
-        eqj = __fadd_rn(eqj, __fmul_rn(__fmul_rn(ro, s3b[PAD + o]), __fsub_rn(1.0f, A[o * NC + cls])));
-    }
-    if (bc3 > 1e-7f) eqj = __fdiv_rn(eqj, bc3);
-    const float tot3 = __fadd_rn(__fadd_rn(bf3, bc3), 1e-9f);
-    const float evsh = jam_value(eqj);
-    cbd[2 * PAD + cls] = __fdiv_rn(__fadd_rn(__fmul_rn(bf3, __fadd_rn(dead, 2.1f)), __fmul_rn(bc3, evsh)), tot3);
-    // BB vs open jam
-    cbj[cls] = __fmul_rn(-1.0f, bf);
-    float mj = 0.0f, eqo = 0.0f;
-    for (int o = 0; o < NC; ++o) {
-        const float r = __fmul_rn(root[o], sbr[2 * PAD + o]);
-        mj = __fadd_rn(mj, r);
-        eqo = __fadd_rn(eqo, __fmul_rn(r, __fsub_rn(1.0f, A[o * NC + cls])));
-    }
-    if (mj > 1e-7f) eqo = __fdiv_rn(eqo, mj);
-    cbj[PAD + cls] = jam_value(eqo);
-    // BTN root
-    cbr[cls] = 0.0f;
-    float fm = 0.0f, cm = 0.0f, jm = 0.0f;
-    for (int o = 0; o < NC; ++o) {
-        const float r = root[o];
-        fm = __fadd_rn(fm, __fmul_rn(r, sbd[o]));
-        cm = __fadd_rn(cm, __fmul_rn(r, sbd[PAD + o]));
-        jm = __fadd_rn(jm, __fmul_rn(r, sbd[2 * PAD + o]));
-    }
-    const float tb = __fadd_rn(__fadd_rn(__fadd_rn(fm, cm), jm), 1e-9f);
-    cbr[PAD + cls] = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(fm, dead), __fmul_rn(cm, d.evb[cls])), __fmul_rn(jm, v3)), tb);
-    float fj = 0.0f, cj = 0.0f, eo = 0.0f;
-    for (int o = 0; o < NC; ++o) {
-        const float r = root[o];
-        fj = __fadd_rn(fj, __fmul_rn(r, sbj[o]));
-        cj = __fadd_rn(cj, __fmul_rn(r, sbj[PAD + o]));
-        eo = __fadd_rn(eo, __fmul_rn(__fmul_rn(r, sbj[PAD + o]), A[cls * NC + o]));
-    }
-    const float toj = __fadd_rn(__fadd_rn(fj, cj), 1e-9f);
-    if (cj > 1e-7f) eo = __fdiv_rn(eo, cj);
-    const float evj = jam_value(eo);
-    cbr[2 * PAD + cls] = __fdiv_rn(__fadd_rn(__fmul_rn(fj, dead), __fmul_rn(cj, evj)), toj);
-}
-
-// kernel_dcfr_step (:387-410) for the four nodes, then the next iteration.
-__global__ void k_pf_dcfr(PfDev d) {
-    const int cls = threadIdx.x, node = blockIdx.x;
-    if (cls >= NC) return;
-    const int t = *d.iter;
-    const float wp = d.tab[2 * (t - 1)], ws = d.tab[2 * (t - 1) + 1];
-    const int A = node_actions(node), off = node_off(node);
-    float* R = d.R + off;
-    float* G = d.G + off;
-    float* S = d.S + off;
-    const float* C = d.C + off;
+    const int A = node_actions(warp), off = node_off(warp);
+    const float* g = G + off;
     float v = 0.0f;
-    for (int a = 0; a < A; ++a) v = __fadd_rn(v, __fmul_rn(G[a * PAD + cls], C[a * PAD + cls]));
-    float pos = 0.0f, nxt[3] = {0.0f, 0.0f, 0.0f};
-    for (int a = 0; a < A; ++a) {
-        const int i = a * PAD + cls;
-        const float nr = __fmul_rn(wp, fmaxf(0.0f, __fadd_rn(R[i], __fsub_rn(C[i], v))));
-        R[i] = nr;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) if (a < A) v = __fadd_rn(v, __fmul_rn(g[a * PAD + cls], C[a]));
+    float pos = 0.0f, nxt[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (a >= A) continue;
+        const int i = off + a * PAD + cls;
+        const float nr = __fmul_rn(wp, fmaxf(0.0f, __fadd_rn(Rc[a], __fsub_rn(C[a], v))));
+        d.R[i] = nr;
         pos = __fadd_rn(pos, nr);
         nxt[a] = nr;
-        S[i] = __fadd_rn(S[i], __fmul_rn(__fmul_rn(ws, d.root[cls]), G[i]));
+        d.S[i] = __fadd_rn(Sc[a], __fmul_rn(__fmul_rn(ws, root[cls]), g[a * PAD + cls]));
     }
-    for (int a = 0; a < A; ++a) G[a * PAD + cls] = pos > 1e-7f ? __fdiv_rn(nxt[a], pos) : __fdiv_rn(1.0f, (float)A);
-}
-
-__global__ void k_pf_next(PfDev d) {
-    if (threadIdx.x == 0) *d.iter += 1;
-}
-
-static int pf_iteration(const PfDev& d, cudaStream_t st) {
-    k_pf_reach<<<1, PAD, 0, st>>>(d);
-    MTT_CHECK_LAUNCH();
-    k_pf_cosolve<<<NC, 128, 0, st>>>(d);
-    MTT_CHECK_LAUNCH();
-    k_pf_cfvs<<<1, PAD, 0, st>>>(d);
-    MTT_CHECK_LAUNCH();
-    k_pf_dcfr<<<4, PAD, 0, st>>>(d);
-    MTT_CHECK_LAUNCH();
-    k_pf_next<<<1, 32, 0, st>>>(d);
-    MTT_CHECK_LAUNCH();
-    return MTT_OK;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        if (a < A) d.Gn[off + a * PAD + cls] = pos > 1e-7f ? __fdiv_rn(nxt[a], pos) : __fdiv_rn(1.0f, (float)A);
 }
 
 }  // namespace pf
@@ -621,53 +828,34 @@ extern "C" int mtt_pf_dcfr(const float* d_flop_weights, const float* d_class_mat
     if (!d_flop_weights || !d_class_mats || n_flops < 1 || !d_allin || !p || p->iters < 0 || !d_sums)
         return MTT_ERR_INVALID;
     cudaStream_t st = as_stream(stream);
-    const int iters = std::max(p->iters, 1);
-    std::vector<float> tab(2 * (size_t)iters);
-    for (int t = 1; t <= iters; ++t) {   // host powf, as the reference's loop (:589-591)
-        const float tf = (float)t;
-        tab[2 * (t - 1)] = powf(tf, 1.5f) / (powf(tf, 1.5f) + 1.0f);
-        tab[2 * (t - 1) + 1] = tf * tf;
-    }
     float* buf = nullptr;
-    int* d_iter = nullptr;
-    const size_t nbuf = 2 * (size_t)iters + 4 * (size_t)STATE + 5 * (size_t)PAD;
-    MTT_TRY(scratch_alloc(reinterpret_cast<void**>(&buf), sizeof(float) * nbuf, st));
-    int s = scratch_alloc(reinterpret_cast<void**>(&d_iter), sizeof(int), st);
+    const size_t nf = (size_t)n_flops;
+    MTT_TRY_CUDA(cudaFuncSetAttribute(k_pf_cosolve, cudaFuncAttributeMaxDynamicSharedMemorySize, COSOLVE_SMEM));
+    MTT_TRY_CUDA(cudaFuncSetAttribute(k_pf_step, cudaFuncAttributeMaxDynamicSharedMemorySize, STEP_SMEM));
+    MTT_TRY(scratch_alloc(&buf, 4 * (size_t)STATE + 3 * (size_t)PAD + 2 * nf * PAD + nf * MAT + (size_t)STEP_TILES * STEP_JAM,
+                          st));
     PfDev d{};
-    d.fw = d_flop_weights; d.mats = d_class_mats; d.allin = d_allin;
-    d.tab = buf;
-    d.R = buf + 2 * (size_t)iters; d.G = d.R + STATE; d.S = d.G + STATE; d.C = d.S + STATE;
-    d.root = d.C + STATE; d.rbc = d.root + PAD; d.rbb = d.rbc + PAD; d.evb = d.rbb + PAD; d.evbb = d.evb + PAD;
-    d.iter = d_iter;
+    d.fw = d_flop_weights;
+    d.R = buf; d.G = d.R + STATE; d.Gn = d.G + STATE; d.S = d.Gn + STATE;
+    d.root = d.S + STATE; d.evb = d.root + PAD; d.evbb = d.evb + PAD;
+    d.nb = d.evbb + PAD; d.nbb = d.nb + nf * PAD;
+    float* const om = d.nbb + nf * PAD;       // every part before it is a multiple of 64 floats
+    float* const oj = om + nf * MAT;
+    d.mats = om; d.jam = oj;
     d.nf = n_flops; d.stack = p->stack_bb; d.bf = p->bubble; d.dead = p->dead_pot;
-    if (!s) s = cuda_status(cudaMemcpyAsync(buf, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, st));
-    if (!s) s = cuda_status(cudaMemsetAsync(d.evb, 0, sizeof(float) * 2 * PAD, st));
-    if (!s) { k_pf_init<<<(STATE + 255) / 256, 256, 0, st>>>(d); s = cuda_status(cudaGetLastError()); }
-    // one iteration captured as a graph, replayed p->iters times
-    cudaGraphExec_t ge = nullptr;
-    if (!s && p->iters > 0) {
-        cudaStream_t cs;
-        s = cuda_status(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-        if (!s) {
-            cudaGraph_t g = nullptr;
-            s = cuda_status(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-            if (!s) s = pf_iteration(d, cs);
-            const int s2 = cuda_status(cudaStreamEndCapture(cs, &g));
-            if (!s) s = s2;
-            if (!s) s = cuda_status(cudaGraphInstantiate(&ge, g, 0));
-            if (g) cudaGraphDestroy(g);
-            cudaStreamDestroy(cs);
-        }
-        for (int t = 0; t < p->iters && !s; ++t) s = cuda_status(cudaGraphLaunch(ge, st));
+    k_pf_init<<<ceil_div(STATE, 256), 256, 0, st>>>(d);
+    k_pf_layout<<<592, 256, 0, st>>>(d_class_mats, d_allin, n_flops, om, oj);
+    int s = cuda_status(cudaGetLastError());
+    for (int t = 1; t <= p->iters && !s; ++t) {
+        const float tf = (float)t;   // host powf, as the reference's loop (:589-591)
+        const float wp = powf(tf, 1.5f) / (powf(tf, 1.5f) + 1.0f), ws = tf * tf;
+        s = cuda_status(launch_pdl(k_pf_cosolve, (unsigned)n_flops, 2 * PAD, COSOLVE_SMEM, st, t > 1, d));
+        if (!s) s = cuda_status(launch_pdl(k_pf_step, (unsigned)STEP_TILES, STEP_THREADS, STEP_SMEM, st, true, d, wp, ws));
+        std::swap(d.G, d.Gn);
     }
     if (!s) s = cuda_status(cudaMemcpyAsync(d_sums, d.S, sizeof(float) * STATE, cudaMemcpyDeviceToDevice, st));
     if (!s && d_sigma) s = cuda_status(cudaMemcpyAsync(d_sigma, d.G, sizeof(float) * STATE, cudaMemcpyDeviceToDevice, st));
-    if (ge) {
-        cudaStreamSynchronize(st);
-        cudaGraphExecDestroy(ge);
-    }
     cudaFreeAsync(buf, st);
-    cudaFreeAsync(d_iter, st);
     return s;
 }
 
