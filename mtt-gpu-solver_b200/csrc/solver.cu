@@ -59,10 +59,31 @@ __device__ __forceinline__ void pf_l2(const void* p) {
 __device__ __forceinline__ float4 max04(float4 a) {
     return make_float4(fmaxf(a.x, 0.f), fmaxf(a.y, 0.f), fmaxf(a.z, 0.f), fmaxf(a.w, 0.f));
 }
-__device__ __forceinline__ float rm1(float pos, float sum, float invA) { return sum > 1e-7f ? __fdiv_rn(pos, sum) : invA; }
+// Regret matching: pos / sum, or uniform where nothing is positive.  A zero
+// numerator would take the division's long special-case path, and under CFR+
+// a large share of the regrets is exactly 0, so those skip the division (the
+// quotient is 0 either way).  rm1 divides in line with the zeros replaced,
+// rm1b branches around the division: on the 1,024-subgame river batch the
+// forward levels took 224 -> 167 us (175 with rm1b) and the backward levels
+// 566 -> 515 us (543 with rm1, whose temporaries spill there).
+__device__ __forceinline__ float rm1(float pos, float sum, float invA) {
+    const bool some = sum > 1e-7f, in = pos > 0.f;
+    const float d = some ? sum : 1.f;
+    const float q = __fdiv_rn(in ? pos : d, d);
+    return some ? (in ? q : 0.f) : invA;
+}
+__device__ __forceinline__ float rm1b(float pos, float sum, float invA) {
+    float q = sum > 1e-7f ? 0.f : invA;
+    if (sum > 1e-7f && pos > 0.f) q = __fdiv_rn(pos, sum);
+    return q;
+}
 __device__ __forceinline__ float4 rm4(float4 pos, float4 sum, float invA) {
     return make_float4(rm1(pos.x, sum.x, invA), rm1(pos.y, sum.y, invA), rm1(pos.z, sum.z, invA),
                        rm1(pos.w, sum.w, invA));
+}
+__device__ __forceinline__ float4 rm4b(float4 pos, float4 sum, float invA) {
+    return make_float4(rm1b(pos.x, sum.x, invA), rm1b(pos.y, sum.y, invA), rm1b(pos.z, sum.z, invA),
+                       rm1b(pos.w, sum.w, invA));
 }
 __device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) {
     return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
@@ -92,7 +113,7 @@ struct SolveDev {
     double* darena;
     double* results;
     const float* iter_tab;
-    int* iter;          // device iteration counter, 1-based
+    int* iter;          // [0]: iteration counter, 1-based; [1]: CTAs done (k_tree); [2]: last iteration of the run
     int* err;           // bit 0: a bounded wait for a bulk copy gave up
     int algo, semantics;
     int span;           // float4 hand groups per sweep work item / 32 (hands per warp / 128)
@@ -581,22 +602,26 @@ static_assert(sizeof(FwdItem) == 64 && sizeof(BwdItem) == 64 && sizeof(TermItem)
 enum { FI_REACH = 1, FI_SUMS = 2, FI_CHANCE = 4 };
 enum { BI_UPDATE = 1, BI_SUMS = 2, BI_CHANCE = 4, BI_NEG = 8 };
 
-__global__ void k_init(SolveDev a, int n_sub) {
-    const int s = blockIdx.x;
-    if (s == 0 && threadIdx.x == 0) { *a.iter = 1; *a.err = 0; }
-    if (s >= n_sub) return;
-    const SubDesc sd = a.desc[s];
-    const long long n0 = (long long)sd.rows0 * sd.Hp0 / 4, n1 = (long long)sd.rows1 * sd.Hp1 / 4;
-    float4* r0 = reinterpret_cast<float4*>(a.R + sd.rs_base0);
-    float4* r1 = reinterpret_cast<float4*>(a.R + sd.rs_base1);
-    float4* s0 = reinterpret_cast<float4*>(a.S + sd.rs_base0);
-    float4* s1 = reinterpret_cast<float4*>(a.S + sd.rs_base1);
-    for (long long i = threadIdx.x; i < n0; i += blockDim.x) { r0[i] = f4(0.f); s0[i] = f4(0.f); }
-    for (long long i = threadIdx.x; i < n1; i += blockDim.x) { r1[i] = f4(0.f); s1[i] = f4(0.f); }
-    const int HS4 = (sd.Hp0 + sd.Hp1) >> 2;
-    const float4* rg = reinterpret_cast<const float4*>(a.ranges + sd.range_base);
-    float4* rr = reinterpret_cast<float4*>(a.arena + sd.arena_base);
-    for (int i = threadIdx.x; i < HS4; i += blockDim.x) rr[i] = rg[i];
+// Zero regrets and strategy sums (n4 float4 each, all subgames) by every
+// block, and the root reach of subgame blockIdx.x, ... : one block per subgame
+// zeroed a 104,463-node turn tree's 0.9 GB alone, in 14.5 ms.
+__global__ void k_init(SolveDev a, int n_sub, long long n4) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.iter[0] = 1; a.iter[1] = 0; *a.err = 0; }
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    float4* r = reinterpret_cast<float4*>(a.R);
+    float4* z = reinterpret_cast<float4*>(a.S);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) { r[i] = f4(0.f); z[i] = f4(0.f); }
+    for (int s = blockIdx.x; s < n_sub; s += gridDim.x) {
+        const SubDesc& sd = a.desc[s];
+        const int HS4 = (sd.Hp0 + sd.Hp1) >> 2;
+        const float4* rg = reinterpret_cast<const float4*>(a.ranges + sd.range_base);
+        float4* rr = reinterpret_cast<float4*>(a.arena + sd.arena_base);
+        for (int i = threadIdx.x; i < HS4; i += blockDim.x) rr[i] = rg[i];
+    }
+}
+// Blocks of k_init: 16 float4 of each array a thread, 8 blocks of 256 an SM at most.
+static unsigned init_blocks(int n_sub, long long n4) {
+    return (unsigned)std::max<long long>(1, std::min<long long>(8 * 148, std::max<long long>(n_sub, n4 / (256 * 16) + 1)));
 }
 
 __global__ void k_next_iter(SolveDev a) {
@@ -1010,7 +1035,7 @@ __device__ __forceinline__ void k_bwd_group(const SolveDev& a, const BwdItem& it
             const float4 wr = mul4(r, f4(w_lin));
             float4* Sb = reinterpret_cast<float4*>(a.S + it.rows);
             for (int k = 0; k < A; ++k) {
-                const float4 sg = rm4(max04(Rb[(size_t)k * H4 + g]), sum, invA);
+                const float4 sg = rm4b(max04(Rb[(size_t)k * H4 + g]), sum, invA);
                 v = fma4(sg, qc[(size_t)k * HS4 + g], v);
                 float4 sv = Sb[(size_t)k * H4 + g];
                 sv = dcfr ? fma4(r, sg, mul4(sv, f4(dstr))) : fma4(wr, sg, sv);
@@ -1018,7 +1043,7 @@ __device__ __forceinline__ void k_bwd_group(const SolveDev& a, const BwdItem& it
             }
         } else {
             for (int k = 0; k < A; ++k)
-                v = fma4(rm4(max04(Rb[(size_t)k * H4 + g]), sum, invA), qc[(size_t)k * HS4 + g], v);
+                v = fma4(rm4b(max04(Rb[(size_t)k * H4 + g]), sum, invA), qc[(size_t)k * HS4 + g], v);
         }
         out[g] = v;
         for (int k = 0; k < A; ++k) {
@@ -1059,6 +1084,273 @@ __global__ void __launch_bounds__(256, 5) k_bwd(SolveDev a, const BwdItem* __res
         if (SPAN > 1 && it.g0 + 32 * s >= it.h4) break;
         k_bwd_group<ALGO, SUMS>(a, it, (threadIdx.x & 31) + 32 * s);
     }
+}
+
+// ------------------------------------------------------------- whole-tree sweeps
+// Between two terminal passes every value of a hand depends on that hand
+// alone: its counterfactual values come up the tree from its own terminals,
+// its regrets and strategy follow, and its reach goes down the tree again.  So
+// where a subgame deals no card and its tree is small enough, one CTA takes
+// one player's slice of 8 to 32 hands through the whole tree: it stages the
+// slice's regret and strategy-sum rows, terminal values and reach in shared
+// memory (asynchronous 16-byte copies, all in flight at once), walks the
+// backward levels and then the forward levels of the new strategy there, with
+// a block barrier between levels instead of a launch, and writes every result
+// as it is formed.  An iteration of alternating updates is then four launches
+// (terminals and tree, per player) instead of one per level, kernel class and
+// player: a 39-node spot's iteration took 61.6 us by levels (47.3 once zero
+// regrets skip their divisions) and takes 26.4 us.  Bound by the chain of
+// levels; the arithmetic of a node and hand is that of k_bwd and k_fwd, in the
+// same order, so the results are the same bit for bit.
+struct alignas(16) TreeSeg {   // one player of one subgame
+    long long reach;      // arena float offset of the player's part of node 0's reach slot
+    long long cfv;        // the same in the value region
+    long long rows;       // R/S float offset of the player's rows
+    int h4, hs4;          // float4 groups of the player; slot stride in float4
+    int n_rows, n_nodes;
+    int node0, n_dec;     // decision nodes, in backward order
+    int int0, n_int;      // integers: [nb + 1 backward bounds][nf + 1 forward bounds][own nodes in forward order][terminals]
+    int nb, nf, n_own, n_term;
+    int pad[2];
+};
+static_assert(sizeof(TreeSeg) == 80, "TreeSeg is 80 bytes");
+struct TreeCta {          // one CTA: hands [4 g0, 4 (g0 + G)) of a TreeSeg, G = 1 << lg lanes
+    int seg, g0, lg, pad;
+};
+// A decision node: first child; node | reach id << 16; node whose slot holds
+// the player's reach; actions | acts << 5 | first regret row << 6.  Reach ids
+// number the slots the player writes: 0 the root, 1 + row + k child k of the
+// own node with that first row.
+using TreeNode = int4;
+struct TreeArgs {
+    const TreeCta* ctas;
+    const TreeSeg* segs;
+    const int* ints;
+    const TreeNode* nodes;
+    int n;                // CTAs of all the launches that close the iteration (TR_NEXT)
+    int flags;            // TR_*
+};
+enum { TR_BWD = 1, TR_FWD = 2, TR_LAST = 4, TR_NEXT = 8 };   // TR_LAST: no forward part in the run's last iteration
+constexpr int TREE_THREADS = 256, TREE_MAX_NODES = 1 << 16;
+
+__host__ __device__ inline int tree_smem_bytes(int n_rows, int n_nodes, int n_dec, int n_int, int lg) {
+    return ((3 * n_rows + 1 + n_nodes) << lg) * 16 + n_dec * 16 + (n_int + 3) / 4 * 16;
+}
+
+template <int ALGO>
+__device__ __forceinline__ float4 upd_regret(float4 rk, float4 qk, float4 v, float dpos, float dneg) {
+    if (ALGO == MTT_ALGO_DCFR)
+        return make_float4(dcfr1(rk.x, __fsub_rn(qk.x, v.x), dpos, dneg), dcfr1(rk.y, __fsub_rn(qk.y, v.y), dpos, dneg),
+                           dcfr1(rk.z, __fsub_rn(qk.z, v.z), dpos, dneg), dcfr1(rk.w, __fsub_rn(qk.w, v.w), dpos, dneg));
+    return make_float4(cfrplus1(rk.x, __fsub_rn(qk.x, v.x)), cfrplus1(rk.y, __fsub_rn(qk.y, v.y)),
+                       cfrplus1(rk.z, __fsub_rn(qk.z, v.z)), cfrplus1(rk.w, __fsub_rn(qk.w, v.w)));
+}
+template <int ALGO>
+__device__ __forceinline__ float4 upd_sum(float4 sv, float4 r, float4 wr, float4 sg, float dstr) {
+    return ALGO == MTT_ALGO_DCFR ? fma4(r, sg, mul4(sv, f4(dstr))) : fma4(wr, sg, sv);
+}
+__device__ __forceinline__ void copy_async16(float4* dst, const float4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// One node of one hand group, its rows and child values G float4 apart in
+// shared memory: the acting player's update (returns the node's value) and the
+// reach of its children.  A: the action count, with every row read before any
+// is used, or 0: na actions.
+template <int A, int ALGO, bool SIM>
+__device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, const float4* q, float4 r, float4* R, float4* S,
+                                              int na, int lg, int H4, const float4& tb) {
+    const int n = A ? A : na;
+    const float invA = __fdiv_rn(1.0f, (float)n);
+    const float4 wr = mul4(r, f4(tb.x));
+    float4 sum = f4(0.f), v = f4(0.f);
+    if constexpr (A > 0) {
+        float4 rk[A], qk[A], sg[A];
+#pragma unroll
+        for (int k = 0; k < A; ++k) { rk[k] = rs[k << lg]; qk[k] = q[k << lg]; }
+#pragma unroll
+        for (int k = 0; k < A; ++k) sum = add4(sum, max04(rk[k]));
+#pragma unroll
+        for (int k = 0; k < A; ++k) sg[k] = rm4(max04(rk[k]), sum, invA);
+#pragma unroll
+        for (int k = 0; k < A; ++k) {
+            v = fma4(sg[k], qk[k], v);
+            if (!SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg[k], tb.w);
+        }
+#pragma unroll
+        for (int k = 0; k < A; ++k) {
+            const float4 x = upd_regret<ALGO>(rk[k], qk[k], v, tb.y, tb.z);
+            R[(size_t)k * H4] = x;
+            rs[k << lg] = x;
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) sum = add4(sum, max04(rs[k << lg]));
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) {
+            const float4 sg = rm4(max04(rs[k << lg]), sum, invA);
+            v = fma4(sg, q[k << lg], v);
+            if (!SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg, tb.w);
+        }
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) {
+            const float4 x = upd_regret<ALGO>(rs[k << lg], q[k << lg], v, tb.y, tb.z);
+            R[(size_t)k * H4] = x;
+            rs[k << lg] = x;
+        }
+    }
+    return v;
+}
+
+template <int A, int ALGO, bool SIM>
+__device__ __forceinline__ void tree_reach(const float4* rs, const float4* ss, float4 r, float4* P, float4* ch, float4* S,
+                                           int na, int lg, int H4, int HS4, const float4& tb) {
+    const int n = A ? A : na;
+    const float invA = __fdiv_rn(1.0f, (float)n);
+    const float4 wr = mul4(r, f4(tb.x));
+    float4 sum = f4(0.f);
+    auto put = [&](int k, float4 sg) {
+        const float4 x = mul4(r, sg);
+        P[k << lg] = x;
+        ch[(size_t)k * HS4] = x;
+        if (SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg, tb.w);
+    };
+    if constexpr (A > 0) {
+        float4 rk[A];
+#pragma unroll
+        for (int k = 0; k < A; ++k) rk[k] = max04(rs[k << lg]);
+#pragma unroll
+        for (int k = 0; k < A; ++k) sum = add4(sum, rk[k]);
+#pragma unroll
+        for (int k = 0; k < A; ++k) rk[k] = rm4(rk[k], sum, invA);
+#pragma unroll
+        for (int k = 0; k < A; ++k) put(k, rk[k]);
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) sum = add4(sum, max04(rs[k << lg]));
+#pragma unroll 1
+        for (int k = 0; k < n; ++k) put(k, rm4(max04(rs[k << lg]), sum, invA));
+    }
+}
+
+// SIM: both players are updated from one terminal pass; the strategy sums are
+// then added by the forward part (of the next iteration), else by the backward
+// part.
+template <int ALGO, bool SIM>
+__global__ void __launch_bounds__(TREE_THREADS, 2) k_tree(SolveDev a, TreeArgs t) {
+    extern __shared__ __align__(16) float4 tree_smem[];
+    const TreeCta c = t.ctas[blockIdx.x];
+    const TreeSeg sg = t.segs[c.seg];
+    const int tid = threadIdx.x, lg = c.lg, G = 1 << lg, groups = TREE_THREADS >> lg;
+    const int lane = tid & (G - 1), grp = tid >> lg, g = c.g0 + lane;
+    const int H4 = sg.h4, HS4 = sg.hs4, n_rows = sg.n_rows;
+    const bool live = g < H4;
+    float4* const Rs = tree_smem + lane;                              // regret rows
+    float4* const Ss = Rs + (n_rows << lg);                           // strategy sums
+    float4* const V = Ss + (n_rows << lg);                            // values by node
+    float4* const P = V + (sg.n_nodes << lg);                         // reach by id
+    TreeNode* const nodes = reinterpret_cast<TreeNode*>(tree_smem + ((3 * n_rows + 1 + sg.n_nodes) << lg));
+    int* const blev = reinterpret_cast<int*>(nodes + sg.n_dec);
+    int* const flev = blev + sg.nb + 1;
+    int* const own = flev + sg.nf + 1;
+    int* const term = own + sg.n_own;
+    for (int i = tid; i < sg.n_dec; i += TREE_THREADS) nodes[i] = t.nodes[sg.node0 + i];
+    for (int i = tid; i < sg.n_int; i += TREE_THREADS) blev[i] = t.ints[sg.int0 + i];
+    float4* const reach = reinterpret_cast<float4*>(a.arena + sg.reach) + g;
+    float4* const cfv = reinterpret_cast<float4*>(a.arena + sg.cfv) + g;
+    float4* const R = reinterpret_cast<float4*>(a.R + sg.rows) + g;
+    float4* const S = reinterpret_cast<float4*>(a.S + sg.rows) + g;
+    __syncthreads();
+    // the tree's description is written once, before any solve; all else
+    // belongs to the kernels before
+    grid_dep_trigger();
+    grid_dep_wait();
+    const int iter = a.iter[0];
+    const bool bwd = t.flags & TR_BWD;
+    const bool fwd = (t.flags & TR_FWD) && !((t.flags & TR_LAST) && iter >= a.iter[2]);
+    if (live) {
+        for (int i = grp; i < n_rows; i += groups) {
+            copy_async16(Rs + (i << lg), R + (size_t)i * H4);
+            if (SIM ? fwd : bwd) copy_async16(Ss + (i << lg), S + (size_t)i * H4);
+        }
+        if (bwd)
+            for (int i = grp; i < sg.n_term; i += groups)
+                copy_async16(V + (term[i] << lg), cfv + (size_t)term[i] * HS4);
+        if (bwd && !SIM) {
+            for (int i = grp; i < sg.n_own; i += groups) {
+                const TreeNode nd = nodes[own[i]];
+                copy_async16(P + ((int)((unsigned)nd.y >> 16) << lg), reach + (size_t)nd.z * HS4);
+            }
+        } else if (grp == 0) {
+            copy_async16(P, reach);
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (bwd) {
+        const float4 tb = *reinterpret_cast<const float4*>(a.iter_tab + 4 * (size_t)(iter - 1));
+        for (int l = 0; l < sg.nb; ++l) {
+            const int hi = blev[l + 1];
+            for (int i = blev[l] + grp; live && i < hi; i += groups) {
+                const TreeNode nd = nodes[i];
+                const int na = nd.w & 31, self = nd.y & 0xFFFF;
+                const float4* const q = V + (nd.x << lg);
+                float4 v = f4(0.f);
+                if (nd.w & 32) {
+                    const int row = (int)((unsigned)nd.w >> 6);
+                    const float4 r = SIM ? f4(0.f) : P[(int)((unsigned)nd.y >> 16) << lg];
+#define TREE_CALL(A) \
+    v = tree_update<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), q, r, R + (size_t)row * H4, S + (size_t)row * H4, na, lg, \
+                                  H4, tb)
+                    switch (na) {
+                        case 2: TREE_CALL(2); break;
+                        case 3: TREE_CALL(3); break;
+                        case 4: TREE_CALL(4); break;
+                        default: TREE_CALL(0); break;
+                    }
+#undef TREE_CALL
+                } else {
+#pragma unroll 4
+                    for (int k = 0; k < na; ++k) v = add4(v, q[k << lg]);
+                }
+                V[self << lg] = v;
+                cfv[(size_t)self * HS4] = v;
+            }
+            __syncthreads();
+        }
+    }
+    if (fwd) {
+        // the sums of simultaneous updates are weighted by the iteration they open
+        const float4 tb = SIM ? *reinterpret_cast<const float4*>(a.iter_tab + 4 * (size_t)(iter - (bwd ? 0 : 1))) : f4(0.f);
+        for (int l = 0; l < sg.nf; ++l) {
+            const int hi = flev[l + 1];
+            for (int i = flev[l] + grp; live && i < hi; i += groups) {
+                const TreeNode nd = nodes[own[i]];
+                const int na = nd.w & 31, row = (int)((unsigned)nd.w >> 6);
+                const float4 r = P[(int)((unsigned)nd.y >> 16) << lg];
+#define TREE_CALL(A) \
+    tree_reach<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), r, P + ((1 + row) << lg), reach + (size_t)nd.x * HS4, \
+                             S + (size_t)row * H4, na, lg, H4, HS4, tb)
+                switch (na) {
+                    case 2: TREE_CALL(2); break;
+                    case 3: TREE_CALL(3); break;
+                    case 4: TREE_CALL(4); break;
+                    default: TREE_CALL(0); break;
+                }
+#undef TREE_CALL
+            }
+            if (l + 1 < sg.nf) __syncthreads();
+        }
+    }
+    // the last CTA of the closing launches opens the next iteration: every CTA has read this one's number
+    if ((t.flags & TR_NEXT) && tid == 0 && atomicAdd(a.iter + 1, 1) == t.n - 1) {
+        a.iter[1] = 0;
+        a.iter[0] = iter + 1;
+    }
+}
+
+__global__ void k_set_last(SolveDev a, int last) {
+    if (threadIdx.x == 0) a.iter[2] = last;
 }
 
 // ------------------------------------------------------------- depth-limit leaves
@@ -1634,11 +1926,21 @@ struct HostLists {
     std::vector<std::vector<Task>> bf, bb;
     std::vector<TermItem> titems;    // by subgame, then table variant
     std::vector<int2> terms;
+    // whole-tree sweeps: two segments per subgame that takes them, with their
+    // subgame, nodes and integers
+    std::vector<TreeSeg> segs;
+    std::vector<int> seg_sub;
+    std::vector<int> ints;
+    std::vector<TreeNode> tnodes;
 };
+
+constexpr int TREE_CLASSES = 3;                      // by shared memory: about 5, 2 and 1 CTAs an SM
+constexpr int TREE_CLASS_BYTES[TREE_CLASSES] = {44 * 1024, 110 * 1024, 224 * 1024};
 
 struct ListSet {
     LevelLists<FwdItem> f_init, f_sim, f_alt[2];
     LevelLists<BwdItem> b_sim, b_alt[2];
+    LevelLists<BwdItem> b_rest;      // b_sim without the subgames of the tree sweeps (where there are some)
     LevelLists<Task> br_fwd, br_bwd;
     TermItem* titems = nullptr;
     long long titems_cap = 0;
@@ -1652,6 +1954,12 @@ struct ListSet {
     int* subs = nullptr;
     long long subs_cap = 0;
     int n_subs = 0;
+    TreeCta* ctas = nullptr;                         // by class, in a class player 0's, then player 1's
+    long long ctas_cap = 0;
+    int n_ctas[TREE_CLASSES][2] = {};
+    int tree_smem[TREE_CLASSES] = {};                // dynamic shared memory of a class's launch
+    bool tree_chain = false;                         // one wave: launches chained across kernel classes
+    bool levels_too = false;                         // some subgame takes the level kernels
 };
 
 }  // namespace mtt
@@ -1679,12 +1987,18 @@ struct mtt_batch {
     float* d_iter_tab = nullptr;
     int iter_cap = 0;
     int levels = 0;
+    std::vector<char> tree;            // subgames that take the whole-tree sweeps
+    bool any_tree = false;
+    TreeSeg* d_segs = nullptr;
+    int* d_ints = nullptr;
+    TreeNode* d_tnodes = nullptr;
     HostLists host;
     ListSet full, act;
     std::vector<SubDesc> desc;
     std::vector<int> iters_done;
     int max_h = 0;
     long long device_bytes = 0, iter_bytes = 0;
+    long long rs4 = 0;                 // float4 of R (and of S)
     int tuned_threads = 0;
     cudaGraphExec_t gexec = nullptr;   // one iteration over the full lists
     int gkernels = 0;                  // kernel nodes in gexec
@@ -1758,7 +2072,7 @@ static void free_set(ListSet& L) {
     dfree(L.f_init.d); dfree(L.f_sim.d); dfree(L.b_sim.d);
     for (int u = 0; u < 2; ++u) { dfree(L.f_alt[u].d); dfree(L.b_alt[u].d); }
     dfree(L.br_fwd.d); dfree(L.br_bwd.d); dfree(L.titems); dfree(L.terms); dfree(L.subs);
-    dfree(L.tgroups);
+    dfree(L.tgroups); dfree(L.ctas); dfree(L.b_rest.d);
 }
 
 // Waits for the batch's own work (the events of the streams it ran on; its
@@ -1778,7 +2092,7 @@ static void free_batch(mtt_batch* b) {
     dfree(b->d_ranges); dfree(b->d_arena); dfree(b->d_R); dfree(b->d_S);
     dfree(b->d_darena); dfree(b->d_results); dfree(b->d_iter);
     dfree(b->d_iter_tab);
-    dfree(b->d_err);
+    dfree(b->d_err); dfree(b->d_segs); dfree(b->d_ints); dfree(b->d_tnodes);
     dfree(b->d_leaves); dfree(b->d_lx); dfree(b->d_ly); dfree(b->d_lm); dfree(b->d_lsd);
     free_set(b->full);
     free_set(b->act);
@@ -1837,6 +2151,119 @@ static int upload_levels(LevelLists<T>& L, const std::vector<std::vector<T>>& lv
     return MTT_OK;
 }
 
+// Shared memory of the smallest slice (8 hands) of one player's tree.
+static int tree_min_bytes(const SubDesc& d, const std::vector<DNode>& nodes, int q) {
+    int dec = 0, own = 0;
+    for (const DNode& nd : nodes) {
+        dec += nd.type == MTT_NODE_DECISION;
+        own += nd.type == MTT_NODE_DECISION && nd.player == q;
+    }
+    // at most one level per node
+    return tree_smem_bytes(q ? d.rows1 : d.rows0, d.n_nodes, dec, 2 * (dec + 1) + own + d.n_nodes - dec, 1);
+}
+
+// One player's view of a chance-free tree: the backward order (all decision
+// nodes, deepest level first) and the forward order (the player's own, by how
+// many of them lie above), each level sorted by role and action count so that
+// a warp's nodes take the same path.
+static void build_tree_seg(const std::vector<DNode>& nodes, const std::vector<int16_t>& depth, const SubDesc& d, int sub,
+                           int q, HostLists& L) {
+    const long long HS = d.Hp0 + d.Hp1, off = q ? d.Hp0 : 0;
+    TreeSeg g{};
+    g.reach = d.arena_base + off;
+    g.cfv = d.arena_base + (long long)d.n_nodes * HS + off;
+    g.rows = q ? d.rs_base1 : d.rs_base0;
+    g.h4 = (q ? d.Hp1 : d.Hp0) / 4;
+    g.hs4 = (int)(HS / 4);
+    g.n_rows = q ? d.rows1 : d.rows0;
+    g.n_nodes = d.n_nodes;
+    g.node0 = (int)L.tnodes.size();
+    g.int0 = (int)L.ints.size();
+    std::vector<int> above(d.n_nodes, 0), id(d.n_nodes, 0), pos(d.n_nodes, 0), order;
+    for (int k = 0; k < d.n_nodes; ++k) {
+        const DNode& nd = nodes[k];
+        if (nd.type != MTT_NODE_DECISION) continue;
+        const bool own = nd.player == q;
+        for (int c = 0; c < nd.na; ++c) {
+            above[nd.first + c] = above[k] + (own ? 1 : 0);
+            if (own) id[nd.first + c] = 1 + nd.row + c;
+        }
+        order.push_back(k);
+    }
+    auto key = [&](int k) { return (nodes[k].player == q ? 32 : 0) | nodes[k].na; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return depth[x] != depth[y] ? depth[x] > depth[y] : key(x) < key(y);
+    });
+    g.n_dec = (int)order.size();
+    for (int i = 0; i < g.n_dec; ++i) {
+        const int k = order[i];
+        const DNode& nd = nodes[k];
+        if (i == 0 || depth[k] != depth[order[i - 1]]) { L.ints.push_back(i); ++g.nb; }
+        const int src = q ? nd.reach_src1 : nd.reach_src0;
+        const bool own = nd.player == q;
+        L.tnodes.push_back(make_int4(nd.first, (int)((unsigned)k | (unsigned)id[src] << 16), src,
+                                     (int)((unsigned)key(k) | (own ? (unsigned)nd.row << 6 : 0u))));
+        pos[k] = i;
+    }
+    L.ints.push_back(g.n_dec);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return above[x] != above[y] ? above[x] < above[y] : key(x) < key(y);
+    });
+    std::vector<int> own;
+    int last = -1;
+    for (int k : order) {
+        if (nodes[k].player != q) continue;
+        if (above[k] != last) { L.ints.push_back((int)own.size()); ++g.nf; last = above[k]; }
+        own.push_back(pos[k]);
+    }
+    L.ints.push_back((int)own.size());
+    g.n_own = (int)own.size();
+    L.ints.insert(L.ints.end(), own.begin(), own.end());
+    for (int k = 0; k < d.n_nodes; ++k)
+        if (nodes[k].type != MTT_NODE_DECISION) { L.ints.push_back(k); ++g.n_term; }
+    g.n_int = (int)L.ints.size() - g.int0;
+    L.segs.push_back(g);
+    L.seg_sub.push_back(sub);
+}
+
+// The CTAs of the whole-tree sweeps.  A slice is 32 hands (128-byte rows), or
+// 16 or 8 where that lets the tree fit a class of less shared memory and more
+// CTAs an SM; costliest first, so that the last CTAs to start are short.
+static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* active, long long& total) {
+    const HostLists& H = b->host;
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    struct Pick { int seg, lg, bytes; };
+    std::vector<Pick> picks[TREE_CLASSES][2];
+    for (int i = 0; i < (int)H.segs.size(); ++i) {
+        if (active && !(*active)[H.seg_sub[i]]) continue;
+        const TreeSeg& g = H.segs[i];
+        auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg); };
+        int lg = 1, cls = TREE_CLASSES - 1;
+        if (bytes(2) <= TREE_CLASS_BYTES[0]) { cls = 0; lg = bytes(3) <= TREE_CLASS_BYTES[0] ? 3 : 2; }
+        else if (bytes(1) <= TREE_CLASS_BYTES[1]) { cls = 1; lg = bytes(3) <= TREE_CLASS_BYTES[1] ? 3 : bytes(2) <= TREE_CLASS_BYTES[1] ? 2 : 1; }
+        picks[cls][i & 1].push_back(Pick{i, lg, bytes(lg)});
+    }
+    std::vector<TreeCta> ctas;
+    for (int c = 0; c < TREE_CLASSES; ++c) {
+        L.tree_smem[c] = 0;
+        for (int q = 0; q < 2; ++q) {
+            auto& v = picks[c][q];
+            std::stable_sort(v.begin(), v.end(), [](const Pick& x, const Pick& y) { return x.bytes > y.bytes; });
+            const size_t n0 = ctas.size();
+            for (const Pick& x : v) {
+                L.tree_smem[c] = std::max(L.tree_smem[c], x.bytes);
+                for (int g0 = 0; g0 < H.segs[x.seg].h4; g0 += 1 << x.lg) ctas.push_back(TreeCta{x.seg, g0, x.lg, 0});
+            }
+            L.n_ctas[c][q] = (int)(ctas.size() - n0);
+        }
+    }
+    L.tree_chain = (long long)ctas.size() <= 4LL * sms;
+    MTT_TRY(grow(&L.ctas, &L.ctas_cap, (long long)ctas.size(), total));
+    if (!ctas.empty()) MTT_TRY_CUDA(cudaMemcpy(L.ctas, ctas.data(), sizeof(TreeCta) * ctas.size(), cudaMemcpyHostToDevice));
+    return MTT_OK;
+}
+
 static int build_set(mtt_batch* b, ListSet& L, const std::vector<char>* active, long long& total) {
     const HostLists& H = b->host;
     // the host lists hold one item per 32 float4 groups; a span of k keeps
@@ -1847,12 +2274,17 @@ static int build_set(mtt_batch* b, ListSet& L, const std::vector<char>* active, 
     auto tkeep = [&](const Task& x) { return !active || (*active)[x.sub]; };
     const bool all_sweep = !active && span == 1;
     MTT_TRY(upload_levels(L.f_init, H.fi, all_sweep, fkeep, total));
-    MTT_TRY(upload_levels(L.f_sim, H.fsim, all_sweep, fkeep, total));
     MTT_TRY(upload_levels(L.b_sim, H.bsim, all_sweep, bkeep, total));
+    // the iterations' level lists hold the subgames that do not take the tree sweeps
+    if (b->any_tree) MTT_TRY(build_tree_ctas(b, L, active, total));
+    auto brest = [&](const BwdItem& x) { return bkeep(x) && !b->tree[x.sub]; };
+    if (b->any_tree) MTT_TRY(upload_levels(L.b_rest, H.bsim, false, brest, total));
+    MTT_TRY(upload_levels(L.f_sim, H.fsim, all_sweep, fkeep, total));
     for (int u = 0; u < 2; ++u) {
         MTT_TRY(upload_levels(L.f_alt[u], H.fal[u], all_sweep, fkeep, total));
         MTT_TRY(upload_levels(L.b_alt[u], H.bal[u], all_sweep, bkeep, total));
     }
+    L.levels_too = L.f_sim.off.back() > 0;
     MTT_TRY(upload_levels(L.br_fwd, H.bf, !active, tkeep, total));
     MTT_TRY(upload_levels(L.br_bwd, H.bb, !active, tkeep, total));
     std::vector<TermItem> ti;
@@ -2041,8 +2473,48 @@ static TermKernel term_kernel(int upd, int semantics) {
     return k[semantics ? 1 : 0][upd - 1];
 }
 
-static int launch_term(const mtt_batch* b, const ListSet& L, const SolveDev& a, int upd, cudaStream_t st) {
-    bool chained = false;
+using TreeKernel = void (*)(SolveDev, TreeArgs);
+static TreeKernel tree_kernel(int algo, bool sim) {
+    static const TreeKernel k[2][2] = {{k_tree<MTT_ALGO_CFRPLUS, false>, k_tree<MTT_ALGO_CFRPLUS, true>},
+                                       {k_tree<MTT_ALGO_DCFR, false>, k_tree<MTT_ALGO_DCFR, true>}};
+    return k[algo == MTT_ALGO_DCFR ? 1 : 0][sim ? 1 : 0];
+}
+
+// Whole-tree sweeps of the players `upd` (TR_* flags).
+static int launch_tree(const mtt_batch* b, const ListSet& L, const SolveDev& a, int upd, bool sim, int flags, bool chained,
+                       cudaStream_t st) {
+    if (!b->any_tree) return MTT_OK;
+    int n[TREE_CLASSES], all = 0;
+    for (int c = 0; c < TREE_CLASSES; ++c) {
+        n[c] = (upd & 1 ? L.n_ctas[c][0] : 0) + (upd & 2 ? L.n_ctas[c][1] : 0);
+        all += n[c];
+    }
+    TreeArgs t;
+    t.segs = b->d_segs;
+    t.ints = b->d_ints;
+    t.nodes = b->d_tnodes;
+    t.n = all;
+    t.flags = flags;
+    const TreeCta* first = L.ctas;
+    for (int c = 0; c < TREE_CLASSES; ++c) {
+        t.ctas = first + (upd == 2 ? L.n_ctas[c][0] : 0);
+        first += L.n_ctas[c][0] + L.n_ctas[c][1];
+        if (!n[c]) continue;
+        MTT_TRY_CUDA(launch_pdl(tree_kernel(a.algo, sim), (unsigned)n[c], TREE_THREADS, L.tree_smem[c], st, chained, a, t));
+        MTT_CHECK_LAUNCH();
+        ++b->launches;
+        chained = true;
+    }
+    if (!all && (flags & TR_NEXT)) {   // no hands on this side
+        k_next_iter<<<1, 32, 0, st>>>(a);
+        MTT_CHECK_LAUNCH();
+        ++b->launches;
+    }
+    return MTT_OK;
+}
+
+static int launch_term(const mtt_batch* b, const ListSet& L, const SolveDev& a, int upd, cudaStream_t st,
+                       bool chained = false) {
     for (size_t k = 0; k < L.tb_start.size(); ++k) {
         if (L.tb_count[k] == 0) continue;
         const int smem = upd == 3 ? L.tb_smem3[k] : L.tb_smem1[k];
@@ -2087,23 +2559,49 @@ static int launch_leaves(const mtt_batch* b, const SolveDev& a, int upd, cudaStr
 // One CFR iteration: per pass forward levels, leaves, terminals, backward levels.
 static int launch_iteration(const mtt_batch* b, const ListSet& L, const SolveDev& a, const mtt_solve_params& p,
                             int threads, cudaStream_t st) {
+    // Subgames of the tree sweeps: the reach of the first pass is in place
+    // (launch_tree_start or the iteration before), and the run's last iteration
+    // leaves out the forward part that would open another.
+    if (b->any_tree && !L.levels_too) {
+        const bool ch = L.tree_chain;
+        if (p.alternate) {
+            MTT_TRY(launch_term(b, L, a, 1, st, ch));
+            MTT_TRY(launch_tree(b, L, a, 1, false, TR_BWD | TR_FWD, ch, st));
+            MTT_TRY(launch_term(b, L, a, 2, st, ch));
+            return launch_tree(b, L, a, 2, false, TR_BWD | TR_FWD | TR_LAST | TR_NEXT, ch, st);
+        }
+        MTT_TRY(launch_term(b, L, a, 3, st, ch));
+        return launch_tree(b, L, a, 3, true, TR_BWD | TR_FWD | TR_LAST | TR_NEXT, ch, st);
+    }
     if (p.alternate) {
         for (int u = 0; u < 2; ++u) {
             MTT_TRY(launch_levels_fwd(b, a, L.f_alt[u], threads, false, st));
             MTT_TRY(launch_leaves(b, a, 1 << u, st));
             MTT_TRY(launch_term(b, L, a, 1 << u, st));
+            MTT_TRY(launch_tree(b, L, a, 1 << u, false, TR_BWD | TR_FWD | (u ? TR_LAST : 0), false, st));
             MTT_TRY(launch_levels_bwd(b, a, L.b_alt[u], threads, true, st));
         }
     } else {
         MTT_TRY(launch_levels_fwd(b, a, L.f_sim, threads, true, st));
         MTT_TRY(launch_leaves(b, a, 3, st));
         MTT_TRY(launch_term(b, L, a, 3, st));
-        MTT_TRY(launch_levels_bwd(b, a, L.b_sim, threads, false, st));
+        MTT_TRY(launch_tree(b, L, a, 3, true, TR_BWD | TR_FWD | TR_LAST, false, st));
+        MTT_TRY(launch_levels_bwd(b, a, b->any_tree ? L.b_rest : L.b_sim, threads, false, st));
     }
     k_next_iter<<<1, 32, 0, st>>>(a);
     MTT_CHECK_LAUNCH();
     ++b->launches;
     return MTT_OK;
+}
+
+// Before a run of whole-tree iterations up to iteration `last`: the forward
+// part of its first pass.
+static int launch_tree_start(const mtt_batch* b, const ListSet& L, const SolveDev& a, const mtt_solve_params& p, int last,
+                             cudaStream_t st) {
+    k_set_last<<<1, 32, 0, st>>>(a, last);
+    MTT_CHECK_LAUNCH();
+    ++b->launches;
+    return launch_tree(b, L, a, p.alternate ? 2 : 3, !p.alternate, TR_FWD, false, st);
 }
 
 static int launch_br(const mtt_batch* b, const ListSet& L, const SolveDev& a, int threads, cudaStream_t st) {
@@ -2145,6 +2643,12 @@ static int set_smem_attrs(const mtt_batch* b, const ListSet& L) {
         MTT_TRY_CUDA(cudaFuncSetAttribute(k_br_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t));
     }
     int tmax = 0;
+    int trmax = 0;
+    for (int v : L.tree_smem) trmax = std::max(trmax, v);
+    if (trmax > 48 * 1024)
+        for (int algo : {MTT_ALGO_CFRPLUS, MTT_ALGO_DCFR})
+            for (int sim = 0; sim < 2; ++sim)
+                MTT_TRY_CUDA(cudaFuncSetAttribute(tree_kernel(algo, sim != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, trmax));
     for (int v : L.tb_smem1) tmax = std::max(tmax, v);
     for (int v : L.tb_smem3) tmax = std::max(tmax, v);
     if (tmax > 48 * 1024) {
@@ -2186,8 +2690,10 @@ static int capture_iteration(const mtt_batch* b, const ListSet& L, const SolveDe
     return s;
 }
 
+// Iterations first .. first + iters - 1 of a solve.
 static int run_iterations(mtt_batch* b, const ListSet& L, const SolveDev& a, const mtt_solve_params& p, int threads,
-                          int iters, bool graph, bool cached, cudaStream_t st) {
+                          int first, int iters, bool graph, bool cached, cudaStream_t st) {
+    if (b->any_tree && iters > 0) MTT_TRY(launch_tree_start(b, L, a, p, first + iters - 1, st));
     if (!graph) {
         for (int t = 0; t < iters; ++t) MTT_TRY(launch_iteration(b, L, a, p, threads, st));
         return MTT_OK;
@@ -2229,11 +2735,11 @@ static int run_solve(mtt_batch* b, const mtt_solve_params& p, cudaStream_t st, b
     MTT_TRY(set_smem_attrs(b, b->full));
     MTT_TRY(fill_iter_table(b, p, gate ? p.max_iters : p.iters, st));
     const SolveDev a = dev_args(b, p);
-    k_init<<<b->n, 256, 0, st>>>(a, b->n);
+    k_init<<<init_blocks(b->n, b->rs4), 256, 0, st>>>(a, b->n, b->rs4);
     MTT_CHECK_LAUNCH();
     ++b->launches;
     MTT_TRY(launch_levels_fwd(b, a, b->full.f_init, threads, false, st));
-    MTT_TRY(run_iterations(b, b->full, a, p, threads, p.iters, graph, true, st));
+    MTT_TRY(run_iterations(b, b->full, a, p, threads, 1, p.iters, graph, true, st));
     std::fill(b->iters_done.begin(), b->iters_done.end(), p.iters);
     if (p.exploitability) MTT_TRY(launch_br(b, b->full, a, threads, st));
     if (!gate) return MTT_OK;
@@ -2253,7 +2759,7 @@ static int run_solve(mtt_batch* b, const mtt_solve_params& p, cudaStream_t st, b
         MTT_TRY(build_set(b, b->act, &active, scratch));
         MTT_TRY(set_smem_attrs(b, b->act));
         const int it = std::min(chunk, p.max_iters - done);
-        MTT_TRY(run_iterations(b, b->act, a, p, threads, it, graph, false, st));
+        MTT_TRY(run_iterations(b, b->act, a, p, threads, done + 1, it, graph, false, st));
         for (int i = 0; i < b->n; ++i) if (active[i]) b->iters_done[i] += it;
         done += it;
         MTT_TRY(launch_br(b, b->act, a, threads, st));
@@ -2313,18 +2819,26 @@ static int mtt_batch_kernel_profile_impl(mtt_batch* b, const mtt_solve_params* p
     if (!gr.empty())
         MTT_TRY_CUDA(cudaMemcpy(gr.data(), L.tgroups, sizeof(TermGroup) * gr.size(), cudaMemcpyDeviceToHost));
     if (p.alternate) {
-        for (int u = 0; u < 2; ++u) {
-            for (const auto& lv : HL.fal[u]) for (const FwdItem& it : lv) bf += fwd_item_bytes(it, b->span);
-            for (const auto& lv : HL.bal[u]) for (const BwdItem& it : lv) bb += bwd_item_bytes(it, b->span);
-            bt += term_launch_bytes(L, gr, HL.titems, 1 << u);
-        }
+        // both passes together hold every node once per direction; the acting
+        // player's backward items also add its strategy sums
+        for (const auto& lv : HL.fi) for (const FwdItem& it : lv) bf += fwd_item_bytes(it, b->span);
+        for (const auto& lv : HL.bsim)
+            for (BwdItem it : lv) {
+                if (it.flags & BI_UPDATE) it.flags |= BI_SUMS;
+                bb += bwd_item_bytes(it, b->span);
+            }
+        for (int u = 0; u < 2; ++u) bt += term_launch_bytes(L, gr, HL.titems, 1 << u);
     } else {
-        for (const auto& lv : HL.fsim) for (const FwdItem& it : lv) bf += fwd_item_bytes(it, b->span);
+        for (const auto& lv : HL.fi)
+            for (FwdItem it : lv) {
+                if (!(it.flags & FI_CHANCE)) it.flags |= FI_SUMS;
+                bf += fwd_item_bytes(it, b->span);
+            }
         for (const auto& lv : HL.bsim) for (const BwdItem& it : lv) bb += bwd_item_bytes(it, b->span);
         bt += term_launch_bytes(L, gr, HL.titems, 3);
     }
     h_bytes[0] = bf; h_bytes[1] = bt; h_bytes[2] = bb;
-    k_init<<<b->n, 256, 0, st>>>(a, b->n);
+    k_init<<<init_blocks(b->n, b->rs4), 256, 0, st>>>(a, b->n, b->rs4);
     MTT_CHECK_LAUNCH();
     ++b->launches;
     MTT_TRY(launch_levels_fwd(b, a, L.f_init, threads, false, st));
@@ -2338,14 +2852,16 @@ static int mtt_batch_kernel_profile_impl(mtt_batch* b, const mtt_solve_params* p
         for (int u = 0; u < passes && !s; ++u) {
             cudaEvent_t* e = ev.data() + 6 * u;
             const LevelLists<FwdItem>& F = p.alternate ? L.f_alt[u] : L.f_sim;
-            const LevelLists<BwdItem>& B = p.alternate ? L.b_alt[u] : L.b_sim;
+            const LevelLists<BwdItem>& B = p.alternate ? L.b_alt[u] : b->any_tree ? L.b_rest : L.b_sim;
             s = cuda_status(cudaEventRecord(e[0], st));
+            if (!s) s = launch_tree(b, L, a, p.alternate ? 2 >> u : 3, !p.alternate, TR_FWD, false, st);
             if (!s) s = launch_levels_fwd(b, a, F, threads, !p.alternate, st);
             if (!s) s = cuda_status(cudaEventRecord(e[1], st));
             if (!s) s = cuda_status(cudaEventRecord(e[2], st));
             if (!s) s = launch_term(b, L, a, p.alternate ? 1 << u : 3, st);
             if (!s) s = cuda_status(cudaEventRecord(e[3], st));
             if (!s) s = cuda_status(cudaEventRecord(e[4], st));
+            if (!s) s = launch_tree(b, L, a, p.alternate ? 1 << u : 3, !p.alternate, TR_BWD, false, st);
             if (!s) s = launch_levels_bwd(b, a, B, threads, p.alternate != 0, st);
             if (!s) s = cuda_status(cudaEventRecord(e[5], st));
         }
@@ -2425,7 +2941,28 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
                       16LL * (long long)d.n_nodes * (d.H0 + d.H1);
     }
     b->iter_bytes = iter_bytes;
+    b->rs4 = rs / 4;
     b->levels = levels;
+    // whole-tree sweeps: batches of few hands, whose level launches are bound by
+    // latency; the subgame deals no card, ends in no leaf and a slice of its
+    // tree fits in shared memory.  The line is where the two met on uneven
+    // river batches (us an iteration, tree / level launches): 1 subgame 36 / 63,
+    // 8 (160 slices of 32 hands) 87 / 103, 16 101 / 109, 24 (480) 122 / 124, 32
+    // 134 / 124; larger batches fill the chip level by level, and there the
+    // tree's barriers cost more than the launches.
+    b->tree.assign(n, 0);
+    long long slices = 0;
+    for (int i = 0; i < n; ++i) slices += (std::max(b->desc[i].Hp0, b->desc[i].Hp1) + 31) / 32;
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    for (int i = 0; i < n && slices <= 3LL * sms; ++i) {
+        bool ok = b->desc[i].n_nodes < TREE_MAX_NODES && b->desc[i].rows0 < TREE_MAX_NODES - 1 &&
+                  b->desc[i].rows1 < TREE_MAX_NODES - 1;
+        for (const DNode& nd : packs[i].nodes) ok &= nd.type != MTT_NODE_CHANCE && nd.type != MTT_NODE_LEAF;
+        for (int q = 0; q < 2 && ok; ++q) ok = tree_min_bytes(b->desc[i], packs[i].nodes, q) <= TREE_CLASS_BYTES[TREE_CLASSES - 1];
+        b->tree[i] = ok;
+        b->any_tree |= ok;
+    }
     // FP64 best-response warp tasks, solver work items per level, terminal items
     HostLists& HL = b->host;
     auto init_lists = [levels](HostLists& L) {
@@ -2460,6 +2997,7 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
                 f.sub = i;
                 for (f.g0 = 0; f.g0 < f.h4; f.g0 += 32) {
                     f.flags = FI_REACH; L.fi[dp].push_back(f);
+                    if (b->tree[i]) continue;         // the iterations' level lists leave it out
                     f.flags = FI_REACH | FI_SUMS; L.fsim[dp].push_back(f);
                     // alternating pass u: the opponent's nodes pass reach down; the
                     // acting player's strategy sums are added by its backward items
@@ -2478,6 +3016,7 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
                     for (bw.g0 = 0; bw.g0 < bw.h4; bw.g0 += 32) {
                         bw.flags = q == p ? (BI_UPDATE | (q ? BI_NEG : 0)) : 0;
                         L.bsim[dp].push_back(bw);
+                        if (b->tree[i]) continue;
                         if (q == p) bw.flags = BI_UPDATE | BI_SUMS;
                         L.bal[q][dp].push_back(bw);
                     }
@@ -2611,8 +3150,19 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     }
     for (int t = 0; t < nlt; ++t) b->h_leaves.insert(b->h_leaves.end(), plv[t].begin(), plv[t].end());
     for (size_t k = 0; k < b->h_leaves.size(); ++k) b->h_leaves[k].row0 = LEAF_RIVERS * (int)k;
+    for (int i = 0; i < n; ++i)
+        for (int q = 0; q < 2 && b->tree[i]; ++q) build_tree_seg(packs[i].nodes, packs[i].depth, b->desc[i], i, q, HL);
     long long total = 0;
     int s = MTT_OK;
+    if (b->any_tree) {
+        s = dalloc(&b->d_segs, HL.segs.size(), total);
+        if (!s) s = dalloc(&b->d_ints, HL.ints.size(), total);
+        if (!s) s = dalloc(&b->d_tnodes, HL.tnodes.size(), total);
+        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, HL.segs.data(), sizeof(TreeSeg) * HL.segs.size(), cudaMemcpyHostToDevice));
+        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, HL.ints.data(), sizeof(int) * HL.ints.size(), cudaMemcpyHostToDevice));
+        if (!s && !HL.tnodes.empty())
+            s = cuda_status(cudaMemcpy(b->d_tnodes, HL.tnodes.data(), sizeof(TreeNode) * HL.tnodes.size(), cudaMemcpyHostToDevice));
+    }
     if (!s) s = dalloc(&b->d_desc, n, total);
     if (!s) s = dalloc(&b->d_nodes, nodes, total);
     if (!s) s = dalloc(&b->d_tabs, tabs, total);
@@ -2623,7 +3173,7 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     if (!s) s = dalloc(&b->d_S, rs, total);
     if (!s) s = dalloc(&b->d_darena, darena, total);
     if (!s) s = dalloc(&b->d_results, 6LL * n, total);
-    if (!s) s = dalloc(&b->d_iter, 1, total);
+    if (!s) s = dalloc(&b->d_iter, 3, total);
     if (!s) s = dalloc(&b->d_err, 1, total);
     if (!s) s = cuda_status(cudaMemset(b->d_err, 0, sizeof(int)));
     if (!s) s = build_set(b, b->full, nullptr, total);
