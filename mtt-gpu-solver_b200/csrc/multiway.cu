@@ -41,6 +41,7 @@
 #include "mtt_bulk.cuh"
 #include "mtt_common.h"
 #include "mtt_device.cuh"
+#include "solver_tree.cuh"
 
 namespace mtt {
 namespace mw {
@@ -274,21 +275,6 @@ struct MwDev {
 
 enum { MODE_SOLVE = 0, MODE_AVG = 1 };
 
-__device__ __forceinline__ float4 f4(float v) { return make_float4(v, v, v, v); }
-__device__ __forceinline__ float4 add4(float4 a, float4 b) {
-    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
-    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) {
-    return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
-                       __fmaf_rn(a.w, b.w, c.w));
-}
-__device__ __forceinline__ float4 max04(float4 a) {
-    return make_float4(fmaxf(a.x, 0.f), fmaxf(a.y, 0.f), fmaxf(a.z, 0.f), fmaxf(a.w, 0.f));
-}
-__device__ __forceinline__ float rm1(float pos, float sum, float invA) { return sum > 1e-7f ? __fdiv_rn(pos, sum) : invA; }
 __device__ __forceinline__ float avg1(float s, float sum, float invA) { return sum > 0.0f ? __fdiv_rn(s, sum) : invA; }
 
 // sigma of action k for one float4 group: regret matching on R (threshold
@@ -309,19 +295,19 @@ __device__ __forceinline__ float4 sigma_sum(const float4* B, int H4, int g, int 
     return s;
 }
 
-__global__ void k_mw_init(MwDev a, int n_sub, int zero_rs) {
-    const int s = blockIdx.x;
-    if (s == 0 && threadIdx.x == 0) *a.iter = 1;
-    if (s >= n_sub) return;
-    const MDesc d = a.desc[s];
-    if (zero_rs) {
-        for (int p = 0; p < NP; ++p) {
-            const long long end = d.rs_base[p] + (long long)d.rows[p] * d.Hp;
-            for (long long i = d.rs_base[p] + threadIdx.x; i < end; i += blockDim.x) { a.R[i] = 0.f; a.S[i] = 0.f; }
-        }
+// The root reach of every subgame, the iteration counter and, for a solve, n4
+// float4 of regrets and of sums zeroed by the whole grid.
+__global__ void k_mw_init(MwDev a, int n_sub, long long n4, int last) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) { a.iter[0] = 1; a.iter[1] = 0; a.iter[2] = last; }
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    float4* r = reinterpret_cast<float4*>(a.R);
+    float4* z = reinterpret_cast<float4*>(a.S);
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += stride) { r[i] = f4(0.f); z[i] = f4(0.f); }
+    for (int s = blockIdx.x; s < n_sub; s += gridDim.x) {
+        const MDesc& d = a.desc[s];
+        float* rr = a.arena + d.arena_base;
+        for (int i = threadIdx.x; i < NP * d.Hp; i += blockDim.x) rr[i] = a.ranges[d.range_base + i];
     }
-    float* rr = a.arena + d.arena_base;
-    for (int i = threadIdx.x; i < NP * d.Hp; i += blockDim.x) rr[i] = a.ranges[d.range_base + i];
 }
 
 __global__ void k_mw_next_iter(MwDev a) {
@@ -749,6 +735,14 @@ struct mtt_mw_batch {
     MBwd* d_bwd = nullptr;
     int2* d_terms = nullptr;
     std::vector<long long> fwd_off, bwd_off;   // per level
+    // whole-tree sweeps of the solve (the values pass keeps the level kernels)
+    bool tree = false;
+    TreeSeg* d_segs = nullptr;
+    int* d_ints = nullptr;
+    TreeNode* d_tnodes = nullptr;
+    TreeCta* d_ctas = nullptr;
+    int n_ctas = 0, tree_smem = 0;
+    long long rs4 = 0;                          // float4 of R (and of S)
     int n_terms = 0;
     std::vector<MDesc> desc;
     std::vector<int> rows;                      // 4 per subgame
@@ -769,6 +763,7 @@ void free_mw(mtt_mw_batch* b) {
     cudaFree(b->d_desc); cudaFree(b->d_nodes); cudaFree(b->d_tabs); cudaFree(b->d_ranges); cudaFree(b->d_arena);
     cudaFree(b->d_R); cudaFree(b->d_S); cudaFree(b->d_iter); cudaFree(b->d_iter_tab); cudaFree(b->d_values);
     cudaFree(b->d_fwd); cudaFree(b->d_bwd); cudaFree(b->d_terms);
+    cudaFree(b->d_segs); cudaFree(b->d_ints); cudaFree(b->d_tnodes); cudaFree(b->d_ctas);
     delete b;
 }
 
@@ -783,6 +778,31 @@ MwDev mw_args(const mtt_mw_batch* b, int algo, int sem) {
     a.desc = b->d_desc; a.nodes = b->d_nodes; a.tabs = b->d_tabs; a.ranges = b->d_ranges; a.arena = b->d_arena;
     a.R = b->d_R; a.S = b->d_S; a.iter_tab = b->d_iter_tab; a.iter = b->d_iter; a.algo = algo; a.semantics = sem;
     return a;
+}
+
+int launch_terms(const mtt_mw_batch* b, const MwDev& a, cudaStream_t st) {
+    if (!b->n_terms) return MTT_OK;
+    if (a.semantics == MTT_SEM_CORRECT) {
+        MTT_TRY_CUDA(launch_pdl(k_mw_term_cr, (unsigned)b->n_terms, MT, term_cr_smem(b), st, true, a,
+                                (const int2*)b->d_terms, b->n_terms));
+    } else {
+        const size_t smem = sizeof(double) * (size_t)NP * ((size_t)b->Hmax + 1);
+        MTT_TRY_CUDA(launch_pdl(k_mw_term, (unsigned)b->n_terms, MT, smem, st, true, a, (const int2*)b->d_terms, b->n_terms));
+    }
+    MTT_CHECK_LAUNCH();
+    return MTT_OK;
+}
+
+int launch_tree(const mtt_mw_batch* b, const MwDev& a, int flags, bool chained, cudaStream_t st) {
+    TreeArgs t;
+    t.arena = a.arena; t.R = a.R; t.S = a.S; t.iter_tab = a.iter_tab; t.iter = a.iter;
+    t.ctas = b->d_ctas; t.segs = b->d_segs; t.ints = b->d_ints; t.nodes = b->d_tnodes;
+    t.n = b->n_ctas;
+    t.flags = flags;
+    MTT_TRY_CUDA(launch_pdl(a.algo == MTT_ALGO_DCFR ? k_tree<MTT_ALGO_DCFR, true> : k_tree<MTT_ALGO_CFRPLUS, true>,
+                            (unsigned)t.n, TREE_THREADS, b->tree_smem, st, chained, t));
+    MTT_CHECK_LAUNCH();
+    return MTT_OK;
 }
 
 int launch_sweep(const mtt_mw_batch* b, const MwDev& a, int mode, cudaStream_t st) {
@@ -802,16 +822,7 @@ int launch_sweep(const mtt_mw_batch* b, const MwDev& a, int mode, cudaStream_t s
         MTT_CHECK_LAUNCH();
         chained = true;
     }
-    if (b->n_terms) {
-        if (a.semantics == MTT_SEM_CORRECT) {
-            MTT_TRY_CUDA(launch_pdl(k_mw_term_cr, (unsigned)b->n_terms, MT, term_cr_smem(b), st, true, a,
-                                    (const int2*)b->d_terms, b->n_terms));
-        } else {
-            const size_t smem = sizeof(double) * (size_t)NP * ((size_t)b->Hmax + 1);
-            MTT_TRY_CUDA(launch_pdl(k_mw_term, (unsigned)b->n_terms, MT, smem, st, true, a, (const int2*)b->d_terms, b->n_terms));
-        }
-        MTT_CHECK_LAUNCH();
-    }
+    MTT_TRY(launch_terms(b, a, st));
     chained = true;
     for (int d = b->levels - 1; d >= 0; --d) {
         const long long n = b->bwd_off[d + 1] - b->bwd_off[d];
@@ -826,7 +837,13 @@ int launch_sweep(const mtt_mw_batch* b, const MwDev& a, int mode, cudaStream_t s
     return MTT_OK;
 }
 
+// One iteration.  With the tree sweeps the reach is in place (the solve's first
+// forward part or the iteration before).
 int launch_iteration(const mtt_mw_batch* b, const MwDev& a, cudaStream_t st) {
+    if (b->tree) {
+        MTT_TRY(launch_terms(b, a, st));
+        return launch_tree(b, a, TR_BWD | TR_FWD | TR_LAST | TR_NEXT, true, st);
+    }
     MTT_TRY(launch_sweep(b, a, MODE_SOLVE, st));
     k_mw_next_iter<<<1, 32, 0, st>>>(a);
     MTT_CHECK_LAUNCH();
@@ -840,6 +857,10 @@ int set_term_smem(const mtt_mw_batch* b) {
     const size_t cr = term_cr_smem(b);
     if (cr > 48 * 1024)
         MTT_TRY_CUDA(cudaFuncSetAttribute(k_mw_term_cr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cr));
+    if (b->tree_smem > 48 * 1024) {
+        MTT_TRY_CUDA(cudaFuncSetAttribute(k_tree<MTT_ALGO_CFRPLUS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->tree_smem));
+        MTT_TRY_CUDA(cudaFuncSetAttribute(k_tree<MTT_ALGO_DCFR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->tree_smem));
+    }
     return MTT_OK;
 }
 }  // namespace
@@ -870,6 +891,9 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     std::vector<std::vector<MFwd>> fl;
     std::vector<std::vector<MBwd>> bl;
     std::vector<int2> tl;
+    TreeHost th;
+    bool fits = true;
+    constexpr int TREE_BYTES = 224 * 1024;
     long long arena = 0, rs = 0;
     b->desc.resize(n);
     b->rows.resize(4 * (size_t)n);
@@ -1031,6 +1055,23 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
                 tl.push_back(make_int2(gn, s));
             }
         }
+        for (int q = 0; q < NP; ++q) {
+            auto node = [&](int k) {
+                const MNode& x = loc[k];
+                return TreeShapeNode{x.type == MTT_NODE_DECISION, x.player, x.na, x.first, x.row, x.src[q], depth[k]};
+            };
+            TreeSeg t{};
+            t.reach = d.arena_base + (long long)q * d.Hp;
+            t.cfv = d.arena_base + (long long)g.n_nodes * HS + (long long)q * d.Hp;
+            t.rows = d.rs_base[q];
+            t.h4 = H4;
+            t.hs4 = (int)(HS / 4);
+            t.n_rows = g.rows[q];
+            t.n_nodes = g.n_nodes;
+            fits &= g.n_nodes < TREE_MAX_NODES && g.rows[q] < TREE_MAX_NODES - 1;
+            if (fits) fits &= tree_min_bytes(g.n_nodes, g.rows[q], q, 0, true, node) <= TREE_BYTES;
+            if (fits) build_tree_seg(th, t, s, q, node);
+        }
         hn.insert(hn.end(), loc.begin(), loc.end());
         b->desc[s] = d;
         for (int p = 0; p < NP; ++p) b->rows[4 * (size_t)s + p] = g.rows[p];
@@ -1047,7 +1088,40 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
         b->bwd_off[d + 1] = (long long)bb.size();
     }
     b->n_terms = (int)tl.size();
+    b->rs4 = rs / 4;
+    // whole-tree sweeps (their reason stands with k_tree): slices of 8 hands
+    // where three CTAs an SM fit, fewer where only that fits at all.  One 1,585-
+    // node subgame of 1,081 hands took 204.7 us an iteration by levels (147.6
+    // once zero regrets skip their divisions) and takes 101; two 231 / 188,
+    // four (2,176 CTAs) 376 / 371, eight 672 / 721, so larger batches keep the
+    // level kernels.
+    std::vector<TreeCta> tc;
+    if (fits) {
+        for (int i = 0; i < (int)th.segs.size(); ++i) {
+            const TreeSeg& g = th.segs[i];
+            auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg, true); };
+            const int lg = bytes(3) <= 72 * 1024 ? 3 : bytes(2) <= 72 * 1024 ? 2 : bytes(1) <= 72 * 1024 ? 1 : 0;
+            b->tree_smem = std::max(b->tree_smem, bytes(lg));
+            for (int g0 = 0; g0 < g.h4; g0 += 1 << lg) tc.push_back(TreeCta{i, g0, lg, 0});
+        }
+        b->n_ctas = (int)tc.size();
+        int sms = 148, dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        b->tree = b->n_ctas <= 12 * sms;
+        if (!b->tree) b->tree_smem = 0;
+    }
     int s = MTT_OK;
+    if (b->tree) {
+        s = dalloc(&b->d_segs, th.segs.size());
+        if (!s) s = dalloc(&b->d_ints, th.ints.size());
+        if (!s) s = dalloc(&b->d_tnodes, th.nodes.size());
+        if (!s) s = dalloc(&b->d_ctas, tc.size());
+        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, th.segs.data(), sizeof(TreeSeg) * th.segs.size(), cudaMemcpyHostToDevice));
+        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, th.ints.data(), sizeof(int) * th.ints.size(), cudaMemcpyHostToDevice));
+        if (!s && !th.nodes.empty())
+            s = cuda_status(cudaMemcpy(b->d_tnodes, th.nodes.data(), sizeof(TreeNode) * th.nodes.size(), cudaMemcpyHostToDevice));
+        if (!s) s = cuda_status(cudaMemcpy(b->d_ctas, tc.data(), sizeof(TreeCta) * tc.size(), cudaMemcpyHostToDevice));
+    }
     if (!s) s = dalloc(&b->d_desc, n);
     if (!s) s = dalloc(&b->d_nodes, hn.size());
     if (!s) s = dalloc(&b->d_tabs, ht.size());
@@ -1055,7 +1129,7 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     if (!s) s = dalloc(&b->d_arena, (size_t)arena);
     if (!s) s = dalloc(&b->d_R, (size_t)rs);
     if (!s) s = dalloc(&b->d_S, (size_t)rs);
-    if (!s) s = dalloc(&b->d_iter, 1);
+    if (!s) s = dalloc(&b->d_iter, 3);
     if (!s) s = dalloc(&b->d_values, 4 * (size_t)n);
     if (!s) s = dalloc(&b->d_fwd, ff.size());
     if (!s) s = dalloc(&b->d_bwd, bb.size());
@@ -1102,8 +1176,10 @@ extern "C" int mtt_mw_batch_solve(mtt_mw_batch* b, const mtt_solve_params* p, in
     MTT_TRY(set_term_smem(b));
     b->last_sem = p->semantics;
     const MwDev a = mw_args(b, p->algo, p->semantics);
-    k_mw_init<<<b->n, 256, 0, st>>>(a, b->n, 1);
+    k_mw_init<<<(unsigned)std::max<long long>(b->n, std::min<long long>(8 * 148, b->rs4 / (256 * 4) + 1)), 256, 0, st>>>(
+        a, b->n, b->rs4, p->iters);
     MTT_CHECK_LAUNCH();
+    if (b->tree && p->iters > 0) MTT_TRY(launch_tree(b, a, TR_FWD, false, st));
     if (!graph) {
         for (int t = 0; t < p->iters; ++t) MTT_TRY(launch_iteration(b, a, st));
         return MTT_OK;
@@ -1133,7 +1209,7 @@ extern "C" int mtt_mw_batch_values(mtt_mw_batch* b, double* h_out, void* stream)
     cudaStream_t st = as_stream(stream);
     MTT_TRY(set_term_smem(b));
     const MwDev a = mw_args(b, MTT_ALGO_CFRPLUS, b->last_sem);
-    k_mw_init<<<b->n, 256, 0, st>>>(a, b->n, 0);
+    k_mw_init<<<b->n, 256, 0, st>>>(a, b->n, 0, 0);
     MTT_CHECK_LAUNCH();
     MTT_TRY(launch_sweep(b, a, MODE_AVG, st));
     k_mw_root<<<b->n, MT, 0, st>>>(a, b->n, b->d_values);

@@ -36,6 +36,7 @@
 #include "mtt_common.h"
 #include "mtt_device.cuh"
 #include "solver_impl.cuh"
+#include "solver_tree.cuh"
 
 namespace mtt {
 
@@ -43,57 +44,6 @@ int validate_tree(const mtt_node* nodes, int n, const int rows[2]);   // tree.cp
 
 
 // ====================================================================== device
-__device__ __forceinline__ float4 f4(float v) { return make_float4(v, v, v, v); }
-__device__ __forceinline__ float4 add4(float4 a, float4 b) {
-    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
-}
-__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
-    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
-}
-// Starts a fetch of the line holding p into L2 (no register is written, so
-// every row of a work item can be requested before its first use).
-__device__ __forceinline__ void pf_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
-}
-
-__device__ __forceinline__ float4 max04(float4 a) {
-    return make_float4(fmaxf(a.x, 0.f), fmaxf(a.y, 0.f), fmaxf(a.z, 0.f), fmaxf(a.w, 0.f));
-}
-// Regret matching: pos / sum, or uniform where nothing is positive.  A zero
-// numerator would take the division's long special-case path, and under CFR+
-// a large share of the regrets is exactly 0, so those skip the division (the
-// quotient is 0 either way).  rm1 divides in line with the zeros replaced,
-// rm1b branches around the division: on the 1,024-subgame river batch the
-// forward levels took 224 -> 167 us (175 with rm1b) and the backward levels
-// 566 -> 515 us (543 with rm1, whose temporaries spill there).
-__device__ __forceinline__ float rm1(float pos, float sum, float invA) {
-    const bool some = sum > 1e-7f, in = pos > 0.f;
-    const float d = some ? sum : 1.f;
-    const float q = __fdiv_rn(in ? pos : d, d);
-    return some ? (in ? q : 0.f) : invA;
-}
-__device__ __forceinline__ float rm1b(float pos, float sum, float invA) {
-    float q = sum > 1e-7f ? 0.f : invA;
-    if (sum > 1e-7f && pos > 0.f) q = __fdiv_rn(pos, sum);
-    return q;
-}
-__device__ __forceinline__ float4 rm4(float4 pos, float4 sum, float invA) {
-    return make_float4(rm1(pos.x, sum.x, invA), rm1(pos.y, sum.y, invA), rm1(pos.z, sum.z, invA),
-                       rm1(pos.w, sum.w, invA));
-}
-__device__ __forceinline__ float4 rm4b(float4 pos, float4 sum, float invA) {
-    return make_float4(rm1b(pos.x, sum.x, invA), rm1b(pos.y, sum.y, invA), rm1b(pos.z, sum.z, invA),
-                       rm1b(pos.w, sum.w, invA));
-}
-__device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) {
-    return make_float4(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y), __fmaf_rn(a.z, b.z, c.z),
-                       __fmaf_rn(a.w, b.w, c.w));
-}
-__device__ __forceinline__ float cfrplus1(float r, float inst) { return fmaxf(0.0f, __fadd_rn(r, inst)); }
-__device__ __forceinline__ float dcfr1(float r, float inst, float dpos, float dneg) {
-    return __fadd_rn(__fmul_rn(r, r > 0.0f ? dpos : dneg), inst);
-}
-
 struct Task {        // one warp: groups [g0, g0 + 32) of float4 hand groups at one node
     int node;        // global node index
     int sub;         // subgame
@@ -1086,269 +1036,6 @@ __global__ void __launch_bounds__(256, 5) k_bwd(SolveDev a, const BwdItem* __res
     }
 }
 
-// ------------------------------------------------------------- whole-tree sweeps
-// Between two terminal passes every value of a hand depends on that hand
-// alone: its counterfactual values come up the tree from its own terminals,
-// its regrets and strategy follow, and its reach goes down the tree again.  So
-// where a subgame deals no card and its tree is small enough, one CTA takes
-// one player's slice of 8 to 32 hands through the whole tree: it stages the
-// slice's regret and strategy-sum rows, terminal values and reach in shared
-// memory (asynchronous 16-byte copies, all in flight at once), walks the
-// backward levels and then the forward levels of the new strategy there, with
-// a block barrier between levels instead of a launch, and writes every result
-// as it is formed.  An iteration of alternating updates is then four launches
-// (terminals and tree, per player) instead of one per level, kernel class and
-// player: a 39-node spot's iteration took 61.6 us by levels (47.3 once zero
-// regrets skip their divisions) and takes 26.4 us.  Bound by the chain of
-// levels; the arithmetic of a node and hand is that of k_bwd and k_fwd, in the
-// same order, so the results are the same bit for bit.
-struct alignas(16) TreeSeg {   // one player of one subgame
-    long long reach;      // arena float offset of the player's part of node 0's reach slot
-    long long cfv;        // the same in the value region
-    long long rows;       // R/S float offset of the player's rows
-    int h4, hs4;          // float4 groups of the player; slot stride in float4
-    int n_rows, n_nodes;
-    int node0, n_dec;     // decision nodes, in backward order
-    int int0, n_int;      // integers: [nb + 1 backward bounds][nf + 1 forward bounds][own nodes in forward order][terminals]
-    int nb, nf, n_own, n_term;
-    int pad[2];
-};
-static_assert(sizeof(TreeSeg) == 80, "TreeSeg is 80 bytes");
-struct TreeCta {          // one CTA: hands [4 g0, 4 (g0 + G)) of a TreeSeg, G = 1 << lg lanes
-    int seg, g0, lg, pad;
-};
-// A decision node: first child; node | reach id << 16; node whose slot holds
-// the player's reach; actions | acts << 5 | first regret row << 6.  Reach ids
-// number the slots the player writes: 0 the root, 1 + row + k child k of the
-// own node with that first row.
-using TreeNode = int4;
-struct TreeArgs {
-    const TreeCta* ctas;
-    const TreeSeg* segs;
-    const int* ints;
-    const TreeNode* nodes;
-    int n;                // CTAs of all the launches that close the iteration (TR_NEXT)
-    int flags;            // TR_*
-};
-enum { TR_BWD = 1, TR_FWD = 2, TR_LAST = 4, TR_NEXT = 8 };   // TR_LAST: no forward part in the run's last iteration
-constexpr int TREE_THREADS = 256, TREE_MAX_NODES = 1 << 16;
-
-__host__ __device__ inline int tree_smem_bytes(int n_rows, int n_nodes, int n_dec, int n_int, int lg) {
-    return ((3 * n_rows + 1 + n_nodes) << lg) * 16 + n_dec * 16 + (n_int + 3) / 4 * 16;
-}
-
-template <int ALGO>
-__device__ __forceinline__ float4 upd_regret(float4 rk, float4 qk, float4 v, float dpos, float dneg) {
-    if (ALGO == MTT_ALGO_DCFR)
-        return make_float4(dcfr1(rk.x, __fsub_rn(qk.x, v.x), dpos, dneg), dcfr1(rk.y, __fsub_rn(qk.y, v.y), dpos, dneg),
-                           dcfr1(rk.z, __fsub_rn(qk.z, v.z), dpos, dneg), dcfr1(rk.w, __fsub_rn(qk.w, v.w), dpos, dneg));
-    return make_float4(cfrplus1(rk.x, __fsub_rn(qk.x, v.x)), cfrplus1(rk.y, __fsub_rn(qk.y, v.y)),
-                       cfrplus1(rk.z, __fsub_rn(qk.z, v.z)), cfrplus1(rk.w, __fsub_rn(qk.w, v.w)));
-}
-template <int ALGO>
-__device__ __forceinline__ float4 upd_sum(float4 sv, float4 r, float4 wr, float4 sg, float dstr) {
-    return ALGO == MTT_ALGO_DCFR ? fma4(r, sg, mul4(sv, f4(dstr))) : fma4(wr, sg, sv);
-}
-__device__ __forceinline__ void copy_async16(float4* dst, const float4* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
-// One node of one hand group, its rows and child values G float4 apart in
-// shared memory: the acting player's update (returns the node's value) and the
-// reach of its children.  A: the action count, with every row read before any
-// is used, or 0: na actions.
-template <int A, int ALGO, bool SIM>
-__device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, const float4* q, float4 r, float4* R, float4* S,
-                                              int na, int lg, int H4, const float4& tb) {
-    const int n = A ? A : na;
-    const float invA = __fdiv_rn(1.0f, (float)n);
-    const float4 wr = mul4(r, f4(tb.x));
-    float4 sum = f4(0.f), v = f4(0.f);
-    if constexpr (A > 0) {
-        float4 rk[A], qk[A], sg[A];
-#pragma unroll
-        for (int k = 0; k < A; ++k) { rk[k] = rs[k << lg]; qk[k] = q[k << lg]; }
-#pragma unroll
-        for (int k = 0; k < A; ++k) sum = add4(sum, max04(rk[k]));
-#pragma unroll
-        for (int k = 0; k < A; ++k) sg[k] = rm4(max04(rk[k]), sum, invA);
-#pragma unroll
-        for (int k = 0; k < A; ++k) {
-            v = fma4(sg[k], qk[k], v);
-            if (!SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg[k], tb.w);
-        }
-#pragma unroll
-        for (int k = 0; k < A; ++k) {
-            const float4 x = upd_regret<ALGO>(rk[k], qk[k], v, tb.y, tb.z);
-            R[(size_t)k * H4] = x;
-            rs[k << lg] = x;
-        }
-    } else {
-#pragma unroll 1
-        for (int k = 0; k < n; ++k) sum = add4(sum, max04(rs[k << lg]));
-#pragma unroll 1
-        for (int k = 0; k < n; ++k) {
-            const float4 sg = rm4(max04(rs[k << lg]), sum, invA);
-            v = fma4(sg, q[k << lg], v);
-            if (!SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg, tb.w);
-        }
-#pragma unroll 1
-        for (int k = 0; k < n; ++k) {
-            const float4 x = upd_regret<ALGO>(rs[k << lg], q[k << lg], v, tb.y, tb.z);
-            R[(size_t)k * H4] = x;
-            rs[k << lg] = x;
-        }
-    }
-    return v;
-}
-
-template <int A, int ALGO, bool SIM>
-__device__ __forceinline__ void tree_reach(const float4* rs, const float4* ss, float4 r, float4* P, float4* ch, float4* S,
-                                           int na, int lg, int H4, int HS4, const float4& tb) {
-    const int n = A ? A : na;
-    const float invA = __fdiv_rn(1.0f, (float)n);
-    const float4 wr = mul4(r, f4(tb.x));
-    float4 sum = f4(0.f);
-    auto put = [&](int k, float4 sg) {
-        const float4 x = mul4(r, sg);
-        P[k << lg] = x;
-        ch[(size_t)k * HS4] = x;
-        if (SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg, tb.w);
-    };
-    if constexpr (A > 0) {
-        float4 rk[A];
-#pragma unroll
-        for (int k = 0; k < A; ++k) rk[k] = max04(rs[k << lg]);
-#pragma unroll
-        for (int k = 0; k < A; ++k) sum = add4(sum, rk[k]);
-#pragma unroll
-        for (int k = 0; k < A; ++k) rk[k] = rm4(rk[k], sum, invA);
-#pragma unroll
-        for (int k = 0; k < A; ++k) put(k, rk[k]);
-    } else {
-#pragma unroll 1
-        for (int k = 0; k < n; ++k) sum = add4(sum, max04(rs[k << lg]));
-#pragma unroll 1
-        for (int k = 0; k < n; ++k) put(k, rm4(max04(rs[k << lg]), sum, invA));
-    }
-}
-
-// SIM: both players are updated from one terminal pass; the strategy sums are
-// then added by the forward part (of the next iteration), else by the backward
-// part.
-template <int ALGO, bool SIM>
-__global__ void __launch_bounds__(TREE_THREADS, 2) k_tree(SolveDev a, TreeArgs t) {
-    extern __shared__ __align__(16) float4 tree_smem[];
-    const TreeCta c = t.ctas[blockIdx.x];
-    const TreeSeg sg = t.segs[c.seg];
-    const int tid = threadIdx.x, lg = c.lg, G = 1 << lg, groups = TREE_THREADS >> lg;
-    const int lane = tid & (G - 1), grp = tid >> lg, g = c.g0 + lane;
-    const int H4 = sg.h4, HS4 = sg.hs4, n_rows = sg.n_rows;
-    const bool live = g < H4;
-    float4* const Rs = tree_smem + lane;                              // regret rows
-    float4* const Ss = Rs + (n_rows << lg);                           // strategy sums
-    float4* const V = Ss + (n_rows << lg);                            // values by node
-    float4* const P = V + (sg.n_nodes << lg);                         // reach by id
-    TreeNode* const nodes = reinterpret_cast<TreeNode*>(tree_smem + ((3 * n_rows + 1 + sg.n_nodes) << lg));
-    int* const blev = reinterpret_cast<int*>(nodes + sg.n_dec);
-    int* const flev = blev + sg.nb + 1;
-    int* const own = flev + sg.nf + 1;
-    int* const term = own + sg.n_own;
-    for (int i = tid; i < sg.n_dec; i += TREE_THREADS) nodes[i] = t.nodes[sg.node0 + i];
-    for (int i = tid; i < sg.n_int; i += TREE_THREADS) blev[i] = t.ints[sg.int0 + i];
-    float4* const reach = reinterpret_cast<float4*>(a.arena + sg.reach) + g;
-    float4* const cfv = reinterpret_cast<float4*>(a.arena + sg.cfv) + g;
-    float4* const R = reinterpret_cast<float4*>(a.R + sg.rows) + g;
-    float4* const S = reinterpret_cast<float4*>(a.S + sg.rows) + g;
-    __syncthreads();
-    // the tree's description is written once, before any solve; all else
-    // belongs to the kernels before
-    grid_dep_trigger();
-    grid_dep_wait();
-    const int iter = a.iter[0];
-    const bool bwd = t.flags & TR_BWD;
-    const bool fwd = (t.flags & TR_FWD) && !((t.flags & TR_LAST) && iter >= a.iter[2]);
-    if (live) {
-        for (int i = grp; i < n_rows; i += groups) {
-            copy_async16(Rs + (i << lg), R + (size_t)i * H4);
-            if (SIM ? fwd : bwd) copy_async16(Ss + (i << lg), S + (size_t)i * H4);
-        }
-        if (bwd)
-            for (int i = grp; i < sg.n_term; i += groups)
-                copy_async16(V + (term[i] << lg), cfv + (size_t)term[i] * HS4);
-        if (bwd && !SIM) {
-            for (int i = grp; i < sg.n_own; i += groups) {
-                const TreeNode nd = nodes[own[i]];
-                copy_async16(P + ((int)((unsigned)nd.y >> 16) << lg), reach + (size_t)nd.z * HS4);
-            }
-        } else if (grp == 0) {
-            copy_async16(P, reach);
-        }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    if (bwd) {
-        const float4 tb = *reinterpret_cast<const float4*>(a.iter_tab + 4 * (size_t)(iter - 1));
-        for (int l = 0; l < sg.nb; ++l) {
-            const int hi = blev[l + 1];
-            for (int i = blev[l] + grp; live && i < hi; i += groups) {
-                const TreeNode nd = nodes[i];
-                const int na = nd.w & 31, self = nd.y & 0xFFFF;
-                const float4* const q = V + (nd.x << lg);
-                float4 v = f4(0.f);
-                if (nd.w & 32) {
-                    const int row = (int)((unsigned)nd.w >> 6);
-                    const float4 r = SIM ? f4(0.f) : P[(int)((unsigned)nd.y >> 16) << lg];
-#define TREE_CALL(A) \
-    v = tree_update<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), q, r, R + (size_t)row * H4, S + (size_t)row * H4, na, lg, \
-                                  H4, tb)
-                    switch (na) {
-                        case 2: TREE_CALL(2); break;
-                        case 3: TREE_CALL(3); break;
-                        case 4: TREE_CALL(4); break;
-                        default: TREE_CALL(0); break;
-                    }
-#undef TREE_CALL
-                } else {
-#pragma unroll 4
-                    for (int k = 0; k < na; ++k) v = add4(v, q[k << lg]);
-                }
-                V[self << lg] = v;
-                cfv[(size_t)self * HS4] = v;
-            }
-            __syncthreads();
-        }
-    }
-    if (fwd) {
-        // the sums of simultaneous updates are weighted by the iteration they open
-        const float4 tb = SIM ? *reinterpret_cast<const float4*>(a.iter_tab + 4 * (size_t)(iter - (bwd ? 0 : 1))) : f4(0.f);
-        for (int l = 0; l < sg.nf; ++l) {
-            const int hi = flev[l + 1];
-            for (int i = flev[l] + grp; live && i < hi; i += groups) {
-                const TreeNode nd = nodes[own[i]];
-                const int na = nd.w & 31, row = (int)((unsigned)nd.w >> 6);
-                const float4 r = P[(int)((unsigned)nd.y >> 16) << lg];
-#define TREE_CALL(A) \
-    tree_reach<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), r, P + ((1 + row) << lg), reach + (size_t)nd.x * HS4, \
-                             S + (size_t)row * H4, na, lg, H4, HS4, tb)
-                switch (na) {
-                    case 2: TREE_CALL(2); break;
-                    case 3: TREE_CALL(3); break;
-                    case 4: TREE_CALL(4); break;
-                    default: TREE_CALL(0); break;
-                }
-#undef TREE_CALL
-            }
-            if (l + 1 < sg.nf) __syncthreads();
-        }
-    }
-    // the last CTA of the closing launches opens the next iteration: every CTA has read this one's number
-    if ((t.flags & TR_NEXT) && tid == 0 && atomicAdd(a.iter + 1, 1) == t.n - 1) {
-        a.iter[1] = 0;
-        a.iter[0] = iter + 1;
-    }
-}
-
 __global__ void k_set_last(SolveDev a, int last) {
     if (threadIdx.x == 0) a.iter[2] = last;
 }
@@ -1926,12 +1613,8 @@ struct HostLists {
     std::vector<std::vector<Task>> bf, bb;
     std::vector<TermItem> titems;    // by subgame, then table variant
     std::vector<int2> terms;
-    // whole-tree sweeps: two segments per subgame that takes them, with their
-    // subgame, nodes and integers
-    std::vector<TreeSeg> segs;
-    std::vector<int> seg_sub;
-    std::vector<int> ints;
-    std::vector<TreeNode> tnodes;
+    // whole-tree sweeps: two segments (players) per subgame that takes them
+    TreeHost tree;
 };
 
 constexpr int TREE_CLASSES = 3;                      // by shared memory: about 5, 2 and 1 CTAs an SM
@@ -2151,79 +1834,9 @@ static int upload_levels(LevelLists<T>& L, const std::vector<std::vector<T>>& lv
     return MTT_OK;
 }
 
-// Shared memory of the smallest slice (8 hands) of one player's tree.
-static int tree_min_bytes(const SubDesc& d, const std::vector<DNode>& nodes, int q) {
-    int dec = 0, own = 0;
-    for (const DNode& nd : nodes) {
-        dec += nd.type == MTT_NODE_DECISION;
-        own += nd.type == MTT_NODE_DECISION && nd.player == q;
-    }
-    // at most one level per node
-    return tree_smem_bytes(q ? d.rows1 : d.rows0, d.n_nodes, dec, 2 * (dec + 1) + own + d.n_nodes - dec, 1);
-}
-
-// One player's view of a chance-free tree: the backward order (all decision
-// nodes, deepest level first) and the forward order (the player's own, by how
-// many of them lie above), each level sorted by role and action count so that
-// a warp's nodes take the same path.
-static void build_tree_seg(const std::vector<DNode>& nodes, const std::vector<int16_t>& depth, const SubDesc& d, int sub,
-                           int q, HostLists& L) {
-    const long long HS = d.Hp0 + d.Hp1, off = q ? d.Hp0 : 0;
-    TreeSeg g{};
-    g.reach = d.arena_base + off;
-    g.cfv = d.arena_base + (long long)d.n_nodes * HS + off;
-    g.rows = q ? d.rs_base1 : d.rs_base0;
-    g.h4 = (q ? d.Hp1 : d.Hp0) / 4;
-    g.hs4 = (int)(HS / 4);
-    g.n_rows = q ? d.rows1 : d.rows0;
-    g.n_nodes = d.n_nodes;
-    g.node0 = (int)L.tnodes.size();
-    g.int0 = (int)L.ints.size();
-    std::vector<int> above(d.n_nodes, 0), id(d.n_nodes, 0), pos(d.n_nodes, 0), order;
-    for (int k = 0; k < d.n_nodes; ++k) {
-        const DNode& nd = nodes[k];
-        if (nd.type != MTT_NODE_DECISION) continue;
-        const bool own = nd.player == q;
-        for (int c = 0; c < nd.na; ++c) {
-            above[nd.first + c] = above[k] + (own ? 1 : 0);
-            if (own) id[nd.first + c] = 1 + nd.row + c;
-        }
-        order.push_back(k);
-    }
-    auto key = [&](int k) { return (nodes[k].player == q ? 32 : 0) | nodes[k].na; };
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        return depth[x] != depth[y] ? depth[x] > depth[y] : key(x) < key(y);
-    });
-    g.n_dec = (int)order.size();
-    for (int i = 0; i < g.n_dec; ++i) {
-        const int k = order[i];
-        const DNode& nd = nodes[k];
-        if (i == 0 || depth[k] != depth[order[i - 1]]) { L.ints.push_back(i); ++g.nb; }
-        const int src = q ? nd.reach_src1 : nd.reach_src0;
-        const bool own = nd.player == q;
-        L.tnodes.push_back(make_int4(nd.first, (int)((unsigned)k | (unsigned)id[src] << 16), src,
-                                     (int)((unsigned)key(k) | (own ? (unsigned)nd.row << 6 : 0u))));
-        pos[k] = i;
-    }
-    L.ints.push_back(g.n_dec);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-        return above[x] != above[y] ? above[x] < above[y] : key(x) < key(y);
-    });
-    std::vector<int> own;
-    int last = -1;
-    for (int k : order) {
-        if (nodes[k].player != q) continue;
-        if (above[k] != last) { L.ints.push_back((int)own.size()); ++g.nf; last = above[k]; }
-        own.push_back(pos[k]);
-    }
-    L.ints.push_back((int)own.size());
-    g.n_own = (int)own.size();
-    L.ints.insert(L.ints.end(), own.begin(), own.end());
-    for (int k = 0; k < d.n_nodes; ++k)
-        if (nodes[k].type != MTT_NODE_DECISION) { L.ints.push_back(k); ++g.n_term; }
-    g.n_int = (int)L.ints.size() - g.int0;
-    L.segs.push_back(g);
-    L.seg_sub.push_back(sub);
+static TreeShapeNode shape_node(const std::vector<DNode>& nodes, const std::vector<int16_t>& depth, int q, int k) {
+    const DNode& nd = nodes[k];
+    return {nd.type == MTT_NODE_DECISION, nd.player, nd.na, nd.first, nd.row, q ? nd.reach_src1 : nd.reach_src0, depth[k]};
 }
 
 // The CTAs of the whole-tree sweeps.  A slice is 32 hands (128-byte rows), or
@@ -2235,10 +1848,10 @@ static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* ac
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     struct Pick { int seg, lg, bytes; };
     std::vector<Pick> picks[TREE_CLASSES][2];
-    for (int i = 0; i < (int)H.segs.size(); ++i) {
-        if (active && !(*active)[H.seg_sub[i]]) continue;
-        const TreeSeg& g = H.segs[i];
-        auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg); };
+    for (int i = 0; i < (int)H.tree.segs.size(); ++i) {
+        if (active && !(*active)[H.tree.sub[i]]) continue;
+        const TreeSeg& g = H.tree.segs[i];
+        auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg, false); };
         int lg = 1, cls = TREE_CLASSES - 1;
         if (bytes(2) <= TREE_CLASS_BYTES[0]) { cls = 0; lg = bytes(3) <= TREE_CLASS_BYTES[0] ? 3 : 2; }
         else if (bytes(1) <= TREE_CLASS_BYTES[1]) { cls = 1; lg = bytes(3) <= TREE_CLASS_BYTES[1] ? 3 : bytes(2) <= TREE_CLASS_BYTES[1] ? 2 : 1; }
@@ -2253,7 +1866,7 @@ static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* ac
             const size_t n0 = ctas.size();
             for (const Pick& x : v) {
                 L.tree_smem[c] = std::max(L.tree_smem[c], x.bytes);
-                for (int g0 = 0; g0 < H.segs[x.seg].h4; g0 += 1 << x.lg) ctas.push_back(TreeCta{x.seg, g0, x.lg, 0});
+                for (int g0 = 0; g0 < H.tree.segs[x.seg].h4; g0 += 1 << x.lg) ctas.push_back(TreeCta{x.seg, g0, x.lg, 0});
             }
             L.n_ctas[c][q] = (int)(ctas.size() - n0);
         }
@@ -2473,7 +2086,7 @@ static TermKernel term_kernel(int upd, int semantics) {
     return k[semantics ? 1 : 0][upd - 1];
 }
 
-using TreeKernel = void (*)(SolveDev, TreeArgs);
+using TreeKernel = void (*)(TreeArgs);
 static TreeKernel tree_kernel(int algo, bool sim) {
     static const TreeKernel k[2][2] = {{k_tree<MTT_ALGO_CFRPLUS, false>, k_tree<MTT_ALGO_CFRPLUS, true>},
                                        {k_tree<MTT_ALGO_DCFR, false>, k_tree<MTT_ALGO_DCFR, true>}};
@@ -2490,6 +2103,7 @@ static int launch_tree(const mtt_batch* b, const ListSet& L, const SolveDev& a, 
         all += n[c];
     }
     TreeArgs t;
+    t.arena = a.arena; t.R = a.R; t.S = a.S; t.iter_tab = a.iter_tab; t.iter = a.iter;
     t.segs = b->d_segs;
     t.ints = b->d_ints;
     t.nodes = b->d_tnodes;
@@ -2500,7 +2114,7 @@ static int launch_tree(const mtt_batch* b, const ListSet& L, const SolveDev& a, 
         t.ctas = first + (upd == 2 ? L.n_ctas[c][0] : 0);
         first += L.n_ctas[c][0] + L.n_ctas[c][1];
         if (!n[c]) continue;
-        MTT_TRY_CUDA(launch_pdl(tree_kernel(a.algo, sim), (unsigned)n[c], TREE_THREADS, L.tree_smem[c], st, chained, a, t));
+        MTT_TRY_CUDA(launch_pdl(tree_kernel(a.algo, sim), (unsigned)n[c], TREE_THREADS, L.tree_smem[c], st, chained, t));
         MTT_CHECK_LAUNCH();
         ++b->launches;
         chained = true;
@@ -2959,7 +2573,11 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
         bool ok = b->desc[i].n_nodes < TREE_MAX_NODES && b->desc[i].rows0 < TREE_MAX_NODES - 1 &&
                   b->desc[i].rows1 < TREE_MAX_NODES - 1;
         for (const DNode& nd : packs[i].nodes) ok &= nd.type != MTT_NODE_CHANCE && nd.type != MTT_NODE_LEAF;
-        for (int q = 0; q < 2 && ok; ++q) ok = tree_min_bytes(b->desc[i], packs[i].nodes, q) <= TREE_CLASS_BYTES[TREE_CLASSES - 1];
+        for (int q = 0; q < 2 && ok; ++q) {
+            auto node = [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); };
+            ok = tree_min_bytes(b->desc[i].n_nodes, q ? b->desc[i].rows1 : b->desc[i].rows0, q, 1, false, node) <=
+                 TREE_CLASS_BYTES[TREE_CLASSES - 1];
+        }
         b->tree[i] = ok;
         b->any_tree |= ok;
     }
@@ -3151,17 +2769,29 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     for (int t = 0; t < nlt; ++t) b->h_leaves.insert(b->h_leaves.end(), plv[t].begin(), plv[t].end());
     for (size_t k = 0; k < b->h_leaves.size(); ++k) b->h_leaves[k].row0 = LEAF_RIVERS * (int)k;
     for (int i = 0; i < n; ++i)
-        for (int q = 0; q < 2 && b->tree[i]; ++q) build_tree_seg(packs[i].nodes, packs[i].depth, b->desc[i], i, q, HL);
+        for (int q = 0; q < 2 && b->tree[i]; ++q) {
+            const SubDesc& d = b->desc[i];
+            const long long HS = d.Hp0 + d.Hp1, off = q ? d.Hp0 : 0;
+            TreeSeg g{};
+            g.reach = d.arena_base + off;
+            g.cfv = d.arena_base + (long long)d.n_nodes * HS + off;
+            g.rows = q ? d.rs_base1 : d.rs_base0;
+            g.h4 = (q ? d.Hp1 : d.Hp0) / 4;
+            g.hs4 = (int)(HS / 4);
+            g.n_rows = q ? d.rows1 : d.rows0;
+            g.n_nodes = d.n_nodes;
+            build_tree_seg(HL.tree, g, i, q, [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
+        }
     long long total = 0;
     int s = MTT_OK;
     if (b->any_tree) {
-        s = dalloc(&b->d_segs, HL.segs.size(), total);
-        if (!s) s = dalloc(&b->d_ints, HL.ints.size(), total);
-        if (!s) s = dalloc(&b->d_tnodes, HL.tnodes.size(), total);
-        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, HL.segs.data(), sizeof(TreeSeg) * HL.segs.size(), cudaMemcpyHostToDevice));
-        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, HL.ints.data(), sizeof(int) * HL.ints.size(), cudaMemcpyHostToDevice));
-        if (!s && !HL.tnodes.empty())
-            s = cuda_status(cudaMemcpy(b->d_tnodes, HL.tnodes.data(), sizeof(TreeNode) * HL.tnodes.size(), cudaMemcpyHostToDevice));
+        s = dalloc(&b->d_segs, HL.tree.segs.size(), total);
+        if (!s) s = dalloc(&b->d_ints, HL.tree.ints.size(), total);
+        if (!s) s = dalloc(&b->d_tnodes, HL.tree.nodes.size(), total);
+        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, HL.tree.segs.data(), sizeof(TreeSeg) * HL.tree.segs.size(), cudaMemcpyHostToDevice));
+        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, HL.tree.ints.data(), sizeof(int) * HL.tree.ints.size(), cudaMemcpyHostToDevice));
+        if (!s && !HL.tree.nodes.empty())
+            s = cuda_status(cudaMemcpy(b->d_tnodes, HL.tree.nodes.data(), sizeof(TreeNode) * HL.tree.nodes.size(), cudaMemcpyHostToDevice));
     }
     if (!s) s = dalloc(&b->d_desc, n, total);
     if (!s) s = dalloc(&b->d_nodes, nodes, total);

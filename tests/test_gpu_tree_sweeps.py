@@ -81,3 +81,35 @@ def test_beside_a_turn_subgame(mtt, wl, cuda, alternate):
         (one,), r, _ = _solve(mtt, [subs[k]], p, True, [0])
         _same(both[k], one)
         assert np.array_equal(res[k], r[0])
+
+
+@pytest.mark.parametrize("algo", [0, 1])
+@pytest.mark.parametrize("semantics", [0, 1])
+def test_four_player_small_batches_equal_level_launches(mtt, wl, cuda, algo, semantics):
+    """Four-player subgames of one batch past the tree sweeps' limit (1,776
+    CTAs) and on their own."""
+    import importlib
+    mw = importlib.import_module("mtt-gpu-solver_b200.multiway")
+    subs = [wl.multiway_icm(seed=4 + k, n_hands=1000 - 37 * k, raise_cap=2) for k in range(5)]
+    subs += [wl.multiway_icm(seed=20, n_hands=3, raise_cap=1), wl.multiway_icm(seed=21, n_hands=129, raise_cap=1)]
+    p = mtt.solve_params(iters=5, algo=algo, semantics=semantics)
+
+    def solve(gs, graph):
+        b = mw.MultiwayBatch(gs)
+        b.solve(p, graph=graph)
+        out = [b.read(s) for s in range(b.n)]
+        v = b.values()
+        b.solve(p, graph=graph)                       # again from zero, after the values pass
+        for s in range(b.n):
+            assert all(np.array_equal(x, y) for x, y in zip(out[s]["R"], b.read(s)["R"]))
+        b.close()
+        return out, v
+
+    many, mv = solve(subs, True)
+    for k in (0, 4, 5, 6):
+        for graph in (False, True):
+            (one,), v = solve([subs[k]], graph)
+            for q in range(4):
+                assert np.array_equal(many[k]["R"][q].view(np.uint32), one["R"][q].view(np.uint32))
+                assert np.array_equal(many[k]["S"][q].view(np.uint32), one["S"][q].view(np.uint32))
+            assert np.array_equal(many[k]["cfv"], one["cfv"]) and np.array_equal(mv[k], v[0])
