@@ -1247,22 +1247,67 @@ __global__ void __launch_bounds__(LV_HANDS) k_leaf_values(SolveDev a, const Leaf
 // -cfv1 at the root (zero-sum payoffs), and for a node of player p
 //   dEV0/dlogit_a(h) = sgn_p * reach_p(h) * sigma_a(h) * (cfv_p(child a, h) - cfv_p(node, h)),
 // sgn_0 = +1, sgn_1 = -1.
-__device__ __forceinline__ void softmax_groups(const float4* Lb, int H4, int g, int A, float4& mx, float4& den) {
-    mx = Lb[g];
+// sigma of one float4 group over A actions, every logit read and every
+// exponential taken once: s[k] = exp(l_k - max) / sum, the sum in action order.
+template <int A>
+__device__ __forceinline__ void softmax_fixed(const float4* Lb, int H4, float4 (&s)[A]) {
+    float4 mx, den = f4(0.f);
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+        s[k] = Lb[(size_t)k * H4];
+        mx = k == 0 ? s[0] : make_float4(fmaxf(mx.x, s[k].x), fmaxf(mx.y, s[k].y), fmaxf(mx.z, s[k].z), fmaxf(mx.w, s[k].w));
+    }
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+        s[k] = make_float4(expf(s[k].x - mx.x), expf(s[k].y - mx.y), expf(s[k].z - mx.z), expf(s[k].w - mx.w));
+        den = add4(den, s[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < A; ++k)
+        s[k] = make_float4(__fdiv_rn(s[k].x, den.x), __fdiv_rn(s[k].y, den.y), __fdiv_rn(s[k].z, den.z),
+                           __fdiv_rn(s[k].w, den.w));
+}
+// The same for any action count, recomputed per action instead of held.
+__device__ __forceinline__ void softmax_groups(const float4* Lb, int H4, int A, float4& mx, float4& den) {
+    mx = Lb[0];
     for (int k = 1; k < A; ++k) {
-        const float4 l = Lb[(size_t)k * H4 + g];
+        const float4 l = Lb[(size_t)k * H4];
         mx = make_float4(fmaxf(mx.x, l.x), fmaxf(mx.y, l.y), fmaxf(mx.z, l.z), fmaxf(mx.w, l.w));
     }
     den = f4(0.f);
     for (int k = 0; k < A; ++k) {
-        const float4 l = Lb[(size_t)k * H4 + g];
+        const float4 l = Lb[(size_t)k * H4];
         den = add4(den, make_float4(expf(l.x - mx.x), expf(l.y - mx.y), expf(l.z - mx.z), expf(l.w - mx.w)));
     }
 }
-__device__ __forceinline__ float4 softmax_at(const float4* Lb, int H4, int g, int k, float4 mx, float4 den) {
-    const float4 l = Lb[(size_t)k * H4 + g];
+__device__ __forceinline__ float4 softmax_at(const float4* Lb, int H4, int k, float4 mx, float4 den) {
+    const float4 l = Lb[(size_t)k * H4];
     return make_float4(__fdiv_rn(expf(l.x - mx.x), den.x), __fdiv_rn(expf(l.y - mx.y), den.y),
                        __fdiv_rn(expf(l.z - mx.z), den.z), __fdiv_rn(expf(l.w - mx.w), den.w));
+}
+
+template <int A>
+__device__ __forceinline__ void ev_reach_fixed(const float4* Lb, float4 r, float4* ch, int H4, int HS4) {
+    float4 s[A];
+    softmax_fixed<A>(Lb, H4, s);
+#pragma unroll
+    for (int k = 0; k < A; ++k) ch[(size_t)k * HS4] = mul4(r, s[k]);
+}
+
+// The acting player's value, and the logit gradients sr * sigma_k * (q_k - v).
+template <int A>
+__device__ __forceinline__ float4 ev_update_fixed(const float4* Lb, const float4* qc, float4 sr, float4* Gb, int H4, int HS4) {
+    float4 s[A], q[A], v = f4(0.f);
+#pragma unroll
+    for (int k = 0; k < A; ++k) q[k] = qc[(size_t)k * HS4];
+    softmax_fixed<A>(Lb, H4, s);
+#pragma unroll
+    for (int k = 0; k < A; ++k) v = fma4(s[k], q[k], v);
+#pragma unroll
+    for (int k = 0; k < A; ++k)
+        Gb[(size_t)k * H4] = mul4(mul4(sr, s[k]), make_float4(__fsub_rn(q[k].x, v.x), __fsub_rn(q[k].y, v.y),
+                                                              __fsub_rn(q[k].z, v.z), __fsub_rn(q[k].w, v.w)));
+    return v;
 }
 
 __global__ void k_ev_init(SolveDev a, int n_sub) {
@@ -1300,10 +1345,19 @@ __device__ __forceinline__ void k_ev_fwd_group(const SolveDev& a, const FwdItem&
         return;
     }
     const float4* Lb = reinterpret_cast<const float4*>(a.R + it.rows);
-    float4 mx, den;
-    softmax_groups(Lb, H4, g, A, mx, den);
     const float4 r = rp[g];
-    for (int k = 0; k < A; ++k) ch[(size_t)k * HS4 + g] = mul4(r, softmax_at(Lb, H4, g, k, mx, den));
+    Lb += g;
+    ch += g;
+    switch (A) {
+        case 2: ev_reach_fixed<2>(Lb, r, ch, H4, HS4); return;
+        case 3: ev_reach_fixed<3>(Lb, r, ch, H4, HS4); return;
+        case 4: ev_reach_fixed<4>(Lb, r, ch, H4, HS4); return;
+        case 5: ev_reach_fixed<5>(Lb, r, ch, H4, HS4); return;
+        default: break;
+    }
+    float4 mx, den;
+    softmax_groups(Lb, H4, A, mx, den);
+    for (int k = 0; k < A; ++k) ch[(size_t)k * HS4] = mul4(r, softmax_at(Lb, H4, k, mx, den));
 }
 
 // One warp per work item; the item covers span x 32 float4 hand groups.
@@ -1350,21 +1404,28 @@ __device__ __forceinline__ void k_ev_bwd_group(const SolveDev& a, const BwdItem&
         out[g] = so;
         return;
     }
-    const float4* Lb = reinterpret_cast<const float4*>(a.R + it.rows);
-    float4* Gb = reinterpret_cast<float4*>(a.S + it.rows);
-    float4 mx, den;
-    softmax_groups(Lb, H4, g, A, mx, den);
-    float4 v = f4(0.f);
-    for (int k = 0; k < A; ++k) v = fma4(softmax_at(Lb, H4, g, k, mx, den), qc[(size_t)k * HS4 + g], v);
-    out[g] = v;
+    const float4* Lb = reinterpret_cast<const float4*>(a.R + it.rows) + g;
+    float4* Gb = reinterpret_cast<float4*>(a.S + it.rows) + g;
     const float4 r = reinterpret_cast<const float4*>(a.arena + it.hc)[g];
     const float sgn = it.flags & BI_NEG ? -1.0f : 1.0f;
     const float4 sr = mul4(r, f4(sgn));
+    qc += g;
+    switch (A) {
+        case 2: out[g] = ev_update_fixed<2>(Lb, qc, sr, Gb, H4, HS4); return;
+        case 3: out[g] = ev_update_fixed<3>(Lb, qc, sr, Gb, H4, HS4); return;
+        case 4: out[g] = ev_update_fixed<4>(Lb, qc, sr, Gb, H4, HS4); return;
+        case 5: out[g] = ev_update_fixed<5>(Lb, qc, sr, Gb, H4, HS4); return;
+        default: break;
+    }
+    float4 mx, den;
+    softmax_groups(Lb, H4, A, mx, den);
+    float4 v = f4(0.f);
+    for (int k = 0; k < A; ++k) v = fma4(softmax_at(Lb, H4, k, mx, den), qc[(size_t)k * HS4], v);
+    out[g] = v;
     for (int k = 0; k < A; ++k) {
-        const float4 sg = softmax_at(Lb, H4, g, k, mx, den);
-        const float4 d = make_float4(__fsub_rn(qc[(size_t)k * HS4 + g].x, v.x), __fsub_rn(qc[(size_t)k * HS4 + g].y, v.y),
-                                     __fsub_rn(qc[(size_t)k * HS4 + g].z, v.z), __fsub_rn(qc[(size_t)k * HS4 + g].w, v.w));
-        Gb[(size_t)k * H4 + g] = mul4(mul4(sr, sg), d);
+        const float4 sg = softmax_at(Lb, H4, k, mx, den), q = qc[(size_t)k * HS4];
+        Gb[(size_t)k * H4] = mul4(mul4(sr, sg), make_float4(__fsub_rn(q.x, v.x), __fsub_rn(q.y, v.y), __fsub_rn(q.z, v.z),
+                                                            __fsub_rn(q.w, v.w)));
     }
 }
 
@@ -2139,8 +2200,17 @@ static int launch_tree(const mtt_batch* b, const ListSet& L, const SolveDev& a, 
     return MTT_OK;
 }
 
+// Both players' values of a large batch (its groups do not fit one wave) take
+// a launch per player: the one-player kernel values sibling terminals with
+// one scan and folds its choices, 2.70 ms for both players on the 4,096-
+// subgame batch against 3.45 ms for the two-player kernel, which is left to
+// small batches, where the second launch would cost more.
 static int launch_term(const mtt_batch* b, const ListSet& L, const SolveDev& a, int upd, cudaStream_t st,
                        bool chained = false) {
+    if (upd == 3 && L.tb_start.size() > 1) {
+        MTT_TRY(launch_term(b, L, a, 1, st, chained));
+        return launch_term(b, L, a, 2, st, false);
+    }
     for (size_t k = 0; k < L.tb_start.size(); ++k) {
         if (L.tb_count[k] == 0) continue;
         const int smem = upd == 3 ? L.tb_smem3[k] : L.tb_smem1[k];

@@ -43,8 +43,8 @@ class _EVFunction:
                 def backward(ctx, grad_ev):
                     g_r, g_l = ctx.saved_tensors
                     o = ctx.owner
-                    gl = g_l * grad_ev[o.seg_rows] if ctx.needs_input_grad[0] else None
-                    gr = g_r * grad_ev[o.seg_range] if ctx.needs_input_grad[1] else None
+                    gl = o._scale(g_l, grad_ev, "rows") if ctx.needs_input_grad[0] else None
+                    gr = o._scale(g_r, grad_ev, "range") if ctx.needs_input_grad[1] else None
                     return gl, gr, None
 
             cls.fn = EVFn
@@ -66,17 +66,15 @@ class StrategyEV:
         self.n = self.batch.n
         self.total_rows, self.total_range = lay["total_rows"], lay["total_range"]
         self.rows_off, self.range_off = lay["rows_off"], lay["range_off"]
-        seg_rows = np.zeros(self.total_rows, np.int64)
-        seg_range = np.zeros(self.total_range, np.int64)
+        self._len_rows, self._len_range = [], []      # packed elements of each subgame
         idx_r = [[], []]          # packed range index of every (subgame, combo) pair, per player
         sub_r = [[], []]
         cmb_r = [[], []]
         for s in range(self.n):
             rows0, rows1, H0, H1 = self.batch.meta[s]
             Hp = [(H0 + 3) // 4 * 4, (H1 + 3) // 4 * 4]
-            seg_rows[self.rows_off[s, 0]:self.rows_off[s, 0] + rows0 * Hp[0]] = s
-            seg_rows[self.rows_off[s, 1]:self.rows_off[s, 1] + rows1 * Hp[1]] = s
-            seg_range[self.range_off[s]:self.range_off[s] + Hp[0] + Hp[1]] = s
+            self._len_rows.append(rows0 * Hp[0] + rows1 * Hp[1])
+            self._len_range.append(Hp[0] + Hp[1])
             for p in range(2):
                 c = self.batch.combos[s][p]
                 base = self.range_off[s] + (Hp[0] if p else 0)
@@ -84,10 +82,32 @@ class StrategyEV:
                 sub_r[p].append(np.full(len(c), s))
                 cmb_r[p].append(c)
         t = lambda a: torch.from_numpy(np.concatenate(a) if isinstance(a, list) else a).to(self.device)
-        self.seg_rows, self.seg_range = t(seg_rows), t(seg_range)
         self._ridx = [t(idx_r[p]) for p in range(2)]
         self._rsub = [t(sub_r[p]) for p in range(2)]
         self._rcmb = [t(cmb_r[p]) for p in range(2)]
+        self._rflat = [self._rsub[p] * 1326 + self._rcmb[p] for p in range(2)]
+        # the index per element: made here where the scaling reads it, otherwise
+        # (equal lengths) when asked for
+        self._seg = {}
+        if len(set(self._len_rows)) > 1:
+            self._segments("rows", self._len_rows)
+        if len(set(self._len_range)) > 1:
+            self._segments("range", self._len_range)
+
+    def _segments(self, name, lengths):
+        import torch
+        if name not in self._seg:
+            self._seg[name] = torch.repeat_interleave(torch.arange(self.n, device=self.device),
+                                                      torch.tensor(lengths, device=self.device))
+        return self._seg[name]
+
+    @property
+    def seg_rows(self):
+        return self._segments("rows", self._len_rows)
+
+    @property
+    def seg_range(self):
+        return self._segments("range", self._len_range)
 
     def pack_ranges(self, r0, r1):
         """[n, 1326] range vectors (combo ids 0..1325) -> packed [total_range].
@@ -95,8 +115,22 @@ class StrategyEV:
         import torch
         out = torch.zeros(self.total_range, dtype=torch.float32, device=self.device)
         for p, r in enumerate((r0, r1)):
-            out = out.index_put((self._ridx[p],), r[self._rsub[p], self._rcmb[p]].float())
+            if r.dim() == 2 and r.shape[1] == 1326 and r.shape[0] >= self.n:
+                # every combo is read once, so the gradient needs no sorted sum:
+                # indexing's took 0.24 ms a player on 1,024 boards
+                v = r.reshape(-1).gather(0, self._rflat[p])
+            else:
+                v = r[self._rsub[p], self._rcmb[p]]
+            out = out.index_put((self._ridx[p],), v.float())
         return out
+
+    def _scale(self, g, grad_ev, name):
+        """g times its subgame's entry of grad_ev; where the subgames' parts
+        are equally long, without reading an index per element."""
+        lengths = self._len_rows if name == "rows" else self._len_range
+        if len(set(lengths)) == 1 and g.numel():
+            return (g.view(self.n, -1) * grad_ev.unsqueeze(-1)).view(g.shape)
+        return g * grad_ev[self.seg_rows if name == "rows" else self.seg_range]
 
     def unpack_rows(self, packed, s):
         """Subgame s's part of a rows-layout tensor: ([rows0, H0], [rows1, H1])."""
