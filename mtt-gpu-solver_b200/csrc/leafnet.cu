@@ -34,6 +34,7 @@ constexpr int INP = 2752, OUTP = 2688;       // padded widths
 constexpr int NL = 4;
 constexpr int DIN[NL] = {INP, HID, HID, HID};
 constexpr int DOUT[NL] = {HID, HID, HID, OUTP};
+static_assert(INP % 64 == 0 && HID % 64 == 0 && OUTP % 32 == 0, "whole Adam tiles");
 enum { F_RELU = 1, F_OUT_BF16 = 2, F_MASK = 4 };
 
 typedef __nv_bfloat16 bf16;
@@ -113,45 +114,79 @@ __global__ void __launch_bounds__(CS_COLS * CS_SLICES) k_colsum(const bf16* __re
     }
 }
 
-// Adam on FP32 masters; refreshes the BF16 copy W [rows][cols] (and, in a
-// second kernel, W^T).  Padding rows/columns stay zero.
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                       long long n, float lr, float b1, float b2, float eps, float c1, float c2,
-                       bf16* __restrict__ wb, const unsigned char* __restrict__ live) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (live && !live[i]) { wb[i] = __float2bfloat16_rn(0.0f); return; }
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    wb[i] = __float2bfloat16_rn(wi);
-}
-
-__global__ void k_adam_bias(float* __restrict__ b, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ g, int n, int n_live, float lr, float b1, float b2, float eps,
-                            float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (i >= n_live) { b[i] = 0.0f; return; }
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    b[i] = b[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
 struct Layer {
     float *w = nullptr, *b = nullptr, *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
     float *gw = nullptr, *gb = nullptr;
     bf16 *wb = nullptr, *wt = nullptr;       // W [out][in] and W^T [in][out]
-    unsigned char* live = nullptr;           // 1 where (out, in) is inside the unpadded shape
     int in = 0, out = 0, in_live = 0, out_live = 0;
 };
+
+struct AdamStep { float lr, b1, b2, eps, c1, c2; };
+
+__device__ __forceinline__ float adam1(float w, float& m, float& v, float g, const AdamStep& s) {
+    // the moments' contractions are written out: a trained network must not
+    // depend on which product the compiler fuses
+    const float mi = __fmaf_rn(1.0f - s.b1, g, __fmul_rn(s.b1, m));
+    const float vi = __fmaf_rn(__fmul_rn(1.0f - s.b2, g), g, __fmul_rn(s.b2, v));
+    m = mi;
+    v = vi;
+    return w - s.lr * (mi / s.c1) / (sqrtf(vi / s.c2) + s.eps);
+}
+
+// Adam on the FP32 masters of all layers in one launch; refreshes the BF16
+// copies W and W^T of the same tile (32 outputs x 64 inputs a CTA, transposed
+// through shared memory).  Elements outside a layer's live shape stay zero.
+// Bound by HBM: 30 bytes a weight, 0.23 GB a step.  A launch per layer for the
+// weights, one for the biases and one for the transpose took 95 us a step.
+constexpr int AD_OUT = 32, AD_IN = 64;
+struct AdamNet {
+    Layer l[NL];
+    int tile0[NL + 1];        // first CTA of each layer's tiles; the last CTAs take the biases
+};
+__global__ void __launch_bounds__(256) k_adam(AdamNet net, AdamStep st) {
+    __shared__ __align__(16) bf16 t[AD_IN][AD_OUT + 8];
+    const int tid = threadIdx.x;
+    int b = blockIdx.x;
+    if (b >= net.tile0[NL]) {                                  // one CTA per layer's biases
+        const Layer& L = net.l[b - net.tile0[NL]];
+        for (int i = tid; i < L.out; i += 256) {
+            if (i >= L.out_live) { L.b[i] = 0.0f; continue; }
+            float m = L.mb[i], v = L.vb[i];
+            L.b[i] = adam1(L.b[i], m, v, L.gb[i], st);
+            L.mb[i] = m;
+            L.vb[i] = v;
+        }
+        return;
+    }
+    int k = 0;
+    while (b >= net.tile0[k + 1]) ++k;
+    b -= net.tile0[k];
+    const Layer& L = net.l[k];
+    const int tiles = L.in / AD_IN, o0 = b / tiles * AD_OUT, i0 = b % tiles * AD_IN;
+    const int c = (tid & 15) * 4;
+#pragma unroll
+    for (int r = tid >> 4; r < AD_OUT; r += 16) {
+        const int o = o0 + r, i = i0 + c;
+        const size_t e = (size_t)o * L.in + i;
+        float4 w = *reinterpret_cast<float4*>(L.w + e), m = *reinterpret_cast<float4*>(L.mw + e);
+        float4 v = *reinterpret_cast<float4*>(L.vw + e);
+        const float4 g = *reinterpret_cast<const float4*>(L.gw + e);
+        const bool row = o < L.out_live;
+        if (row && i < L.in_live) w.x = adam1(w.x, m.x, v.x, g.x, st);
+        if (row && i + 1 < L.in_live) w.y = adam1(w.y, m.y, v.y, g.y, st);
+        if (row && i + 2 < L.in_live) w.z = adam1(w.z, m.z, v.z, g.z, st);
+        if (row && i + 3 < L.in_live) w.w = adam1(w.w, m.w, v.w, g.w, st);
+        *reinterpret_cast<float4*>(L.w + e) = w;
+        *reinterpret_cast<float4*>(L.mw + e) = m;
+        *reinterpret_cast<float4*>(L.vw + e) = v;
+        const __nv_bfloat162 x = __floats2bfloat162_rn(w.x, w.y), y = __floats2bfloat162_rn(w.z, w.w);
+        *reinterpret_cast<uint2*>(L.wb + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&x), *reinterpret_cast<const uint32_t*>(&y));
+        t[c][r] = x.x; t[c + 1][r] = x.y; t[c + 2][r] = y.x; t[c + 3][r] = y.y;
+    }
+    __syncthreads();
+    const int q = tid >> 2, h = (tid & 3) * 8;                 // 8 outputs of input i0 + q
+    *reinterpret_cast<uint4*>(L.wt + (size_t)(i0 + q) * L.out + o0 + h) = *reinterpret_cast<const uint4*>(&t[q][h]);
+}
 
 }  // namespace leaf
 }  // namespace mtt
@@ -184,7 +219,7 @@ void free_net(mtt_leafnet* n) {
     if (!n) return;
     for (Layer& l : n->L) {
         cudaFree(l.w); cudaFree(l.b); cudaFree(l.mw); cudaFree(l.vw); cudaFree(l.mb); cudaFree(l.vb);
-        cudaFree(l.gw); cudaFree(l.gb); cudaFree(l.wb); cudaFree(l.wt); cudaFree(l.live);
+        cudaFree(l.gw); cudaFree(l.gb); cudaFree(l.wb); cudaFree(l.wt);
     }
     cudaFree(n->X0); cudaFree(n->dY); cudaFree(n->T1); cudaFree(n->T2); cudaFree(n->Y); cudaFree(n->partial);
     cudaFree(n->err); cudaFree(n->ws);
@@ -288,14 +323,12 @@ extern "C" int mtt_leafnet_create(int32_t batch_cap, uint64_t seed, int32_t flag
         L.in = DIN[l]; L.out = DOUT[l]; L.in_live = in_live[l]; L.out_live = out_live[l];
         const size_t cnt = (size_t)L.in * L.out;
         std::vector<float> w(cnt, 0.0f);
-        std::vector<unsigned char> live(cnt, 0);
         // He initialisation; the output layer starts at zero when asked
         const double sd = (l == NL - 1 && (flags & MTT_LEAF_ZERO_OUTPUT)) ? 0.0 : std::sqrt(2.0 / (double)L.in_live);
         for (int o = 0; o < L.out_live; ++o)
             for (int i = 0; i < L.in_live; ++i) {
                 const double u1 = urand(), u2 = urand();
                 w[(size_t)o * L.in + i] = (float)(sd * std::sqrt(-2.0 * std::log(u1)) * std::cos(6.283185307179586 * u2));
-                live[(size_t)o * L.in + i] = 1;
             }
         if (!s) s = dmalloc(&L.w, cnt);
         if (!s) s = dmalloc(&L.mw, cnt);
@@ -303,13 +336,11 @@ extern "C" int mtt_leafnet_create(int32_t batch_cap, uint64_t seed, int32_t flag
         if (!s) s = dmalloc(&L.gw, cnt);
         if (!s) s = dmalloc(&L.wb, cnt);
         if (!s) s = dmalloc(&L.wt, cnt);
-        if (!s) s = dmalloc(&L.live, cnt);
         if (!s) s = dmalloc(&L.b, L.out);
         if (!s) s = dmalloc(&L.mb, L.out);
         if (!s) s = dmalloc(&L.vb, L.out);
         if (!s) s = dmalloc(&L.gb, L.out);
         if (!s) s = cuda_status(cudaMemcpy(L.w, w.data(), 4 * cnt, cudaMemcpyHostToDevice));
-        if (!s) s = cuda_status(cudaMemcpy(L.live, live.data(), cnt, cudaMemcpyHostToDevice));
         if (!s) s = cuda_status(cudaMemset(L.mw, 0, 4 * cnt));
         if (!s) s = cuda_status(cudaMemset(L.vw, 0, 4 * cnt));
         if (!s) s = cuda_status(cudaMemset(L.b, 0, 4 * (size_t)L.out));
@@ -369,17 +400,14 @@ extern "C" int mtt_leafnet_train_step(mtt_leafnet* n, const float* d_x, const fl
     n->step += 1;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = (float)(1.0 - std::pow(0.9, (double)n->step)), c2 = (float)(1.0 - std::pow(0.999, (double)n->step));
+    AdamNet net;
+    net.tile0[0] = 0;
     for (int l = 0; l < NL; ++l) {
-        Layer& L = n->L[l];
-        const long long cnt = (long long)L.in * L.out;
-        k_adam<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(L.w, L.mw, L.vw, L.gw, cnt, lr, b1, b2, eps, c1, c2, L.wb,
-                                                             L.live);
-        MTT_CHECK_LAUNCH();
-        k_adam_bias<<<(unsigned)((L.out + 255) / 256), 256, 0, st>>>(L.b, L.mb, L.vb, L.gb, L.out, L.out_live, lr, b1,
-                                                                     b2, eps, c1, c2);
-        MTT_CHECK_LAUNCH();
-        MTT_TRY(transpose(L.wb, L.out, L.in, L.in, L.wt, L.out, st));
+        net.l[l] = n->L[l];
+        net.tile0[l + 1] = net.tile0[l] + (DOUT[l] / AD_OUT) * (DIN[l] / AD_IN);
     }
+    k_adam<<<net.tile0[NL] + NL, 256, 0, st>>>(net, AdamStep{lr, b1, b2, eps, c1, c2});
+    MTT_CHECK_LAUNCH();
     return MTT_OK;
 }
 
