@@ -102,6 +102,9 @@ def validate_tree(nodes, rows):
 # ------------------------------------------------------------------ device helpers
 def _stream(stream=None):
     import torch
+    if stream is None and torch.cuda.is_initialized():
+        # the handle alone: building a Stream object took 3.5 of a small call's 11.4 us
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
 

@@ -251,7 +251,7 @@ constexpr int BC_TILE = 64, BC_WCHUNK = 32;
 __global__ void __launch_bounds__(256)
 k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
                const uint8_t* __restrict__ hands, const uint8_t* __restrict__ board, int nboard,
-               int n_const, int32_t* __restrict__ W, int32_t* __restrict__ T, int32_t* __restrict__ L) {
+               int n_const, int32_t* __restrict__ W, int32_t* __restrict__ T, int32_t* __restrict__ L, uint32_t one) {
     __shared__ alignas(16) uint32_t hk[BC_WCHUNK][BC_TILE];
     __shared__ alignas(16) uint32_t vk[BC_WCHUNK][BC_TILE];
     const int tid = threadIdx.x, ti = tid & 15, tj = tid >> 4;
@@ -280,8 +280,8 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
                     const uint32_t t = pair_2w_t(hv[a], vv[b]);
-                    sc[a][b] += t;
-                    wc[a][b] += t & 0x00020002u;
+                    sc[a][b] = add_on_fma(sc[a][b], t, one);
+                    wc[a][b] = add_on_fma(wc[a][b], t & 0x00020002u, one);
                 }
         }
         __syncthreads();
@@ -382,11 +382,11 @@ k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys) {
 // The numerator is the sum of one packed clamp per word; N is counted from the
 // hands' deck positions by inclusion and exclusion over the runout pairs (192
 // less the runouts that hold a card of either hand), so the loop spends
-// nothing on it.  Bound by the clamps and their adds: all 1,755 flops took
-// 48.8 ms with half-word compares and a popcount of usable runouts per pair.
+// nothing on it.  Bound by the clamps: all 1,755 flops took 48.8 ms with
+// half-word compares and a popcount of usable runouts per pair, 8.1 ms now.
 constexpr int FE_TH = 64, FE_TV = 64, FE_WCH = 32;
 __global__ void __launch_bounds__(256)
-k_flop_pair_eq(const uint32_t* __restrict__ keys, float* __restrict__ eqT) {
+k_flop_pair_eq(const uint32_t* __restrict__ keys, float* __restrict__ eqT, uint32_t one) {
     __shared__ alignas(16) uint32_t hk[FE_WCH][FE_TH];
     __shared__ alignas(16) uint32_t vk[FE_WCH][FE_TV];
     __shared__ uint64_t adj[49];             // bit y of adj[x]: deck positions x and y are a runout
@@ -438,7 +438,10 @@ k_flop_pair_eq(const uint32_t* __restrict__ keys, float* __restrict__ eqT) {
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) sc[a][b] += pair_2w_t(hv[a], vv[b]) + pair_2w_t(gv[a], uv[b]);
+                for (int b = 0; b < 4; ++b) {
+                    sc[a][b] = add_on_fma(sc[a][b], pair_2w_t(hv[a], vv[b]), one);
+                    sc[a][b] = add_on_fma(sc[a][b], pair_2w_t(gv[a], uv[b]), one);
+                }
         }
         __syncthreads();
     }
@@ -562,7 +565,7 @@ static int flop_ev_batched(const uint8_t* d_flops, int nflops, const float* d_re
         const uint8_t* fl = d_flops + 3 * (size_t)f0;
         k_flop_keys<<<dim3(ceil_div(FE_ALIVE, 128), n), 128, 0, st>>>(fl, keys);
         k_flop_pair_eq<<<dim3(ceil_div(FE_ALIVE, FE_TH), ceil_div(FE_VILL, FE_TV), n), 256, 0, st>>>(
-            keys, eqT);
+            keys, eqT, 1u);
         k_flop_accumulate<<<dim3(ceil_div(FE_ALIVE, 128), n), 128, 0, st>>>(
             eqT, d_reach0, d_reach1, n, d_ev0 + (size_t)f0 * FE_ALIVE, d_ev1 + (size_t)f0 * FE_ALIVE);
         s = cuda_status(cudaGetLastError());
@@ -585,7 +588,7 @@ extern "C" int mtt_eval7(const uint8_t* d_cards7, uint32_t* d_out, int64_t n, vo
         if ((reinterpret_cast<uintptr_t>(d_out) & 15u) == 0u) k_eval7_quad<true><<<grid, EV_THREADS, 0, st>>>(d_cards7, d_out, n);
         else k_eval7_quad<false><<<grid, EV_THREADS, 0, st>>>(d_cards7, d_out, n);
     } else {
-        k_eval7_plain<<<(unsigned)ceil_div_ll(n, 256), 256, 0, st>>>(d_cards7, d_out, n);
+        k_eval7_plain<<<(unsigned)ceil_div_ll(n, 64), 64, 0, st>>>(d_cards7, d_out, n);   // few hands: spread over the SMs
     }
     MTT_CHECK_LAUNCH();
     return MTT_OK;
@@ -628,7 +631,7 @@ extern "C" int mtt_board_showdown_counts(const uint8_t* d_board, int32_t nboard,
     int s = cuda_status(cudaGetLastError());
     if (s == MTT_OK) {
         k_board_counts<<<dim3(Hp / BC_TILE, Hp / BC_TILE), 256, 0, st>>>(keys, ncw, H, Hp, d_hands, d_board,
-                                                                        nboard, n_const, d_w, d_t, d_l);
+                                                                        nboard, n_const, d_w, d_t, d_l, 1u);
         s = cuda_status(cudaGetLastError());
     }
     cudaFreeAsync(keys, st);
@@ -687,7 +690,7 @@ extern "C" int mtt_board_showdown_counts_noalloc(const uint8_t* d_board, int32_t
     k_completion_keys<<<dim3(Hp / 64, ncw), 64, 0, st>>>(d_board, nboard, d_hands, H, Hp, ncomp, keys);
     MTT_TRY_CUDA(cudaGetLastError());
     k_board_counts<<<dim3(Hp / BC_TILE, Hp / BC_TILE), 256, 0, st>>>(keys, ncw, H, Hp, d_hands, d_board, nboard,
-                                                                    n_const, d_w, d_t, d_l);
+                                                                    n_const, d_w, d_t, d_l, 1u);
     MTT_TRY_CUDA(cudaGetLastError());
     return MTT_OK;
 }
