@@ -17,7 +17,6 @@
 #include <mutex>
 #include <vector>
 
-#include "mtt_bulk.cuh"
 #include "mtt_common.h"
 #include "mtt_device.cuh"
 #include "mtt_pairs.cuh"

@@ -1089,25 +1089,38 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     }
     b->n_terms = (int)tl.size();
     b->rs4 = rs / 4;
-    // whole-tree sweeps (their reason stands with k_tree): slices of 8 hands
-    // where three CTAs an SM fit, fewer where only that fits at all.  One 1,585-
-    // node subgame of 1,081 hands took 204.7 us an iteration by levels (147.6
-    // once zero regrets skip their divisions) and takes 101; two 231 / 188,
-    // four (2,176 CTAs) 376 / 371, eight 672 / 721, so larger batches keep the
-    // level kernels.
+    // whole-tree sweeps (their reason stands with k_tree): slices of 8 hands, or
+    // 16 or 32 where those still fit two CTAs an SM and the batch would
+    // otherwise need more than one such wave; fewer lanes where only that fits
+    // at all.  One 1,585-node subgame of 1,081 hands took 204.7 us an iteration
+    // by levels (147.6 once zero regrets skip their divisions) and takes 72.5 by
+    // tree: 272 CTAs, one wave, against 101 in slices of 8 hands; two subgames
+    // 231 / 144, four 376 / 286, eight (2,176 CTAs) 671 / 549.  Larger batches
+    // keep the level kernels, unmeasured.
     std::vector<TreeCta> tc;
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (fits) {
+        auto bytes = [&](const TreeSeg& g, int lg) { return tree_smem_bytes(g.n_rows, g.n_term, g.n_dec, g.n_int, lg, true); };
+        auto lanes = [&](const TreeSeg& g, int want) {
+            int lg = want;
+            while (lg > 0 && bytes(g, lg) > 112 * 1024) --lg;
+            return lg;
+        };
+        int want = 1;
+        for (; want < 3; ++want) {
+            long long n_ctas = 0;
+            for (const TreeSeg& g : th.segs) n_ctas += (g.h4 + (1 << lanes(g, want)) - 1) >> lanes(g, want);
+            if (n_ctas <= 2LL * sms) break;
+        }
         for (int i = 0; i < (int)th.segs.size(); ++i) {
             const TreeSeg& g = th.segs[i];
-            auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg, true); };
-            const int lg = bytes(3) <= 72 * 1024 ? 3 : bytes(2) <= 72 * 1024 ? 2 : bytes(1) <= 72 * 1024 ? 1 : 0;
-            b->tree_smem = std::max(b->tree_smem, bytes(lg));
+            const int lg = lanes(g, want);
+            b->tree_smem = std::max(b->tree_smem, bytes(g, lg));
             for (int g0 = 0; g0 < g.h4; g0 += 1 << lg) tc.push_back(TreeCta{i, g0, lg, 0});
         }
         b->n_ctas = (int)tc.size();
-        int sms = 148, dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        b->tree = b->n_ctas <= 12 * sms;
+        b->tree = b->n_ctas <= 16 * sms;
         if (!b->tree) b->tree_smem = 0;
     }
     int s = MTT_OK;

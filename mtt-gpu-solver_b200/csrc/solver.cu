@@ -1924,7 +1924,7 @@ static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* ac
     for (int i = 0; i < (int)H.tree.segs.size(); ++i) {
         if (active && !(*active)[H.tree.sub[i]]) continue;
         const TreeSeg& g = H.tree.segs[i];
-        auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_nodes, g.n_dec, g.n_int, lg, false); };
+        auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_term, g.n_dec, g.n_int, lg, false); };
         int lg = 1, cls = TREE_CLASSES - 1;
         if (bytes(2) <= TREE_CLASS_BYTES[0]) { cls = 0; lg = bytes(3) <= TREE_CLASS_BYTES[0] ? 3 : 2; }
         else if (bytes(1) <= TREE_CLASS_BYTES[1]) { cls = 1; lg = bytes(3) <= TREE_CLASS_BYTES[1] ? 3 : bytes(2) <= TREE_CLASS_BYTES[1] ? 2 : 1; }
@@ -2642,9 +2642,9 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     // whole-tree sweeps: batches of few hands, whose level launches are bound by
     // latency; the subgame deals no card, ends in no leaf and a slice of its
     // tree fits in shared memory.  The line is where the two met on uneven
-    // river batches (us an iteration, tree / level launches): 1 subgame 36 / 63,
-    // 8 (160 slices of 32 hands) 87 / 103, 16 101 / 109, 24 (480) 122 / 124, 32
-    // 134 / 124; larger batches fill the chip level by level, and there the
+    // river batches (us an iteration, tree / level launches): 1 subgame 37 / 63,
+    // 8 (160 slices of 32 hands) 64 / 103, 16 79 / 107, 24 (480) 134 / 124, 32
+    // 146 / 125; larger batches fill the chip level by level, and there the
     // tree's barriers cost more than the launches.
     b->tree.assign(n, 0);
     long long slices = 0;

@@ -85,7 +85,8 @@ struct alignas(16) TreeSeg {   // one player of one subgame
     int h4, hs4;          // float4 groups of the player; slot stride in float4
     int n_rows, n_nodes;
     int node0, n_dec;     // decision nodes, in backward order
-    int int0, n_int;      // integers: [nb + 1 backward bounds][nf + 1 forward bounds][own nodes in forward order][terminals]
+    int int0, n_int;      // integers: [nb + 1 backward bounds][nf + 1 forward bounds][own nodes in forward order]
+                          // [terminals][value slot of every node, two a word]
     int nb, nf, n_own, n_term;
     int pad[2];
 };
@@ -115,12 +116,14 @@ constexpr int TREE_THREADS = 256, TREE_MAX_NODES = 1 << 16;
 // float4 slots a lane: regret rows, sums, values and reach.  With simultaneous
 // updates the sums are added by the forward part, so sums and reach take the
 // place of the values once the backward part is done with them.
-__host__ __device__ inline int tree_slots(int n_rows, int n_nodes, bool sim) {
+// A decision node's value takes the slot of its first child, which only it
+// reads, so values need a slot per terminal.
+__host__ __device__ inline int tree_slots(int n_rows, int n_term, bool sim) {
     const int sr = 2 * n_rows + 1;
-    return n_rows + (sim ? (sr > n_nodes ? sr : n_nodes) : sr + n_nodes);
+    return n_rows + (sim ? (sr > n_term ? sr : n_term) : sr + n_term);
 }
-__host__ __device__ inline int tree_smem_bytes(int n_rows, int n_nodes, int n_dec, int n_int, int lg, bool sim) {
-    return (tree_slots(n_rows, n_nodes, sim) << lg) * 16 + n_dec * 16 + (n_int + 3) / 4 * 16;
+__host__ __device__ inline int tree_smem_bytes(int n_rows, int n_term, int n_dec, int n_int, int lg, bool sim) {
+    return (tree_slots(n_rows, n_term, sim) << lg) * 16 + n_dec * 16 + (n_int + 3) / 4 * 16;
 }
 
 template <int ALGO>
@@ -144,8 +147,8 @@ __device__ __forceinline__ void copy_async16(float4* dst, const float4* src) {
 // reach of its children.  A: the action count, with every row read before any
 // is used, or 0: na actions.
 template <int A, int ALGO, bool SIM>
-__device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, const float4* q, float4 r, float4* R, float4* S,
-                                              int na, int lg, int H4, const float4& tb) {
+__device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, const float4* V, const uint16_t* slot, float4 r,
+                                              float4* R, float4* S, int na, int lg, int H4, const float4& tb) {
     const int n = A ? A : na;
     const float invA = __fdiv_rn(1.0f, (float)n);
     const float4 wr = mul4(r, f4(tb.x));
@@ -153,7 +156,7 @@ __device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, cons
     if constexpr (A > 0) {
         float4 rk[A], qk[A], sg[A];
 #pragma unroll
-        for (int k = 0; k < A; ++k) { rk[k] = rs[k << lg]; qk[k] = q[k << lg]; }
+        for (int k = 0; k < A; ++k) { rk[k] = rs[k << lg]; qk[k] = V[(int)slot[k] << lg]; }
 #pragma unroll
         for (int k = 0; k < A; ++k) sum = add4(sum, max04(rk[k]));
 #pragma unroll
@@ -175,12 +178,12 @@ __device__ __forceinline__ float4 tree_update(float4* rs, const float4* ss, cons
 #pragma unroll 1
         for (int k = 0; k < n; ++k) {
             const float4 sg = rm4(max04(rs[k << lg]), sum, invA);
-            v = fma4(sg, q[k << lg], v);
+            v = fma4(sg, V[(int)slot[k] << lg], v);
             if (!SIM) S[(size_t)k * H4] = upd_sum<ALGO>(ss[k << lg], r, wr, sg, tb.w);
         }
 #pragma unroll 1
         for (int k = 0; k < n; ++k) {
-            const float4 x = upd_regret<ALGO>(rs[k << lg], q[k << lg], v, tb.y, tb.z);
+            const float4 x = upd_regret<ALGO>(rs[k << lg], V[(int)slot[k] << lg], v, tb.y, tb.z);
             R[(size_t)k * H4] = x;
             rs[k << lg] = x;
         }
@@ -223,7 +226,7 @@ __device__ __forceinline__ void tree_reach(const float4* rs, const float4* ss, f
 // then added by the forward part (of the next iteration), else by the backward
 // part.
 template <int ALGO, bool SIM>
-__global__ void __launch_bounds__(TREE_THREADS, SIM ? 3 : 2) k_tree(TreeArgs t) {
+__global__ void __launch_bounds__(TREE_THREADS, 2) k_tree(TreeArgs t) {
     extern __shared__ __align__(16) float4 tree_smem[];
     const TreeCta c = t.ctas[blockIdx.x];
     const TreeSeg sg = t.segs[c.seg];
@@ -234,12 +237,13 @@ __global__ void __launch_bounds__(TREE_THREADS, SIM ? 3 : 2) k_tree(TreeArgs t) 
     float4* const Rs = tree_smem + lane;                              // regret rows
     float4* const Ss = Rs + (n_rows << lg);                           // strategy sums
     float4* const P = Ss + (n_rows << lg);                            // reach by id
-    float4* const V = SIM ? Ss : P + ((n_rows + 1) << lg);            // values by node
-    TreeNode* const nodes = reinterpret_cast<TreeNode*>(tree_smem + (tree_slots(n_rows, sg.n_nodes, SIM) << lg));
+    float4* const V = SIM ? Ss : P + ((n_rows + 1) << lg);            // values by slot
+    TreeNode* const nodes = reinterpret_cast<TreeNode*>(tree_smem + (tree_slots(n_rows, sg.n_term, SIM) << lg));
     int* const blev = reinterpret_cast<int*>(nodes + sg.n_dec);
     int* const flev = blev + sg.nb + 1;
     int* const own = flev + sg.nf + 1;
     int* const term = own + sg.n_own;
+    const uint16_t* const slot = reinterpret_cast<const uint16_t*>(term + sg.n_term);
     for (int i = tid; i < sg.n_dec; i += TREE_THREADS) nodes[i] = t.nodes[sg.node0 + i];
     for (int i = tid; i < sg.n_int; i += TREE_THREADS) blev[i] = t.ints[sg.int0 + i];
     float4* const reach = reinterpret_cast<float4*>(t.arena + sg.reach) + g;
@@ -261,7 +265,7 @@ __global__ void __launch_bounds__(TREE_THREADS, SIM ? 3 : 2) k_tree(TreeArgs t) 
         }
         if (bwd)
             for (int i = grp; i < sg.n_term; i += groups)
-                copy_async16(V + (term[i] << lg), cfv + (size_t)term[i] * HS4);
+                copy_async16(V + (i << lg), cfv + (size_t)term[i] * HS4);
         if (!SIM && bwd)
             for (int i = grp; i < sg.n_own; i += groups) {
                 const TreeNode nd = nodes[own[i]];
@@ -278,13 +282,13 @@ __global__ void __launch_bounds__(TREE_THREADS, SIM ? 3 : 2) k_tree(TreeArgs t) 
             for (int i = blev[l] + grp; live && i < hi; i += groups) {
                 const TreeNode nd = nodes[i];
                 const int na = nd.w & 31, self = nd.y & 0xFFFF;
-                const float4* const q = V + (nd.x << lg);
+                const uint16_t* const cs = slot + nd.x;
                 float4 v = f4(0.f);
                 if (nd.w & 32) {
                     const int row = (int)((unsigned)nd.w >> 6);
                     const float4 r = SIM ? f4(0.f) : P[(int)((unsigned)nd.y >> 16) << lg];
 #define TREE_CALL(A) \
-    v = tree_update<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), q, r, R + (size_t)row * H4, S + (size_t)row * H4, na, lg, \
+    v = tree_update<A, ALGO, SIM>(Rs + (row << lg), Ss + (row << lg), V, cs, r, R + (size_t)row * H4, S + (size_t)row * H4, na, lg, \
                                   H4, tb)
                     switch (na) {
                         case 2: TREE_CALL(2); break;
@@ -295,9 +299,9 @@ __global__ void __launch_bounds__(TREE_THREADS, SIM ? 3 : 2) k_tree(TreeArgs t) 
 #undef TREE_CALL
                 } else {
 #pragma unroll 4
-                    for (int k = 0; k < na; ++k) v = add4(v, q[k << lg]);
+                    for (int k = 0; k < na; ++k) v = add4(v, V[(int)cs[k] << lg]);
                 }
-                V[self << lg] = v;
+                V[(int)cs[0] << lg] = v;
                 cfv[(size_t)self * HS4] = v;
             }
             __syncthreads();
@@ -366,7 +370,7 @@ inline int tree_min_bytes(int n_nodes, int n_rows, int q, int lg, bool sim, Node
         own += nd.dec && nd.player == q;
     }
     // at most one level per node
-    return tree_smem_bytes(n_rows, n_nodes, dec, 2 * (dec + 1) + own + n_nodes - dec, lg, sim);
+    return tree_smem_bytes(n_rows, n_nodes - dec, dec, 2 * (dec + 1) + own + n_nodes - dec + (n_nodes + 1) / 2, lg, sim);
 }
 
 // One player's view of a chance-free tree: the backward order (all decision
@@ -417,8 +421,12 @@ inline void build_tree_seg(TreeHost& L, TreeSeg g, int sub, int q, Node node) {
     L.ints.push_back((int)own.size());
     g.n_own = (int)own.size();
     L.ints.insert(L.ints.end(), own.begin(), own.end());
+    std::vector<uint16_t> slot(n + (n & 1), 0);
     for (int k = 0; k < n; ++k)
-        if (!nd[k].dec) { L.ints.push_back(k); ++g.n_term; }
+        if (!nd[k].dec) { slot[k] = (uint16_t)g.n_term++; L.ints.push_back(k); }
+    for (int k = n - 1; k >= 0; --k)               // children follow their parents
+        if (nd[k].dec) slot[k] = slot[nd[k].first];
+    for (int k = 0; k < n; k += 2) L.ints.push_back((int)((unsigned)slot[k] | (unsigned)slot[k + 1] << 16));
     g.n_int = (int)L.ints.size() - g.int0;
     L.segs.push_back(g);
     L.sub.push_back(sub);

@@ -86,11 +86,12 @@ def test_beside_a_turn_subgame(mtt, wl, cuda, alternate):
 @pytest.mark.parametrize("algo", [0, 1])
 @pytest.mark.parametrize("semantics", [0, 1])
 def test_four_player_small_batches_equal_level_launches(mtt, wl, cuda, algo, semantics):
-    """Four-player subgames of one batch past the tree sweeps' limit (1,776
-    CTAs) and on their own."""
+    """Four-player subgames of one batch past the tree sweeps' limit (2,368
+    CTAs of 16 hands of one player) and on their own."""
     import importlib
     mw = importlib.import_module("mtt-gpu-solver_b200.multiway")
-    subs = [wl.multiway_icm(seed=4 + k, n_hands=1000 - 37 * k, raise_cap=2) for k in range(5)]
+    subs = [wl.multiway_icm(seed=4 + k, n_hands=1050 - 11 * k, raise_cap=2) for k in range(13)]
+    assert sum(4 * ((len(g["combos"]) + 15) // 16) for g in subs) > 2368
     subs += [wl.multiway_icm(seed=20, n_hands=3, raise_cap=1), wl.multiway_icm(seed=21, n_hands=129, raise_cap=1)]
     p = mtt.solve_params(iters=5, algo=algo, semantics=semantics)
 
@@ -106,7 +107,7 @@ def test_four_player_small_batches_equal_level_launches(mtt, wl, cuda, algo, sem
         return out, v
 
     many, mv = solve(subs, True)
-    for k in (0, 4, 5, 6):
+    for k in (0, 12, 13, 14):
         for graph in (False, True):
             (one,), v = solve([subs[k]], graph)
             for q in range(4):
