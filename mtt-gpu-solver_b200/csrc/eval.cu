@@ -85,11 +85,7 @@ __global__ void k_eval7_plain(const uint8_t* __restrict__ cards, uint32_t* __res
                               long long n) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint8_t* c = cards + 7 * i;
-    Planes p; planes_clear(p);
-#pragma unroll
-    for (int k = 0; k < 7; ++k) planes_add(p, c[k]);
-    out[i] = score_planes(p);
+    out[i] = score7(cards + 7 * i);
 }
 
 static int sm_count(int* out) {
@@ -142,15 +138,16 @@ k_enumerate7(unsigned long long* __restrict__ hist, unsigned long long* __restri
         int c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3], c4 = c[4], c5 = c[5], c6 = c[6];
         const unsigned long long end = min((unsigned long long)N_HANDS7, idx + ENUM_CHUNK);
         for (; idx < end; ++idx) {
-            Planes p; planes_clear(p);
-            planes_add(p, c0); planes_add(p, c1); planes_add(p, c2); planes_add(p, c3);
-            planes_add(p, c4); planes_add(p, c5); planes_add(p, c6);
-            const uint32_t s = score_planes(p);
+            const int hand[7] = {c0, c1, c2, c3, c4, c5, c6};
+            const uint32_t s = score7(hand);
             const uint32_t cat = s >> 24;
 #pragma unroll
             for (int k = 0; k < 9; ++k) cnt[k] += (cat == (uint32_t)k) ? 1u : 0u;
             cs += (unsigned long long)s * (idx + 1ull);
             if (key_table) {
+                Planes p; planes_clear(p);
+#pragma unroll
+                for (int k = 0; k < 7; ++k) planes_add(p, hand[k]);
                 const uint32_t key = key_planes(p);
                 if (key_table[key] != s) {
                     const uint32_t old = atomicCAS(&key_table[key], 0xFFFFFFFFu, s);
