@@ -2,6 +2,7 @@
 // the whole-tree sweep kernel, shared by the heads-up and four-player solvers.
 #pragma once
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <vector>
@@ -361,13 +362,22 @@ struct TreeHost {
 };
 
 // Shared memory of the smallest slice (4 << lg hands) of one player's tree.
+// Past any limit where two nodes share regret rows: a level launch adds both
+// nodes' sums to them, one level after the other, while a slice stages the sums
+// once and numbers its reach by row.
 template <typename Node>
 inline int tree_min_bytes(int n_nodes, int n_rows, int q, int lg, bool sim, Node node) {
     int dec = 0, own = 0;
+    std::vector<char> used(n_rows, 0);
     for (int k = 0; k < n_nodes; ++k) {
         const TreeShapeNode nd = node(k);
         dec += nd.dec;
-        own += nd.dec && nd.player == q;
+        if (!nd.dec || nd.player != q) continue;
+        ++own;
+        for (int a = 0; a < nd.na; ++a) {
+            if (used[nd.row + a]) return INT_MAX;
+            used[nd.row + a] = 1;
+        }
     }
     // at most one level per node
     return tree_smem_bytes(n_rows, n_nodes - dec, dec, 2 * (dec + 1) + own + n_nodes - dec + (n_nodes + 1) / 2, lg, sim);

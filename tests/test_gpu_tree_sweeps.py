@@ -42,6 +42,34 @@ def test_small_batches_equal_level_launches(mtt, wl, cuda, algo, alternate, sema
             assert np.array_equal(wres[k], gres[n])
 
 
+@pytest.mark.parametrize("alternate", [True, False])
+def test_nodes_that_share_rows_equal_level_launches(mtt, wl, cuda, alternate):
+    """A caller's tree in which a node uses its ancestor's regret rows: one
+    level works on them after the other, in small batches as in large ones."""
+    subs = wl.river_batch(n=40, seed=17, min_support=350, max_support=700)
+    g = max(subs, key=lambda s: len(s["nodes"]))
+    nodes = g["nodes"].copy()
+    parent = np.full(len(nodes), -1)
+    for i, nd in enumerate(nodes):
+        if nd["type"] == 0:
+            parent[nd["children_offset"]:nd["children_offset"] + nd["num_actions"]] = i
+    shared = 0
+    for i, nd in enumerate(nodes):
+        a = parent[i]
+        while nd["type"] == 0 and a >= 0 and not shared:
+            if nodes[a]["player"] == nd["player"] and nodes[a]["num_actions"] >= nd["num_actions"]:
+                nodes[i]["infoset_offset"] = nodes[a]["infoset_offset"]
+                shared += 1
+            a = parent[a]
+    assert shared == 1
+    g["nodes"] = nodes
+    k = next(i for i, s in enumerate(subs) if s is g)
+    p = mtt.solve_params(iters=7, alternate=alternate)
+    want, _, _ = _solve(mtt, subs, p, True, [k])
+    got, _, _ = _solve(mtt, [g], p, True, [0])
+    _same(want[k], got[0])
+
+
 @pytest.mark.parametrize("hands", [1, 3, 31, 33, 128])
 def test_slice_edges(mtt, wl, orc, cuda, hands):
     g = wl.river_uniform(seed=hands, n_hands=hands, raise_cap=2)
