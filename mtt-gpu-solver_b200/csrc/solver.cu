@@ -1970,7 +1970,9 @@ static int build_set(mtt_batch* b, ListSet& L, const std::vector<char>* active, 
         MTT_TRY(upload_levels(L.f_alt[u], H.fal[u], all_sweep, fkeep, total));
         MTT_TRY(upload_levels(L.b_alt[u], H.bal[u], all_sweep, bkeep, total));
     }
-    L.levels_too = L.f_sim.off.back() > 0;
+    // a subgame that is one depth-limit leaf has no level items, but its values are the levels' work too
+    L.levels_too = false;
+    for (int i = 0; i < b->n; ++i) L.levels_too |= (!active || (*active)[i]) && !b->tree[i];
     MTT_TRY(upload_levels(L.br_fwd, H.bf, !active, tkeep, total));
     MTT_TRY(upload_levels(L.br_bwd, H.bb, !active, tkeep, total));
     std::vector<TermItem> ti;
