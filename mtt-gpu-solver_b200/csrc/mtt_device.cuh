@@ -67,11 +67,21 @@ __host__ __device__ __forceinline__ uint32_t flush_mask(const Planes& p) {
     return (f & 0x80008000u ? half >> 16 : half) & 0x1FFFu;
 }
 
-// Score of a flush's rank mask.
+// Score of a flush's rank mask, which holds fewer than five ranks where cards
+// of the hand repeat: those add their ranks one by one.  (One test ahead costs
+// 30 million hands nothing; one in every step made them 1% slower.)
 __host__ __device__ __forceinline__ uint32_t score_flush(uint32_t fm) {
     const int sf = straight_high(fm);
     if (sf >= 0) return (8u << 24) | (uint32_t)sf;
     uint32_t m = fm, score = 5u << 24;
+    if (bit_count(fm) < 5) {
+        for (int shift = 16; m; shift -= 4) {
+            const int r = hi_bit(m);
+            score |= (uint32_t)r << shift;
+            m ^= 1u << r;
+        }
+        return score;
+    }
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         const int r = hi_bit(m);
