@@ -451,7 +451,8 @@ typedef struct mtt_pf_params {
  * and the loop at preflop_grid_generator.cu:228-421,588-614).  d_sums / d_sigma
  * ([10][192]): strategy sums / last strategies of the nodes BTN root (fold,
  * min-raise, jam), BB vs min-raise (fold, call, 3-bet jam), BTN vs 3-bet (fold,
- * call), BB vs open jam (fold, call), one 192-wide row per action. */
+ * call), BB vs open jam (fold, call), one 192-wide row per action.  With
+ * iters > 0 the call waits for the stream, unless the stream is being captured. */
 int mtt_pf_dcfr(const float* d_flop_weights, const float* d_class_mats, int32_t n_flops, const float* d_allin,
                 const mtt_pf_params* p, float* d_sums, float* d_sigma, void* stream);
 /* Read a flop-subset file (uint32 count, then per flop c1, c2, c3, pad, float

@@ -856,6 +856,11 @@ extern "C" int mtt_pf_dcfr(const float* d_flop_weights, const float* d_class_mat
     if (!s) s = cuda_status(cudaMemcpyAsync(d_sums, d.S, sizeof(float) * STATE, cudaMemcpyDeviceToDevice, st));
     if (!s && d_sigma) s = cuda_status(cudaMemcpyAsync(d_sigma, d.G, sizeof(float) * STATE, cudaMemcpyDeviceToDevice, st));
     cudaFreeAsync(buf, st);
+    // the call returns with its results in place (a caller on another stream
+    // reads them, and frees its inputs, at once), unless it is only recorded
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!s && p->iters > 0) s = cuda_status(cudaStreamIsCapturing(st, &cap));
+    if (!s && p->iters > 0 && cap == cudaStreamCaptureStatusNone) s = cuda_status(cudaStreamSynchronize(st));
     return s;
 }
 
