@@ -81,11 +81,13 @@ class StrategyEV:
                 idx_r[p].append(base + np.arange(len(c)))
                 sub_r[p].append(np.full(len(c), s))
                 cmb_r[p].append(c)
+        # the indexes are finished on the host: a copy from pageable memory is
+        # complete when it returns, so the calls' streams need not wait for it
         t = lambda a: torch.from_numpy(np.concatenate(a) if isinstance(a, list) else a).to(self.device)
         self._ridx = [t(idx_r[p]) for p in range(2)]
         self._rsub = [t(sub_r[p]) for p in range(2)]
         self._rcmb = [t(cmb_r[p]) for p in range(2)]
-        self._rflat = [self._rsub[p] * 1326 + self._rcmb[p] for p in range(2)]
+        self._rflat = [t([s * 1326 + c for s, c in zip(sub_r[p], cmb_r[p])]) for p in range(2)]
         # the index per element: made here where the scaling reads it, otherwise
         # (equal lengths) when asked for
         self._seg = {}
@@ -97,8 +99,7 @@ class StrategyEV:
     def _segments(self, name, lengths):
         import torch
         if name not in self._seg:
-            self._seg[name] = torch.repeat_interleave(torch.arange(self.n, device=self.device),
-                                                      torch.tensor(lengths, device=self.device))
+            self._seg[name] = torch.from_numpy(np.repeat(np.arange(self.n), lengths)).to(self.device)
         return self._seg[name]
 
     @property
