@@ -663,7 +663,8 @@ constexpr int STEP_SMEM = 4 * (STEP_JAM + STEP_FLOPS * (2 * STEP_CLS + 1));
 enum { M_M3, M_BF3, M_BC3, M_MJ, M_CJ, M_FM, M_CM, M_JM, M_FJ, N_MASS };   // mass order; the first of each equity sum's too
 __global__ void __launch_bounds__(STEP_THREADS) k_pf_step(PfDev d, float wp, float ws) {
     extern __shared__ __align__(16) float step_smem[];
-    __shared__ float G[STATE], root[PAD];
+    __shared__ __align__(16) float G[STATE];                 // filled 16 bytes at a time
+    __shared__ __align__(16) float root[PAD];
     __shared__ float reach[N_MASS][PAD];                     // summands of the masses
     __shared__ float mass[N_MASS];
     __shared__ float sums[6][STEP_CLS];                      // equity sums of warps 0..3, flop sums of warps 4, 5
