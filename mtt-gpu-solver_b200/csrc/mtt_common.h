@@ -30,6 +30,16 @@ inline int scratch_alloc(T** p, size_t count, cudaStream_t st) {
 unsigned long long current_context_id();
 int scratch_trim();   // returns what the current device's scratch pool keeps; the caller has synchronised
 
+// Raises a kernel's limit on dynamic shared memory, where `need` is above it, to
+// all that a block can have.  Always to the same value: a limit set to one
+// batch's need could be lowered by another thread's batch between this one's
+// call and its launches, which then failed as invalid.
+int allow_smem(const void* kernel, size_t need);
+template <typename... Args>
+inline int allow_smem(void (*kernel)(Args...), size_t need) {
+    return allow_smem(reinterpret_cast<const void*>(kernel), need);
+}
+
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 

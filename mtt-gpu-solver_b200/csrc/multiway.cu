@@ -851,15 +851,11 @@ int launch_iteration(const mtt_mw_batch* b, const MwDev& a, cudaStream_t st) {
 }
 
 int set_term_smem(const mtt_mw_batch* b) {
-    const size_t smem = sizeof(double) * (size_t)NP * ((size_t)b->Hmax + 1);
-    if (smem > 48 * 1024)
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_mw_term, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const size_t cr = term_cr_smem(b);
-    if (cr > 48 * 1024)
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_mw_term_cr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cr));
-    if (b->tree_smem > 48 * 1024) {
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_tree<MTT_ALGO_CFRPLUS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->tree_smem));
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_tree<MTT_ALGO_DCFR, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b->tree_smem));
+    MTT_TRY(allow_smem(k_mw_term, sizeof(double) * (size_t)NP * ((size_t)b->Hmax + 1)));
+    MTT_TRY(allow_smem(k_mw_term_cr, term_cr_smem(b)));
+    if (b->tree) {
+        MTT_TRY(allow_smem(k_tree<MTT_ALGO_CFRPLUS, true>, b->tree_smem));
+        MTT_TRY(allow_smem(k_tree<MTT_ALGO_DCFR, true>, b->tree_smem));
     }
     return MTT_OK;
 }

@@ -2336,25 +2336,17 @@ static int launch_br(const mtt_batch* b, const ListSet& L, const SolveDev& a, in
 
 static int set_smem_attrs(const mtt_batch* b, const ListSet& L) {
     const size_t t = sizeof(double) * (size_t)term_xstride(b);
-    if (t > 48 * 1024) {
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_br_term, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t));
-        MTT_TRY_CUDA(cudaFuncSetAttribute(k_br_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t));
-    }
-    int tmax = 0;
-    int trmax = 0;
+    MTT_TRY(allow_smem(k_br_term, t));
+    MTT_TRY(allow_smem(k_br_final, t));
+    int tmax = 0, trmax = 0;
     for (int v : L.tree_smem) trmax = std::max(trmax, v);
-    if (trmax > 48 * 1024)
+    if (trmax)
         for (int algo : {MTT_ALGO_CFRPLUS, MTT_ALGO_DCFR})
-            for (int sim = 0; sim < 2; ++sim)
-                MTT_TRY_CUDA(cudaFuncSetAttribute(tree_kernel(algo, sim != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, trmax));
+            for (int sim = 0; sim < 2; ++sim) MTT_TRY(allow_smem(tree_kernel(algo, sim != 0), trmax));
     for (int v : L.tb_smem1) tmax = std::max(tmax, v);
     for (int v : L.tb_smem3) tmax = std::max(tmax, v);
-    if (tmax > 48 * 1024) {
-        for (int sem = 0; sem < 2; ++sem)
-            for (int upd = 1; upd <= 3; ++upd)
-                MTT_TRY_CUDA(cudaFuncSetAttribute(term_kernel(upd, sem), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  tmax));
-    }
+    for (int sem = 0; sem < 2; ++sem)
+        for (int upd = 1; upd <= 3; ++upd) MTT_TRY(allow_smem(term_kernel(upd, sem), tmax));
     return MTT_OK;
 }
 
@@ -3064,8 +3056,7 @@ extern "C" int mtt_batch_set_leafnet(mtt_batch* b, mtt_leafnet* net, int32_t fla
             for (int q = 0; q < 2; ++q) smem = std::max(smem, leaf_sd_smem(lf.H[1 - q], lf.H[q], lf.Hp[1 - q]));
         }
         if (smem > 227 * 1024) return MTT_ERR_UNSUPPORTED;
-        if (smem > 48 * 1024)
-            MTT_TRY_CUDA(cudaFuncSetAttribute(k_leaf_showdown, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        MTT_TRY(allow_smem(k_leaf_showdown, smem));
         long long total = 0;
         int s = dalloc(&b->d_lx, (size_t)rows * LEAF_IN, total);
         if (!s) s = dalloc(&b->d_ly, (size_t)rows * LEAF_OUT, total);

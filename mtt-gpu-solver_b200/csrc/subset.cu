@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kStepThreads) k_ss_nnls(SsDev d, int s) {
 template <bool VEC>
 int run(SsDev& d, cudaStream_t st) {
     const size_t smem = StepSmem::bytes(d.nsel);
-    MTT_TRY_CUDA(cudaFuncSetAttribute(k_ss_nnls<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MTT_TRY(allow_smem(k_ss_nnls<VEC>, smem));
     k_ss_norms<VEC><<<ceil_div(d.ncols, 8), 256, 0, st>>>(d);
     MTT_CHECK_LAUNCH();
     k_ss_target_part<<<dim3(ceil_div(d.nfeat, 256), kTargetChunks), 256, 0, st>>>(d);
