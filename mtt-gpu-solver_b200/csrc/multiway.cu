@@ -1065,7 +1065,7 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
             t.n_rows = g.rows[q];
             t.n_nodes = g.n_nodes;
             fits &= g.n_nodes < TREE_MAX_NODES && g.rows[q] < TREE_MAX_NODES - 1;
-            if (fits) fits &= tree_min_bytes(g.n_nodes, g.rows[q], q, 0, true, node) <= TREE_BYTES;
+            if (fits) fits &= tree_size(g.n_nodes, g.rows[q], q, node).bytes(0, true) <= TREE_BYTES;
             if (fits) build_tree_seg(th, t, s, q, node);
         }
         hn.insert(hn.end(), loc.begin(), loc.end());

@@ -1687,8 +1687,19 @@ struct HostLists {
     TreeHost tree;
 };
 
-constexpr int TREE_CLASSES = 3;                      // by shared memory: about 5, 2 and 1 CTAs an SM
+// By shared memory: two CTAs an SM of the first two classes (registers allow no
+// more; the first keeps slices narrow), one of the last.
+constexpr int TREE_CLASSES = 3;
 constexpr int TREE_CLASS_BYTES[TREE_CLASSES] = {44 * 1024, 110 * 1024, 224 * 1024};
+struct TreePick { int cls, lg; };
+// The slice of one player's tree, bytes(lg) of shared memory for 4 << lg hands:
+// 32 hands (128-byte rows), or 16 or 8 where that lets it fit a smaller class.
+template <typename Bytes>
+static TreePick tree_pick(Bytes bytes) {
+    if (bytes(2) <= TREE_CLASS_BYTES[0]) return {0, bytes(3) <= TREE_CLASS_BYTES[0] ? 3 : 2};
+    if (bytes(1) > TREE_CLASS_BYTES[1]) return {2, 1};
+    return {1, bytes(3) <= TREE_CLASS_BYTES[1] ? 3 : bytes(2) <= TREE_CLASS_BYTES[1] ? 2 : 1};
+}
 
 struct ListSet {
     LevelLists<FwdItem> f_init, f_sim, f_alt[2];
@@ -1912,9 +1923,8 @@ static TreeShapeNode shape_node(const std::vector<DNode>& nodes, const std::vect
     return {nd.type == MTT_NODE_DECISION, nd.player, nd.na, nd.first, nd.row, q ? nd.reach_src1 : nd.reach_src0, depth[k]};
 }
 
-// The CTAs of the whole-tree sweeps.  A slice is 32 hands (128-byte rows), or
-// 16 or 8 where that lets the tree fit a class of less shared memory and more
-// CTAs an SM; costliest first, so that the last CTAs to start are short.
+// The CTAs of the whole-tree sweeps, costliest first, so that the last CTAs to
+// start are short.
 static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* active, long long& total) {
     const HostLists& H = b->host;
     int sms = 148, dev = 0;
@@ -1925,10 +1935,8 @@ static int build_tree_ctas(mtt_batch* b, ListSet& L, const std::vector<char>* ac
         if (active && !(*active)[H.tree.sub[i]]) continue;
         const TreeSeg& g = H.tree.segs[i];
         auto bytes = [&](int lg) { return tree_smem_bytes(g.n_rows, g.n_term, g.n_dec, g.n_int, lg, false); };
-        int lg = 1, cls = TREE_CLASSES - 1;
-        if (bytes(2) <= TREE_CLASS_BYTES[0]) { cls = 0; lg = bytes(3) <= TREE_CLASS_BYTES[0] ? 3 : 2; }
-        else if (bytes(1) <= TREE_CLASS_BYTES[1]) { cls = 1; lg = bytes(3) <= TREE_CLASS_BYTES[1] ? 3 : bytes(2) <= TREE_CLASS_BYTES[1] ? 2 : 1; }
-        picks[cls][i & 1].push_back(Pick{i, lg, bytes(lg)});
+        const TreePick t = tree_pick(bytes);
+        picks[t.cls][i & 1].push_back(Pick{i, t.lg, bytes(t.lg)});
     }
     std::vector<TreeCta> ctas;
     for (int c = 0; c < TREE_CLASSES; ++c) {
@@ -2635,27 +2643,41 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     b->levels = levels;
     // whole-tree sweeps: batches of few hands, whose level launches are bound by
     // latency; the subgame deals no card, ends in no leaf and a slice of its
-    // tree fits in shared memory.  The line is where the two met on uneven
+    // tree fits in shared memory.  One line is where the two met on uneven
     // river batches (us an iteration, tree / level launches): 1 subgame 37 / 63,
     // 8 (160 slices of 32 hands) 64 / 103, 16 79 / 107, 24 (480) 134 / 124, 32
     // 146 / 125; larger batches fill the chip level by level, and there the
-    // tree's barriers cost more than the launches.
+    // tree's barriers cost more than the launches.  The other line is two waves
+    // of one player's slices, which large trees, whose slices are of 8 hands,
+    // reach with fewer subgames: 783 nodes, 4 subgames of 1,081 hands (1.8
+    // waves) 137 / 144, 13 (6) 396 / 287; 2,181 nodes, one CTA an SM, 1 (0.9)
+    // 100 / 140, 10 of 300 hands (2.6) 318 / 286, 13 of 1,081 (12) 989 / 643
     b->tree.assign(n, 0);
     long long slices = 0;
     for (int i = 0; i < n; ++i) slices += (std::max(b->desc[i].Hp0, b->desc[i].Hp1) + 31) / 32;
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    long long halves[2] = {0, 0};        // of an SM, that a player's slices fill
     for (int i = 0; i < n && slices <= 3LL * sms; ++i) {
-        bool ok = b->desc[i].n_nodes < TREE_MAX_NODES && b->desc[i].rows0 < TREE_MAX_NODES - 1 &&
-                  b->desc[i].rows1 < TREE_MAX_NODES - 1;
+        const SubDesc& d = b->desc[i];
+        bool ok = d.n_nodes < TREE_MAX_NODES && d.rows0 < TREE_MAX_NODES - 1 && d.rows1 < TREE_MAX_NODES - 1;
         for (const DNode& nd : packs[i].nodes) ok &= nd.type != MTT_NODE_CHANCE && nd.type != MTT_NODE_LEAF;
+        long long fill[2] = {0, 0};
         for (int q = 0; q < 2 && ok; ++q) {
-            auto node = [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); };
-            ok = tree_min_bytes(b->desc[i].n_nodes, q ? b->desc[i].rows1 : b->desc[i].rows0, q, 1, false, node) <=
-                 TREE_CLASS_BYTES[TREE_CLASSES - 1];
+            const TreeSize z = tree_size(d.n_nodes, q ? d.rows1 : d.rows0, q,
+                                         [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
+            ok = z.bytes(1, false) <= TREE_CLASS_BYTES[TREE_CLASSES - 1];
+            if (!ok) break;
+            const TreePick t = tree_pick([&](int lg) { return z.bytes(lg, false); });
+            fill[q] = (long long)(((q ? d.Hp1 : d.Hp0) / 4 + (1 << t.lg) - 1) >> t.lg) * (t.cls == 2 ? 2 : 1);
         }
         b->tree[i] = ok;
         b->any_tree |= ok;
+        if (ok) { halves[0] += fill[0]; halves[1] += fill[1]; }
+    }
+    if (std::max(halves[0], halves[1]) > 4LL * sms) {
+        b->tree.assign(n, 0);
+        b->any_tree = false;
     }
     // FP64 best-response warp tasks, solver work items per level, terminal items
     HostLists& HL = b->host;

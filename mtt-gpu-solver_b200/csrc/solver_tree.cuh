@@ -361,26 +361,36 @@ struct TreeHost {
     std::vector<TreeNode> nodes;
 };
 
-// Shared memory of the smallest slice (4 << lg hands) of one player's tree.
-// Past any limit where two nodes share regret rows: a level launch adds both
-// nodes' sums to them, one level after the other, while a slice stages the sums
-// once and numbers its reach by row.
+// What a slice of one player's tree needs of shared memory, at most one level
+// per node.  No slice fits where two nodes share regret rows: a level launch
+// adds both nodes' sums to them, one level after the other, while a slice
+// stages the sums once and numbers its reach by row.
+struct TreeSize {
+    int n_rows = 0, n_term = 0, n_dec = 0, n_int = 0;
+    bool shared = false;
+    int bytes(int lg, bool sim) const {        // of 4 << lg hands
+        return shared ? INT_MAX : tree_smem_bytes(n_rows, n_term, n_dec, n_int, lg, sim);
+    }
+};
 template <typename Node>
-inline int tree_min_bytes(int n_nodes, int n_rows, int q, int lg, bool sim, Node node) {
-    int dec = 0, own = 0;
+inline TreeSize tree_size(int n_nodes, int n_rows, int q, Node node) {
+    TreeSize z;
+    int own = 0;
     std::vector<char> used(n_rows, 0);
     for (int k = 0; k < n_nodes; ++k) {
         const TreeShapeNode nd = node(k);
-        dec += nd.dec;
+        z.n_dec += nd.dec;
         if (!nd.dec || nd.player != q) continue;
         ++own;
         for (int a = 0; a < nd.na; ++a) {
-            if (used[nd.row + a]) return INT_MAX;
+            z.shared |= used[nd.row + a] != 0;
             used[nd.row + a] = 1;
         }
     }
-    // at most one level per node
-    return tree_smem_bytes(n_rows, n_nodes - dec, dec, 2 * (dec + 1) + own + n_nodes - dec + (n_nodes + 1) / 2, lg, sim);
+    z.n_rows = n_rows;
+    z.n_term = n_nodes - z.n_dec;
+    z.n_int = 2 * (z.n_dec + 1) + own + z.n_term + (n_nodes + 1) / 2;
+    return z;
 }
 
 // One player's view of a chance-free tree: the backward order (all decision
