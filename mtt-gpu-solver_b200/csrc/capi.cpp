@@ -1,7 +1,6 @@
 // capi.cpp — status strings, version and the per-thread CUDA error slot.
 #include <cuda.h>   // CUcontext / CUresult types only: the driver entry points are resolved at run time
 
-#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -93,19 +92,6 @@ int scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
     MTT_TRY_CUDA(cudaStreamIsCapturing(st, &cap));
     cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool(true) : nullptr;
     return cuda_status(pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st));
-}
-
-int allow_smem(const void* kernel, size_t need) {
-    cudaFuncAttributes at;
-    MTT_TRY_CUDA(cudaFuncGetAttributes(&at, kernel));
-    if (need + at.sharedSizeBytes <= 48 * 1024) return MTT_OK;   // within every kernel's own limit
-    int dev = 0, most = 0;
-    MTT_TRY_CUDA(cudaGetDevice(&dev));
-    MTT_TRY_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    most -= (int)at.sharedSizeBytes;
-    if (need > (size_t)std::max(most, 0)) return cuda_status(cudaErrorInvalidValue);
-    if (at.maxDynamicSharedSizeBytes >= most) return MTT_OK;
-    return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 }
 
 int scratch_trim() {

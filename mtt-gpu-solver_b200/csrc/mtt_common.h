@@ -30,14 +30,18 @@ inline int scratch_alloc(T** p, size_t count, cudaStream_t st) {
 unsigned long long current_context_id();
 int scratch_trim();   // returns what the current device's scratch pool keeps; the caller has synchronised
 
-// Raises a kernel's limit on dynamic shared memory, where `need` is above it, to
-// all that a block can have.  Always to the same value: a limit set to one
-// batch's need could be lowered by another thread's batch between this one's
-// call and its launches, which then failed as invalid.
-int allow_smem(const void* kernel, size_t need);
+// Raises a kernel's limit on dynamic shared memory, where `need` is above the
+// default (48 KB with the kernel's static part, at most 2.4 KB here), to 224 KB.
+// Always to the same value: a limit set to one batch's need could be lowered by
+// another thread's batch between this one's call and its launches, which then
+// failed as invalid.  One call a kernel, and none for small needs: asking for
+// the kernel's attributes first cost a solve 70 us.
+constexpr size_t SMEM_FREE = 45 * 1024, SMEM_MOST = 224 * 1024;
 template <typename... Args>
 inline int allow_smem(void (*kernel)(Args...), size_t need) {
-    return allow_smem(reinterpret_cast<const void*>(kernel), need);
+    if (need <= SMEM_FREE) return MTT_OK;
+    return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)(need > SMEM_MOST ? need : SMEM_MOST)));
 }
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
