@@ -35,6 +35,7 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <numeric>
 #include <vector>
 
@@ -731,15 +732,14 @@ struct mtt_mw_batch {
     float* d_iter_tab = nullptr;
     int iter_cap = 0;
     double* d_values = nullptr;
+    uint8_t* d_lists = nullptr;                 // holds the work lists: levels, terminals, trees
     MFwd* d_fwd = nullptr;
     MBwd* d_bwd = nullptr;
     int2* d_terms = nullptr;
     std::vector<long long> fwd_off, bwd_off;   // per level
     // whole-tree sweeps of the solve (the values pass keeps the level kernels)
     bool tree = false;
-    TreeSeg* d_segs = nullptr;
-    int* d_ints = nullptr;
-    TreeNode* d_tnodes = nullptr;
+    TreeDev dtree;
     TreeCta* d_ctas = nullptr;
     int n_ctas = 0, tree_smem = 0;
     long long rs4 = 0;                          // float4 of R (and of S)
@@ -762,8 +762,7 @@ void free_mw(mtt_mw_batch* b) {
     if (b->gexec) cudaGraphExecDestroy(b->gexec);
     cudaFree(b->d_desc); cudaFree(b->d_nodes); cudaFree(b->d_tabs); cudaFree(b->d_ranges); cudaFree(b->d_arena);
     cudaFree(b->d_R); cudaFree(b->d_S); cudaFree(b->d_iter); cudaFree(b->d_iter_tab); cudaFree(b->d_values);
-    cudaFree(b->d_fwd); cudaFree(b->d_bwd); cudaFree(b->d_terms);
-    cudaFree(b->d_segs); cudaFree(b->d_ints); cudaFree(b->d_tnodes); cudaFree(b->d_ctas);
+    cudaFree(b->d_lists);
     delete b;
 }
 
@@ -796,7 +795,7 @@ int launch_terms(const mtt_mw_batch* b, const MwDev& a, cudaStream_t st) {
 int launch_tree(const mtt_mw_batch* b, const MwDev& a, int flags, bool chained, cudaStream_t st) {
     TreeArgs t;
     t.arena = a.arena; t.R = a.R; t.S = a.S; t.iter_tab = a.iter_tab; t.iter = a.iter;
-    t.ctas = b->d_ctas; t.segs = b->d_segs; t.ints = b->d_ints; t.nodes = b->d_tnodes;
+    t.ctas = b->d_ctas; t.segs = b->dtree.segs; t.ints = b->dtree.ints; t.nodes = b->dtree.nodes;
     t.n = b->n_ctas;
     t.flags = flags;
     MTT_TRY_CUDA(launch_pdl(a.algo == MTT_ALGO_DCFR ? k_tree<MTT_ALGO_DCFR, true> : k_tree<MTT_ALGO_CFRPLUS, true>,
@@ -887,9 +886,7 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     std::vector<std::vector<MFwd>> fl;
     std::vector<std::vector<MBwd>> bl;
     std::vector<int2> tl;
-    TreeHost th;
-    bool fits = true;
-    constexpr int TREE_BYTES = 224 * 1024;
+    std::vector<std::vector<int>> depths;      // of every subgame's nodes
     long long arena = 0, rs = 0;
     b->desc.resize(n);
     b->rows.resize(4 * (size_t)n);
@@ -1051,37 +1048,16 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
                 tl.push_back(make_int2(gn, s));
             }
         }
-        for (int q = 0; q < NP; ++q) {
-            auto node = [&](int k) {
-                const MNode& x = loc[k];
-                return TreeShapeNode{x.type == MTT_NODE_DECISION, x.player, x.na, x.first, x.row, x.src[q], depth[k]};
-            };
-            TreeSeg t{};
-            t.reach = d.arena_base + (long long)q * d.Hp;
-            t.cfv = d.arena_base + (long long)g.n_nodes * HS + (long long)q * d.Hp;
-            t.rows = d.rs_base[q];
-            t.h4 = H4;
-            t.hs4 = (int)(HS / 4);
-            t.n_rows = g.rows[q];
-            t.n_nodes = g.n_nodes;
-            fits &= g.n_nodes < TREE_MAX_NODES && g.rows[q] < TREE_MAX_NODES - 1;
-            if (fits) fits &= tree_size(g.n_nodes, g.rows[q], q, node).bytes(0, true) <= TREE_BYTES;
-            if (fits) build_tree_seg(th, t, s, q, node);
-        }
+        depths.push_back(std::move(depth));
         hn.insert(hn.end(), loc.begin(), loc.end());
         b->desc[s] = d;
         for (int p = 0; p < NP; ++p) b->rows[4 * (size_t)s + p] = g.rows[p];
     }
-    // flatten the level lists
-    std::vector<MFwd> ff;
-    std::vector<MBwd> bb;
     b->fwd_off.assign(b->levels + 1, 0);
     b->bwd_off.assign(b->levels + 1, 0);
     for (int d = 0; d < b->levels; ++d) {
-        ff.insert(ff.end(), fl[d].begin(), fl[d].end());
-        bb.insert(bb.end(), bl[d].begin(), bl[d].end());
-        b->fwd_off[d + 1] = (long long)ff.size();
-        b->bwd_off[d + 1] = (long long)bb.size();
+        b->fwd_off[d + 1] = b->fwd_off[d] + (long long)fl[d].size();
+        b->bwd_off[d + 1] = b->bwd_off[d] + (long long)bl[d].size();
     }
     b->n_terms = (int)tl.size();
     b->rs4 = rs / 4;
@@ -1093,6 +1069,46 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     // tree: 272 CTAs, one wave, against 101 in slices of 8 hands; two subgames
     // 231 / 144, four 376 / 286, eight (2,176 CTAs) 671 / 549.  Larger batches
     // keep the level kernels, unmeasured.
+    constexpr int TREE_BYTES = 224 * 1024;
+    std::vector<TreeHost> part(NP * (size_t)n);
+    std::atomic<bool> fits{true};
+    auto plan = [&](int i) {             // player i % NP of subgame i / NP
+        const int s = i / NP, q = i % NP;
+        const MDesc& d = b->desc[s];
+        const MNode* nd = hn.data() + d.node_base;
+        const int* depth = depths[s].data();
+        const int n_nodes = (int)depths[s].size(), n_rows = b->rows[i];
+        auto node = [=](int k) {
+            const MNode& x = nd[k];
+            return TreeShapeNode{x.type == MTT_NODE_DECISION, x.player, x.na, x.first, x.row, x.src[q], depth[k]};
+        };
+        if (!fits) return;
+        if (n_nodes >= TREE_MAX_NODES || n_rows >= TREE_MAX_NODES - 1 ||
+            tree_size(n_nodes, n_rows, q, node).bytes(0, true) > TREE_BYTES) {
+            fits = false;
+            return;
+        }
+        TreeSeg t{};
+        t.reach = d.arena_base + (long long)q * d.Hp;
+        t.cfv = d.arena_base + (long long)n_nodes * NP * d.Hp + (long long)q * d.Hp;
+        t.rows = d.rs_base[q];
+        t.h4 = d.Hp / 4;
+        t.hs4 = NP * d.Hp / 4;
+        t.n_rows = n_rows;
+        t.n_nodes = n_nodes;
+        build_tree_seg(part[i], t, s, q, node);
+    };
+    on_threads(NP * n, 60 * NP * (long long)hn.size(), plan);
+    std::vector<TreeSeg> segs;
+    size_t n_tnodes = 0, n_ints = 0;
+    if (fits)
+        for (const TreeHost& x : part) {
+            segs.push_back(x.segs[0]);
+            segs.back().node0 = (int)n_tnodes;
+            segs.back().int0 = (int)n_ints;
+            n_tnodes += x.nodes.size();
+            n_ints += x.ints.size();
+        }
     std::vector<TreeCta> tc;
     int sms = 148, dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1106,11 +1122,11 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
         int want = 1;
         for (; want < 3; ++want) {
             long long n_ctas = 0;
-            for (const TreeSeg& g : th.segs) n_ctas += (g.h4 + (1 << lanes(g, want)) - 1) >> lanes(g, want);
+            for (const TreeSeg& g : segs) n_ctas += (g.h4 + (1 << lanes(g, want)) - 1) >> lanes(g, want);
             if (n_ctas <= 2LL * sms) break;
         }
-        for (int i = 0; i < (int)th.segs.size(); ++i) {
-            const TreeSeg& g = th.segs[i];
+        for (int i = 0; i < (int)segs.size(); ++i) {
+            const TreeSeg& g = segs[i];
             const int lg = lanes(g, want);
             b->tree_smem = std::max(b->tree_smem, bytes(g, lg));
             for (int g0 = 0; g0 < g.h4; g0 += 1 << lg) tc.push_back(TreeCta{i, g0, lg, 0});
@@ -1119,18 +1135,39 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
         b->tree = b->n_ctas <= 16 * sms;
         if (!b->tree) b->tree_smem = 0;
     }
-    int s = MTT_OK;
-    if (b->tree) {
-        s = dalloc(&b->d_segs, th.segs.size());
-        if (!s) s = dalloc(&b->d_ints, th.ints.size());
-        if (!s) s = dalloc(&b->d_tnodes, th.nodes.size());
-        if (!s) s = dalloc(&b->d_ctas, tc.size());
-        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, th.segs.data(), sizeof(TreeSeg) * th.segs.size(), cudaMemcpyHostToDevice));
-        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, th.ints.data(), sizeof(int) * th.ints.size(), cudaMemcpyHostToDevice));
-        if (!s && !th.nodes.empty())
-            s = cuda_status(cudaMemcpy(b->d_tnodes, th.nodes.data(), sizeof(TreeNode) * th.nodes.size(), cudaMemcpyHostToDevice));
-        if (!s) s = cuda_status(cudaMemcpy(b->d_ctas, tc.data(), sizeof(TreeCta) * tc.size(), cudaMemcpyHostToDevice));
-    }
+    // every list in one allocation and one copy; each part but the last two is a
+    // multiple of 16 bytes
+    if (!b->tree) { part.clear(); segs.clear(); tc.clear(); n_tnodes = n_ints = 0; }
+    const size_t fwd_n = (size_t)b->fwd_off[b->levels], bwd_n = (size_t)b->bwd_off[b->levels];
+    const size_t at_bwd = sizeof(MFwd) * fwd_n, at_nodes = at_bwd + sizeof(MBwd) * bwd_n;
+    const size_t at_segs = at_nodes + sizeof(TreeNode) * n_tnodes, at_ctas = at_segs + sizeof(TreeSeg) * segs.size();
+    const size_t at_terms = at_ctas + sizeof(TreeCta) * tc.size(), at_ints = at_terms + sizeof(int2) * tl.size();
+    const size_t list_bytes = at_ints + sizeof(int) * n_ints;
+    std::unique_ptr<uint8_t[]> lists(new uint8_t[list_bytes]);
+    auto put = [&](size_t at, const auto& v) {
+        if (!v.empty()) std::memcpy(lists.get() + at, v.data(), sizeof(v[0]) * v.size());
+    };
+    put(at_segs, segs);
+    put(at_ctas, tc);
+    put(at_terms, tl);
+    on_threads(b->levels + (int)part.size(), (long long)list_bytes / 8, [&](int i) {
+        if (i < b->levels) {
+            put(sizeof(MFwd) * (size_t)b->fwd_off[i], fl[i]);
+            put(at_bwd + sizeof(MBwd) * (size_t)b->bwd_off[i], bl[i]);
+        } else {
+            const TreeSeg& g = segs[i - b->levels];
+            put(at_nodes + sizeof(TreeNode) * (size_t)g.node0, part[i - b->levels].nodes);
+            put(at_ints + sizeof(int) * (size_t)g.int0, part[i - b->levels].ints);
+        }
+    });
+    int s = dalloc(&b->d_lists, list_bytes);
+    if (!s && list_bytes) s = cuda_status(cudaMemcpy(b->d_lists, lists.get(), list_bytes, cudaMemcpyHostToDevice));
+    b->d_fwd = reinterpret_cast<MFwd*>(b->d_lists);
+    b->d_bwd = reinterpret_cast<MBwd*>(b->d_lists + at_bwd);
+    b->dtree = {reinterpret_cast<TreeNode*>(b->d_lists + at_nodes), reinterpret_cast<TreeSeg*>(b->d_lists + at_segs),
+                reinterpret_cast<int*>(b->d_lists + at_ints)};
+    b->d_ctas = reinterpret_cast<TreeCta*>(b->d_lists + at_ctas);
+    b->d_terms = reinterpret_cast<int2*>(b->d_lists + at_terms);
     if (!s) s = dalloc(&b->d_desc, n);
     if (!s) s = dalloc(&b->d_nodes, hn.size());
     if (!s) s = dalloc(&b->d_tabs, ht.size());
@@ -1140,16 +1177,10 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     if (!s) s = dalloc(&b->d_S, (size_t)rs);
     if (!s) s = dalloc(&b->d_iter, 3);
     if (!s) s = dalloc(&b->d_values, 4 * (size_t)n);
-    if (!s) s = dalloc(&b->d_fwd, ff.size());
-    if (!s) s = dalloc(&b->d_bwd, bb.size());
-    if (!s) s = dalloc(&b->d_terms, tl.size());
     if (!s) s = cuda_status(cudaMemcpy(b->d_desc, b->desc.data(), sizeof(MDesc) * n, cudaMemcpyHostToDevice));
     if (!s) s = cuda_status(cudaMemcpy(b->d_nodes, hn.data(), sizeof(MNode) * hn.size(), cudaMemcpyHostToDevice));
     if (!s) s = cuda_status(cudaMemcpy(b->d_tabs, ht.data(), 2 * ht.size(), cudaMemcpyHostToDevice));
     if (!s) s = cuda_status(cudaMemcpy(b->d_ranges, hr.data(), 4 * hr.size(), cudaMemcpyHostToDevice));
-    if (!s && !ff.empty()) s = cuda_status(cudaMemcpy(b->d_fwd, ff.data(), sizeof(MFwd) * ff.size(), cudaMemcpyHostToDevice));
-    if (!s && !bb.empty()) s = cuda_status(cudaMemcpy(b->d_bwd, bb.data(), sizeof(MBwd) * bb.size(), cudaMemcpyHostToDevice));
-    if (!s && !tl.empty()) s = cuda_status(cudaMemcpy(b->d_terms, tl.data(), sizeof(int2) * tl.size(), cudaMemcpyHostToDevice));
     if (!s) s = cuda_status(cudaMemset(b->d_arena, 0, sizeof(float) * (size_t)std::max(arena, 1LL)));
     if (s) { free_mw(b); return s; }
     *out = b;

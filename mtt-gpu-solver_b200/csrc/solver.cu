@@ -1755,9 +1755,8 @@ struct mtt_batch {
     int levels = 0;
     std::vector<char> tree;            // subgames that take the whole-tree sweeps
     bool any_tree = false;
-    TreeSeg* d_segs = nullptr;
-    int* d_ints = nullptr;
-    TreeNode* d_tnodes = nullptr;
+    uint8_t* d_tree = nullptr;         // holds dtree
+    TreeDev dtree;
     HostLists host;
     ListSet full, act;
     std::vector<SubDesc> desc;
@@ -1859,7 +1858,7 @@ static void free_batch(mtt_batch* b) {
     dfree(b->d_darena); dfree(b->d_results); dfree(b->d_roots); dfree(b->d_iter);
     if (b->h_roots) cudaFreeHost(b->h_roots);
     dfree(b->d_iter_tab);
-    dfree(b->d_err); dfree(b->d_segs); dfree(b->d_ints); dfree(b->d_tnodes);
+    dfree(b->d_err); dfree(b->d_tree);
     dfree(b->d_leaves); dfree(b->d_lx); dfree(b->d_ly); dfree(b->d_lm); dfree(b->d_lsd);
     free_set(b->full);
     free_set(b->act);
@@ -2187,9 +2186,9 @@ static int launch_tree(const mtt_batch* b, const ListSet& L, const SolveDev& a, 
     }
     TreeArgs t;
     t.arena = a.arena; t.R = a.R; t.S = a.S; t.iter_tab = a.iter_tab; t.iter = a.iter;
-    t.segs = b->d_segs;
-    t.ints = b->d_ints;
-    t.nodes = b->d_tnodes;
+    t.segs = b->dtree.segs;
+    t.ints = b->dtree.ints;
+    t.nodes = b->dtree.nodes;
     t.n = all;
     t.flags = flags;
     const TreeCta* first = L.ctas;
@@ -2598,10 +2597,46 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     *out = nullptr;
     std::vector<SubPack> packs(n);
     const int nthr = std::max(1, std::min<int>((int)std::thread::hardware_concurrency(), 32));
+    int sms = 148, dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // whole-tree sweeps: batches of few hands, whose level launches are bound by
+    // latency; the subgame deals no card, ends in no leaf and a slice of its
+    // tree fits in shared memory.  One line is where the two met on uneven
+    // river batches (us an iteration, tree / level launches): 1 subgame 37 / 63,
+    // 8 (160 slices of 32 hands) 64 / 103, 16 79 / 107, 24 (480) 134 / 124, 32
+    // 146 / 125; larger batches fill the chip level by level, and there the
+    // tree's barriers cost more than the launches.  The other line is two waves
+    // of one player's slices, which large trees, whose slices are of 8 hands,
+    // reach with fewer subgames: 783 nodes, 4 subgames of 1,081 hands (1.8
+    // waves) 137 / 144, 13 (6) 396 / 287; 2,181 nodes, one CTA an SM, 1 (0.9)
+    // 100 / 140, 10 of 300 hands (2.6) 318 / 286, 13 of 1,081 (12) 989 / 643
+    long long slices = 0;
+    for (int i = 0; i < n; ++i) slices += (std::max(subs[i].H[0], subs[i].H[1]) + 31) / 32;
+    const bool few = slices <= 3LL * sms;
+    struct Fill { bool ok; long long halves[2]; };       // halves of an SM that each player's slices fill
+    std::vector<Fill> fill(few ? n : 0);
+    auto size_tree = [&](int i) {
+        const SubDesc& d = packs[i].d;
+        Fill& f = fill[i];
+        f.ok = d.n_nodes < TREE_MAX_NODES && d.rows0 < TREE_MAX_NODES - 1 && d.rows1 < TREE_MAX_NODES - 1;
+        for (const DNode& nd : packs[i].nodes) f.ok &= nd.type != MTT_NODE_CHANCE && nd.type != MTT_NODE_LEAF;
+        for (int q = 0; q < 2 && f.ok; ++q) {
+            const TreeSize z = tree_size(d.n_nodes, q ? d.rows1 : d.rows0, q,
+                                         [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
+            const TreePick t = tree_pick([&](int lg) { return z.bytes(lg, false); });
+            f.ok = z.bytes(1, false) <= TREE_CLASS_BYTES[TREE_CLASSES - 1];
+            f.halves[q] = (long long)(((q ? d.Hp1 : d.Hp0) / 4 + (1 << t.lg) - 1) >> t.lg) * (t.cls == 2 ? 2 : 1);
+        }
+    };
     {
         std::vector<std::thread> th;
         for (int t = 0; t < nthr; ++t)
-            th.emplace_back([&, t]() { for (int i = t; i < n; i += nthr) pack_one(subs[i], packs[i]); });
+            th.emplace_back([&, t]() {
+                for (int i = t; i < n; i += nthr) {
+                    pack_one(subs[i], packs[i]);
+                    if (few && !packs[i].status) size_tree(i);
+                }
+            });
         for (auto& x : th) x.join();
     }
     for (int i = 0; i < n; ++i) if (packs[i].status) return packs[i].status;
@@ -2641,44 +2676,12 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     b->iter_bytes = iter_bytes;
     b->rs4 = rs / 4;
     b->levels = levels;
-    // whole-tree sweeps: batches of few hands, whose level launches are bound by
-    // latency; the subgame deals no card, ends in no leaf and a slice of its
-    // tree fits in shared memory.  One line is where the two met on uneven
-    // river batches (us an iteration, tree / level launches): 1 subgame 37 / 63,
-    // 8 (160 slices of 32 hands) 64 / 103, 16 79 / 107, 24 (480) 134 / 124, 32
-    // 146 / 125; larger batches fill the chip level by level, and there the
-    // tree's barriers cost more than the launches.  The other line is two waves
-    // of one player's slices, which large trees, whose slices are of 8 hands,
-    // reach with fewer subgames: 783 nodes, 4 subgames of 1,081 hands (1.8
-    // waves) 137 / 144, 13 (6) 396 / 287; 2,181 nodes, one CTA an SM, 1 (0.9)
-    // 100 / 140, 10 of 300 hands (2.6) 318 / 286, 13 of 1,081 (12) 989 / 643
     b->tree.assign(n, 0);
-    long long slices = 0;
-    for (int i = 0; i < n; ++i) slices += (std::max(b->desc[i].Hp0, b->desc[i].Hp1) + 31) / 32;
-    int sms = 148, dev = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long long halves[2] = {0, 0};        // of an SM, that a player's slices fill
-    for (int i = 0; i < n && slices <= 3LL * sms; ++i) {
-        const SubDesc& d = b->desc[i];
-        bool ok = d.n_nodes < TREE_MAX_NODES && d.rows0 < TREE_MAX_NODES - 1 && d.rows1 < TREE_MAX_NODES - 1;
-        for (const DNode& nd : packs[i].nodes) ok &= nd.type != MTT_NODE_CHANCE && nd.type != MTT_NODE_LEAF;
-        long long fill[2] = {0, 0};
-        for (int q = 0; q < 2 && ok; ++q) {
-            const TreeSize z = tree_size(d.n_nodes, q ? d.rows1 : d.rows0, q,
-                                         [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
-            ok = z.bytes(1, false) <= TREE_CLASS_BYTES[TREE_CLASSES - 1];
-            if (!ok) break;
-            const TreePick t = tree_pick([&](int lg) { return z.bytes(lg, false); });
-            fill[q] = (long long)(((q ? d.Hp1 : d.Hp0) / 4 + (1 << t.lg) - 1) >> t.lg) * (t.cls == 2 ? 2 : 1);
-        }
-        b->tree[i] = ok;
-        b->any_tree |= ok;
-        if (ok) { halves[0] += fill[0]; halves[1] += fill[1]; }
-    }
-    if (std::max(halves[0], halves[1]) > 4LL * sms) {
-        b->tree.assign(n, 0);
-        b->any_tree = false;
-    }
+    long long halves[2] = {0, 0};
+    for (const Fill& f : fill)
+        for (int q = 0; q < 2 && f.ok; ++q) halves[q] += f.halves[q];
+    if (std::max(halves[0], halves[1]) <= 4LL * sms)
+        for (int i = 0; i < (int)fill.size(); ++i) { b->tree[i] = fill[i].ok; b->any_tree |= fill[i].ok; }
     // FP64 best-response warp tasks, solver work items per level, terminal items
     HostLists& HL = b->host;
     auto init_lists = [levels](HostLists& L) {
@@ -2838,10 +2841,27 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
         dst.reserve(k);
         for (int t = 0; t < nlt; ++t) dst.insert(dst.end(), get(part[t]).begin(), get(part[t]).end());
     };
-    // every list is merged by its own job (distinct vectors), the jobs on the
-    // host threads
+    // every list is merged and every tree segment built by its own job (distinct
+    // vectors), the jobs on the host threads
     std::vector<std::function<void()>> jobs;
     auto add = [&](auto get) { jobs.emplace_back([&merge, get]() { merge(get); }); };
+    std::vector<TreeHost> trees(b->any_tree ? 2 * (size_t)n : 0);
+    for (int j = 0; j < (int)trees.size(); ++j)
+        if (b->tree[j / 2])
+            jobs.emplace_back([&, j]() {
+                const int i = j / 2, q = j % 2;
+                const SubDesc& d = b->desc[i];
+                const long long HS = d.Hp0 + d.Hp1, off = q ? d.Hp0 : 0;
+                TreeSeg g{};
+                g.reach = d.arena_base + off;
+                g.cfv = d.arena_base + (long long)d.n_nodes * HS + off;
+                g.rows = q ? d.rs_base1 : d.rs_base0;
+                g.h4 = (q ? d.Hp1 : d.Hp0) / 4;
+                g.hs4 = (int)(HS / 4);
+                g.n_rows = q ? d.rows1 : d.rows0;
+                g.n_nodes = d.n_nodes;
+                build_tree_seg(trees[j], g, i, q, [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
+            });
     for (int d = 0; d < levels; ++d) {
         add([d](HostLists& L) -> std::vector<Task>& { return L.bf[d]; });
         add([d](HostLists& L) -> std::vector<Task>& { return L.bb[d]; });
@@ -2866,30 +2886,20 @@ extern "C" int mtt_batch_create(const mtt_subgame* subs, int32_t n, mtt_batch** 
     }
     for (int t = 0; t < nlt; ++t) b->h_leaves.insert(b->h_leaves.end(), plv[t].begin(), plv[t].end());
     for (size_t k = 0; k < b->h_leaves.size(); ++k) b->h_leaves[k].row0 = LEAF_RIVERS * (int)k;
-    for (int i = 0; i < n; ++i)
-        for (int q = 0; q < 2 && b->tree[i]; ++q) {
-            const SubDesc& d = b->desc[i];
-            const long long HS = d.Hp0 + d.Hp1, off = q ? d.Hp0 : 0;
-            TreeSeg g{};
-            g.reach = d.arena_base + off;
-            g.cfv = d.arena_base + (long long)d.n_nodes * HS + off;
-            g.rows = q ? d.rs_base1 : d.rs_base0;
-            g.h4 = (q ? d.Hp1 : d.Hp0) / 4;
-            g.hs4 = (int)(HS / 4);
-            g.n_rows = q ? d.rows1 : d.rows0;
-            g.n_nodes = d.n_nodes;
-            build_tree_seg(HL.tree, g, i, q, [&](int k) { return shape_node(packs[i].nodes, packs[i].depth, q, k); });
-        }
+    for (const TreeHost& x : trees) HL.tree.append(x);
     long long total = 0;
     int s = MTT_OK;
     if (b->any_tree) {
-        s = dalloc(&b->d_segs, HL.tree.segs.size(), total);
-        if (!s) s = dalloc(&b->d_ints, HL.tree.ints.size(), total);
-        if (!s) s = dalloc(&b->d_tnodes, HL.tree.nodes.size(), total);
-        if (!s) s = cuda_status(cudaMemcpy(b->d_segs, HL.tree.segs.data(), sizeof(TreeSeg) * HL.tree.segs.size(), cudaMemcpyHostToDevice));
-        if (!s) s = cuda_status(cudaMemcpy(b->d_ints, HL.tree.ints.data(), sizeof(int) * HL.tree.ints.size(), cudaMemcpyHostToDevice));
-        if (!s && !HL.tree.nodes.empty())
-            s = cuda_status(cudaMemcpy(b->d_tnodes, HL.tree.nodes.data(), sizeof(TreeNode) * HL.tree.nodes.size(), cudaMemcpyHostToDevice));
+        const TreeHost& t = HL.tree;
+        const size_t nb = sizeof(TreeNode) * t.nodes.size(), sb = sizeof(TreeSeg) * t.segs.size(), ib = sizeof(int) * t.ints.size();
+        std::vector<uint8_t> all(nb + sb + ib);
+        if (nb) std::memcpy(all.data(), t.nodes.data(), nb);
+        std::memcpy(all.data() + nb, t.segs.data(), sb);
+        std::memcpy(all.data() + nb + sb, t.ints.data(), ib);
+        s = dalloc(&b->d_tree, all.size(), total);
+        b->dtree = {reinterpret_cast<TreeNode*>(b->d_tree), reinterpret_cast<TreeSeg*>(b->d_tree + nb),
+                    reinterpret_cast<int*>(b->d_tree + nb + sb)};
+        if (!s) s = cuda_status(cudaMemcpy(b->d_tree, all.data(), all.size(), cudaMemcpyHostToDevice));
     }
     if (!s) s = dalloc(&b->d_desc, n, total);
     if (!s) s = dalloc(&b->d_nodes, nodes, total);

@@ -2,9 +2,11 @@
 // the whole-tree sweep kernel, shared by the heads-up and four-player solvers.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <thread>
 #include <vector>
 
 #include "mtt_bulk.cuh"
@@ -359,7 +361,37 @@ struct TreeHost {
     std::vector<int> sub;            // subgame of each segment
     std::vector<int> ints;
     std::vector<TreeNode> nodes;
+    void append(const TreeHost& o) {
+        for (TreeSeg g : o.segs) {
+            g.node0 += (int)nodes.size();
+            g.int0 += (int)ints.size();
+            segs.push_back(g);
+        }
+        sub.insert(sub.end(), o.sub.begin(), o.sub.end());
+        ints.insert(ints.end(), o.ints.begin(), o.ints.end());
+        nodes.insert(nodes.end(), o.nodes.begin(), o.nodes.end());
+    }
 };
+
+// Their device copies, parts of one allocation.
+struct TreeDev {
+    TreeNode* nodes = nullptr;
+    TreeSeg* segs = nullptr;
+    int* ints = nullptr;
+};
+
+// fn(0) .. fn(n - 1), about `ns` nanoseconds in all, on up to 16 host threads
+// with 200 us each or more (starting one takes some 30).
+template <typename Fn>
+inline void on_threads(int n, long long ns, Fn fn) {
+    const int nt = (int)std::min<long long>({n, (long long)std::thread::hardware_concurrency(), 16, ns / 200000});
+    std::atomic<int> next{0};
+    auto run = [&]() { for (int i; (i = next.fetch_add(1)) < n;) fn(i); };
+    std::vector<std::thread> th;
+    for (int t = 1; t < nt; ++t) th.emplace_back(run);
+    run();
+    for (std::thread& x : th) x.join();
+}
 
 // What a slice of one player's tree needs of shared memory, at most one level
 // per node.  No slice fits where two nodes share regret rows: a level launch
