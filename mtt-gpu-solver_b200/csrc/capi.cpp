@@ -38,10 +38,6 @@ unsigned long long current_context_id() {
 }
 
 namespace {
-// Kept between calls.  The largest scratch of one call at the sizes in use is
-// 134 MB (flop-EV chain).
-constexpr uint64_t SCRATCH_KEEP = 256ull << 20;
-
 // Scratch pools by device and context (a cudaDeviceReset replaces the context
 // and ends its pools).  A context without an id, or one past the table's
 // limit, has none and allocates from the device's default pool.

@@ -22,6 +22,9 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // device's default pool returns its memory to the driver at the next
 // synchronisation, and mapping it again cost 0.4 ms to several ms a call.
 // While the stream is being captured the allocation is a plain graph node.
+// The largest scratch of one call at the sizes in use is 239 MB (the flop
+// matrices of 21 flops with all 1,326 combos); the flop-EV chain takes 134 MB.
+constexpr size_t SCRATCH_KEEP = 256ull << 20;
 int scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 template <typename T>
 inline int scratch_alloc(T** p, size_t count, cudaStream_t st) {

@@ -489,26 +489,41 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
     cudaStream_t st = as_stream(stream);
     const Lists L = make_lists(mode);
     const int ld = mode == MTT_PF_REFERENCE ? LD_REF : LD_OK;
-    // flops per pass: one CTA of k_pf_flop_eq per (villain tile, flop) and SM,
-    // as many flops as fit three waves (23 of the reference's 19 tiles, 217 MB)
+    // flops per pass: one CTA of k_pf_flop_eq per (villain tile, flop) and SM, as
+    // many flops as fit three waves and the scratch that is kept between calls
+    // (23 of the reference's 19 tiles, 223 MB), and fewer where the device has
+    // not that much left
     const int tiles = ceil_div(L.ncombo, EQ_VILL);
     int dev = 0, sms = 0;
     MTT_TRY_CUDA(cudaGetDevice(&dev));
     MTT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     MTT_TRY_CUDA(cudaFuncSetAttribute(k_pf_flop_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, EQ_SMEM));
-    const int chunk = std::max(1, std::min(n, std::min(3 * sms / tiles, 23)));
+    const size_t keys = (size_t)NPAIR * ld, runs = (size_t)L.ncombo * RUNS, eqs = (size_t)ld * ld;
+    const int fit = (int)(SCRATCH_KEEP / (sizeof(uint16_t) * keys + sizeof(uint32_t) * runs + sizeof(float) * eqs));
+    int chunk = std::max(1, std::min({n, 3 * sms / tiles, fit}));
     uint16_t* d_cc = nullptr;
     int *d_lists = nullptr, *d_counts = nullptr;
     uint16_t* d_KT = nullptr;
     uint32_t* d_HL = nullptr;
     float* d_E = nullptr;
+    auto drop = [st](auto*& p) {
+        if (p) cudaFreeAsync(p, st);
+        p = nullptr;
+    };
     int s = MTT_OK;
     if (!s) s = scratch_alloc(&d_cc, L.cc.size(), st);
     if (!s) s = scratch_alloc(&d_lists, L.lists.size(), st);
     if (!s) s = scratch_alloc(&d_counts, L.counts.size(), st);
-    if (!s) s = scratch_alloc(&d_KT, (size_t)chunk * NPAIR * ld, st);
-    if (!s) s = scratch_alloc(&d_HL, (size_t)chunk * L.ncombo * RUNS, st);
-    if (!s) s = scratch_alloc(&d_E, (size_t)chunk * ld * ld, st);
+    while (!s) {
+        s = scratch_alloc(&d_KT, chunk * keys, st);
+        if (!s) s = scratch_alloc(&d_HL, chunk * runs, st);
+        if (!s) s = scratch_alloc(&d_E, chunk * eqs, st);
+        if (s != MTT_ERR_NOMEM || chunk == 1) break;
+        cudaGetLastError();                    // the refusal is dealt with here
+        drop(d_KT); drop(d_HL); drop(d_E);
+        chunk = (chunk + 1) / 2;
+        s = MTT_OK;
+    }
     if (!s) s = cuda_status(cudaMemcpyAsync(d_cc, L.cc.data(), sizeof(uint16_t) * L.cc.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_lists, L.lists.data(), sizeof(int) * L.lists.size(), cudaMemcpyHostToDevice, st));
     if (!s) s = cuda_status(cudaMemcpyAsync(d_counts, L.counts.data(), sizeof(int) * L.counts.size(), cudaMemcpyHostToDevice, st));
@@ -521,8 +536,8 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
         k_pf_reduce<<<dim3(NC, nf), PAD, 0, st>>>(d_E, ld, d_lists, d_counts, d_out + (size_t)f0 * NC * NC);
         s = cuda_status(cudaGetLastError());
     }
-    cudaFreeAsync(d_cc, st); cudaFreeAsync(d_lists, st); cudaFreeAsync(d_counts, st);
-    cudaFreeAsync(d_KT, st); cudaFreeAsync(d_HL, st); cudaFreeAsync(d_E, st);
+    drop(d_cc); drop(d_lists); drop(d_counts);
+    drop(d_KT); drop(d_HL); drop(d_E);
     return s;
 }
 
