@@ -1067,8 +1067,10 @@ extern "C" int mtt_mw_batch_create(const mtt_mw_subgame* subs, int32_t n, mtt_mw
     // at all.  One 1,585-node subgame of 1,081 hands took 204.7 us an iteration
     // by levels (147.6 once zero regrets skip their divisions) and takes 72.5 by
     // tree: 272 CTAs, one wave, against 101 in slices of 8 hands; two subgames
-    // 231 / 144, four 376 / 286, eight (2,176 CTAs) 671 / 549.  Larger batches
-    // keep the level kernels, unmeasured.
+    // 231 / 144, four 376 / 286, eight (2,176 CTAs) 671 / 549.  Up to 16 CTAs an
+    // SM no batch was slower so than by levels (677 to 3,213 nodes, 40 to 1,081
+    // hands, 1 to 55 subgames: 1.06 to 2.9 times as fast, least where the CTAs
+    // are many and narrow); larger ones keep the level kernels, unmeasured.
     constexpr int TREE_BYTES = 224 * 1024;
     std::vector<TreeHost> part(NP * (size_t)n);
     std::atomic<bool> fits{true};

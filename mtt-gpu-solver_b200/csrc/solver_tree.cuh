@@ -70,7 +70,7 @@ __device__ __forceinline__ float dcfr1(float r, float inst, float dpos, float dn
 // alone: its counterfactual values come up the tree from its own terminals,
 // its regrets and strategy follow, and its reach goes down the tree again.  So
 // where a subgame deals no card and its tree is small enough, one CTA takes
-// one player's slice of 8 to 32 hands through the whole tree: it stages the
+// one player's slice of 4 to 32 hands through the whole tree: it stages the
 // slice's regret and strategy-sum rows, terminal values and reach in shared
 // memory (asynchronous 16-byte copies, all in flight at once), walks the
 // backward levels and then the forward levels of the new strategy there, with
