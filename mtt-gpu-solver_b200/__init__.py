@@ -329,9 +329,10 @@ class RiverBatch:
         """FP64 root values of subgame s from the last best-response pass:
         (ev0, ev1, br0, br1), each over that player's combos."""
         rows0, rows1, H0, H1 = self.meta[s]
-        out = [np.zeros(H0), np.zeros(H1), np.zeros(H0), np.zeros(H1)]
-        check("mtt_batch_root_values", lib().mtt_batch_root_values(self._h, s, *[o.ctypes.data for o in out]))
-        return tuple(out)
+        out = np.zeros(2 * (H0 + H1))          # the four parts of one array
+        at, p = (0, H0, H0 + H1, 2 * H0 + H1, 2 * (H0 + H1)), out.ctypes.data
+        check("mtt_batch_root_values", lib().mtt_batch_root_values(self._h, s, *[p + 8 * a for a in at[:4]]))
+        return tuple(out[a:z] for a, z in zip(at, at[1:]))
 
     def info(self):
         db = ctypes.c_int64()

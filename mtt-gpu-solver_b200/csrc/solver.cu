@@ -27,6 +27,7 @@
 #include <functional>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <mutex>
 #include <thread>
@@ -1747,7 +1748,6 @@ struct mtt_batch {
     double* d_darena = nullptr;
     double* d_results = nullptr;
     double* d_roots = nullptr;         // root values of the last best-response pass (SolveDev::roots)
-    double* h_roots = nullptr;         // pinned: one subgame's part of it, on its way to the caller
     int* d_iter = nullptr;
     int* d_err = nullptr;             // bounded-wait error word of the staged kernels
     float* d_iter_tab = nullptr;
@@ -1856,7 +1856,6 @@ static void free_batch(mtt_batch* b) {
     dfree(b->d_desc); dfree(b->d_nodes); dfree(b->d_tabs); dfree(b->d_hcards);
     dfree(b->d_ranges); dfree(b->d_arena); dfree(b->d_R); dfree(b->d_S);
     dfree(b->d_darena); dfree(b->d_results); dfree(b->d_roots); dfree(b->d_iter);
-    if (b->h_roots) cudaFreeHost(b->h_roots);
     dfree(b->d_iter_tab);
     dfree(b->d_err); dfree(b->d_tree);
     dfree(b->d_leaves); dfree(b->d_lx); dfree(b->d_ly); dfree(b->d_lm); dfree(b->d_lsd);
@@ -3030,10 +3029,11 @@ extern "C" int mtt_batch_root_values(mtt_batch* b, int32_t s, double* h_ev0, dou
     MTT_TRY_CUDA(cudaDeviceSynchronize());
     const SubDesc& d = b->desc[s];
     const size_t HS = (size_t)d.Hp0 + d.Hp1;
-    if (!b->h_roots) MTT_TRY_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&b->h_roots), sizeof(double) * 4 * (size_t)b->max_h,
-                                                cudaHostAllocDefault));
-    MTT_TRY_CUDA(cudaMemcpy(b->h_roots, b->d_roots + 2 * d.range_base, sizeof(double) * 2 * HS, cudaMemcpyDeviceToHost));
-    const double* v = b->h_roots;
+    // not page-locked: freeing such a buffer with the batch would wait for all
+    // other work of the device
+    std::unique_ptr<double[]> root(new double[2 * HS]);
+    MTT_TRY_CUDA(cudaMemcpy(root.get(), b->d_roots + 2 * d.range_base, sizeof(double) * 2 * HS, cudaMemcpyDeviceToHost));
+    const double* v = root.get();
     if (h_ev0) std::memcpy(h_ev0, v, sizeof(double) * d.H0);
     if (h_ev1) std::memcpy(h_ev1, v + d.Hp0, sizeof(double) * d.H1);
     if (h_br0) std::memcpy(h_br0, v + HS, sizeof(double) * d.H0);
