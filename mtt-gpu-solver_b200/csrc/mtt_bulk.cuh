@@ -59,6 +59,12 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// Asynchronous copy of 16 bytes to shared memory; both addresses are multiples
+// of 16.
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
 // Programmatic dependent launch.  A kernel launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization may start while the
 // previous kernel on the stream drains; grid_dep_wait returns once that

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(AI_THREADS) k_pf_allin(float* __restrict__ out
         ties += sh == sv;
     }
     if (SPLIT > 1) {
-        const unsigned mask = (SPLIT == 32 ? 0xFFFFFFFFu : ((1u << SPLIT) - 1u)) << ((tid & 31) / SPLIT * SPLIT);
+        const unsigned mask = ((1u << SPLIT) - 1u) << ((tid & 31) / SPLIT * SPLIT);
 #pragma unroll
         for (int o = SPLIT / 2; o > 0; o >>= 1) {
             wins += __shfl_down_sync(mask, wins, o, SPLIT);
@@ -614,11 +614,8 @@ __global__ void k_pf_init(PfDev d) {
 // the loads left in the chains.  The five launches before (thread per flop
 // over one class's strided column, all classes' sums in one CTA) took 80 us.
 
-// Asynchronous copies of 16 and 4 bytes to shared memory; copies_done waits
-// for this thread's copies (a barrier must follow).
-__device__ __forceinline__ void copy16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
+// Asynchronous copy of 4 bytes to shared memory; copies_done waits for this
+// thread's copies, of 16 bytes too (a barrier must follow).
 __device__ __forceinline__ void copy4(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
@@ -634,7 +631,7 @@ __global__ void __launch_bounds__(2 * PAD) k_pf_cosolve(PfDev d) {
     __shared__ float rsum[2];
     const int f = blockIdx.x, tid = threadIdx.x;
     const int side = tid / PAD, cls = tid % PAD;   // side 0: BTN's EV, 1: BB's
-    for (int i = tid; i < MAT / 4; i += 2 * PAD) copy16(eqm + 4 * i, d.mats + (size_t)f * MAT + 4 * i);
+    for (int i = tid; i < MAT / 4; i += 2 * PAD) copy_async16(eqm + 4 * i, d.mats + (size_t)f * MAT + 4 * i);
     grid_dep_wait();
     grid_dep_trigger();
     if (cls < NC)                             // side 0 sums over BB's reach, side 1 over BTN's
@@ -692,7 +689,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pf_step(PfDev d, float wp, flo
     const int cls = blockIdx.x * STEP_CLS + lane;
     const int col = min(cls, NC - 1);
     for (int i = tid; i < STEP_JAM / 4; i += STEP_THREADS)
-        copy16(step_smem + 4 * i, d.jam + (size_t)blockIdx.x * STEP_JAM + 4 * i);
+        copy_async16(step_smem + 4 * i, d.jam + (size_t)blockIdx.x * STEP_JAM + 4 * i);
     auto stage_flops = [&](int f0) {                         // flops [f0, f0 + STEP_FLOPS)
         const int n = min(STEP_FLOPS, d.nf - f0);
         for (int k = warp; k < n; k += STEP_WARPS) {
@@ -703,8 +700,8 @@ __global__ void __launch_bounds__(STEP_THREADS) k_pf_step(PfDev d, float wp, flo
     };
     grid_dep_wait();
     grid_dep_trigger();
-    for (int i = tid; i < STATE / 4; i += STEP_THREADS) copy16(G + 4 * i, d.G + 4 * i);
-    for (int i = tid; i < PAD / 4; i += STEP_THREADS) copy16(root + 4 * i, d.root + 4 * i);
+    for (int i = tid; i < STATE / 4; i += STEP_THREADS) copy_async16(G + 4 * i, d.G + 4 * i);
+    for (int i = tid; i < PAD / 4; i += STEP_THREADS) copy_async16(root + 4 * i, d.root + 4 * i);
     stage_flops(0);
     float Rc[3] = {0.0f, 0.0f, 0.0f}, Sc[3] = {0.0f, 0.0f, 0.0f};   // the updated node's rows of this class
     if (warp < 4 && cls < NC)

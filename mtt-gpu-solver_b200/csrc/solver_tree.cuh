@@ -141,9 +141,6 @@ template <int ALGO>
 __device__ __forceinline__ float4 upd_sum(float4 sv, float4 r, float4 wr, float4 sg, float dstr) {
     return ALGO == MTT_ALGO_DCFR ? fma4(r, sg, mul4(sv, f4(dstr))) : fma4(wr, sg, sv);
 }
-__device__ __forceinline__ void copy_async16(float4* dst, const float4* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
 
 // One node of one hand group, its rows and child values G float4 apart in
 // shared memory: the acting player's update (returns the node's value) and the
