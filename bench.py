@@ -602,8 +602,9 @@ def run_b200(args, rank, world, local):
                             "max_expl_pct_pot": float(np.max(fixed_expl) * 100)},
             "evals_per_s": evals_per_s,
             "plain_kernel": {"value": plain_value, "unit": "solves/s", "ms": plain_ms,
-                             "sample": f"{n_plain} subgames solved one at a time (same parameters and gate), level "
-                                       f"launches, no graph; CUDA events around the solves, inputs resident"},
+                             "sample": f"{n_plain} subgames solved one at a time (same parameters and gate), the "
+                                       f"library's launches for one subgame (a terminal and a whole-tree launch a "
+                                       f"player), no graph; CUDA events around the solves, inputs resident"},
             "vs_plain": value / plain_value,
             "reference_kernels": ref_kernels,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",

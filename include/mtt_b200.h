@@ -339,6 +339,9 @@ int mtt_batch_set_leafnet(mtt_batch* b, mtt_leafnet* net, int32_t flags);
  * h_ms[3] = device time and h_bytes[3] = compulsory bytes (every element a
  * work item reads or writes, counted once) of {forward sweeps, terminal
  * launches, backward sweeps}.  Restarts the batch's solve state.  Blocks.
+ * Batches whose solve sweeps whole trees in one launch run its forward and
+ * its backward part apart here, so their two figures add up to more than the
+ * launch of a solve.
  * No reference counterpart (instrumentation). */
 int mtt_batch_kernel_profile(mtt_batch* b, const mtt_solve_params* prm, int32_t iters, double* h_ms,
                              double* h_bytes, void* stream);

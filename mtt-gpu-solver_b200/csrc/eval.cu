@@ -28,7 +28,7 @@ constexpr int EV_THREADS = 256;
 constexpr long long EV_QUAD_MIN = 4096;      // below this, a thread per hand: the shorter chain wins (1.9 us)
 
 // Four hands a thread, read as seven aligned words.  Bound by the integer pipe
-// (ALU 92% busy, 173 instructions a hand): the suits are only counted (a byte each, in one word), so a
+// (ALU 91% busy, 162 issue slots a hand): the suits are only counted (a byte each, in one word), so a
 // hand costs its rank planes, the count and the scores without a flush; one
 // hand in 33 holds a flush, and those are read again and scored after all
 // four, when most warps have one pass of them left instead of up to four.
