@@ -326,14 +326,17 @@ k_board_counts(const uint32_t* __restrict__ keys, int ncw, int H, int Hp,
 // index r1 = 0,2,..,46 into the 49-card deck, river index r2 = r1+1, r1+4,
 // .. < 47.  192 (r1, r2) pairs, packed two per key word.
 constexpr int FE_RUNOUTS = 192, FE_WORDS = 96, FE_ALIVE = 1176, FE_VILL = 294;
-__constant__ uint8_t c_runout_r1[FE_RUNOUTS];
-__constant__ uint8_t c_runout_r2[FE_RUNOUTS];
-
-static void host_runouts(uint8_t* r1s, uint8_t* r2s) {
+struct Runouts { uint8_t r1[FE_RUNOUTS], r2[FE_RUNOUTS]; };
+constexpr Runouts make_runouts() {
+    Runouts t{};
     int k = 0;
     for (int r1 = 0; r1 < 47; r1 += 2)
-        for (int r2 = r1 + 1; r2 < 47; r2 += 3) { r1s[k] = (uint8_t)r1; r2s[k] = (uint8_t)r2; ++k; }
+        for (int r2 = r1 + 1; r2 < 47; r2 += 3) { t.r1[k] = (uint8_t)r1; t.r2[k] = (uint8_t)r2; ++k; }
+    return t;
 }
+// Part of the module: copied in by each call, a captured call's replay read the
+// copy's source when it was gone, and indexed the deck with what was there.
+__constant__ Runouts c_runouts = make_runouts();
 
 __device__ __forceinline__ void flop_deck(const uint8_t* f, uint8_t* deck) {
     const uint64_t fm = (1ull << f[0]) | (1ull << f[1]) | (1ull << f[2]);
@@ -363,7 +366,7 @@ k_flop_keys(const uint8_t* __restrict__ flops, uint32_t* __restrict__ keys) {
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int k = 2 * w + half;
-            const int t = deck[c_runout_r1[k]], r = deck[c_runout_r2[k]];
+            const int t = deck[c_runouts.r1[k]], r = deck[c_runouts.r2[k]];
             if (t == hc1 || t == hc2 || r == hc1 || r == hc2) continue;
             Planes p = base;
             planes_add(p, t); planes_add(p, r);
@@ -538,19 +541,10 @@ __global__ void k_dump_aggregate(const uint8_t* __restrict__ flops, const float*
     out[idx] = acc;
 }
 
-static int upload_runouts(cudaStream_t st) {
-    uint8_t r1[FE_RUNOUTS], r2[FE_RUNOUTS];
-    host_runouts(r1, r2);
-    MTT_TRY_CUDA(cudaMemcpyToSymbolAsync(c_runout_r1, r1, sizeof(r1), 0, cudaMemcpyHostToDevice, st));
-    MTT_TRY_CUDA(cudaMemcpyToSymbolAsync(c_runout_r2, r2, sizeof(r2), 0, cudaMemcpyHostToDevice, st));
-    return MTT_OK;
-}
-
 constexpr int FE_BATCH = 64;    // flops per scratch batch: keys and equities (117 MB) stay in the 126 MB L2
 
 static int flop_ev_batched(const uint8_t* d_flops, int nflops, const float* d_reach0,
                            const float* d_reach1, float* d_ev0, float* d_ev1, cudaStream_t st) {
-    MTT_TRY(upload_runouts(st));
     const int nb = nflops < FE_BATCH ? nflops : FE_BATCH;
     uint32_t* keys = nullptr;
     float* eqT = nullptr;
