@@ -89,7 +89,7 @@ __host__ __device__ inline void class_cards_avoid(int cls, uint64_t dead, int& c
 }
 
 // combo -> class (host set-up, :475-483).
-__host__ __device__ inline int combo_class(int c1, int c2) {
+__host__ __device__ constexpr int combo_class(int c1, int c2) {
     const int r1 = c1 / 4, s1 = c1 % 4, r2 = c2 / 4, s2 = c2 % 4;
     const int hi = r1 > r2 ? r1 : r2, lo = r1 < r2 ? r1 : r2;
     if (r1 == r2) return 12 - hi;
@@ -439,32 +439,30 @@ __global__ void k_pf_reduce(const float* __restrict__ E, int ld, const int* __re
     out[((size_t)f * NC + vcl) * NC + hcl] = valid > 0 ? __fdiv_rn(sum, (float)valid) : 0.5f;
 }
 
-// Host lists: combos of the matrix (reference: the first 1,176 in
-// lexicographic order; correct: all 1,326, those touching a flop are zeroed
-// per flop by the kernels) and up to `cap` combos per class.
+// Combos of the matrix (reference: the first 1,176 in lexicographic order;
+// correct: all 1,326, those touching a flop are zeroed per flop by the kernels)
+// and up to CLS_CAP combos per class.  Part of the module: copied in by each
+// call, a captured call's replay read the copy's source when it was gone.
+constexpr int CLS_CAP = 12;              // the largest class (offsuit) has 12 combos
 struct Lists {
-    std::vector<uint16_t> cc;     // 2 per combo
-    std::vector<int> lists, counts;
-    int ncombo = 0;
+    uint16_t cc[2 * 1326];               // 2 per combo
+    int lists[NC * CLS_CAP], counts[NC];
+    int ncombo;
 };
-
-static Lists make_lists(int mode) {
-    Lists L;
-    const int limit = mode == MTT_PF_REFERENCE ? ALIVE : 1326;
-    const int cap = 12;                  // the largest class (offsuit) has 12 combos
-    L.lists.assign(NC * 12, 0);
-    L.counts.assign(NC, 0);
+constexpr Lists make_lists(int limit) {
+    Lists L{};
     for (int c1 = 0; c1 < 52; ++c1)
         for (int c2 = c1 + 1; c2 < 52; ++c2) {
             if (L.ncombo >= limit) continue;
             const int cls = combo_class(c1, c2);
-            L.cc.push_back((uint16_t)c1);
-            L.cc.push_back((uint16_t)c2);
-            if (L.counts[cls] < cap) L.lists[cls * 12 + L.counts[cls]++] = L.ncombo;
+            L.cc[2 * L.ncombo] = (uint16_t)c1;
+            L.cc[2 * L.ncombo + 1] = (uint16_t)c2;
+            if (L.counts[cls] < CLS_CAP) L.lists[cls * CLS_CAP + L.counts[cls]++] = L.ncombo;
             ++L.ncombo;
         }
     return L;
 }
+__device__ const Lists g_lists_ref = make_lists(ALIVE), g_lists_ok = make_lists(1326);
 
 }  // namespace pf
 }  // namespace mtt
@@ -487,22 +485,23 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
     if (!d_flops || !d_out || n < 0 || (mode != MTT_PF_REFERENCE && mode != MTT_PF_CORRECT)) return MTT_ERR_INVALID;
     if (n == 0) return MTT_OK;
     cudaStream_t st = as_stream(stream);
-    const Lists L = make_lists(mode);
-    const int ld = mode == MTT_PF_REFERENCE ? LD_REF : LD_OK;
+    const bool ref = mode == MTT_PF_REFERENCE;
+    const int ncombo = ref ? ALIVE : 1326, ld = ref ? LD_REF : LD_OK;
+    void* sym = nullptr;
+    MTT_TRY_CUDA(ref ? cudaGetSymbolAddress(&sym, g_lists_ref) : cudaGetSymbolAddress(&sym, g_lists_ok));
+    const Lists* L = static_cast<const Lists*>(sym);     // on the device
     // flops per pass: one CTA of k_pf_flop_eq per (villain tile, flop) and SM, as
     // many flops as fit three waves and the scratch that is kept between calls
     // (23 of the reference's 19 tiles, 223 MB), and fewer where the device has
     // not that much left
-    const int tiles = ceil_div(L.ncombo, EQ_VILL);
+    const int tiles = ceil_div(ncombo, EQ_VILL);
     int dev = 0, sms = 0;
     MTT_TRY_CUDA(cudaGetDevice(&dev));
     MTT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     MTT_TRY_CUDA(cudaFuncSetAttribute(k_pf_flop_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, EQ_SMEM));
-    const size_t keys = (size_t)NPAIR * ld, runs = (size_t)L.ncombo * RUNS, eqs = (size_t)ld * ld;
+    const size_t keys = (size_t)NPAIR * ld, runs = (size_t)ncombo * RUNS, eqs = (size_t)ld * ld;
     const int fit = (int)(SCRATCH_KEEP / (sizeof(uint16_t) * keys + sizeof(uint32_t) * runs + sizeof(float) * eqs));
     int chunk = std::max(1, std::min({n, 3 * sms / tiles, fit}));
-    uint16_t* d_cc = nullptr;
-    int *d_lists = nullptr, *d_counts = nullptr;
     uint16_t* d_KT = nullptr;
     uint32_t* d_HL = nullptr;
     float* d_E = nullptr;
@@ -511,9 +510,6 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
         p = nullptr;
     };
     int s = MTT_OK;
-    if (!s) s = scratch_alloc(&d_cc, L.cc.size(), st);
-    if (!s) s = scratch_alloc(&d_lists, L.lists.size(), st);
-    if (!s) s = scratch_alloc(&d_counts, L.counts.size(), st);
     while (!s) {
         s = scratch_alloc(&d_KT, chunk * keys, st);
         if (!s) s = scratch_alloc(&d_HL, chunk * runs, st);
@@ -524,19 +520,15 @@ extern "C" int mtt_pf_flop_class_matrices(int32_t mode, const uint8_t* d_flops, 
         chunk = (chunk + 1) / 2;
         s = MTT_OK;
     }
-    if (!s) s = cuda_status(cudaMemcpyAsync(d_cc, L.cc.data(), sizeof(uint16_t) * L.cc.size(), cudaMemcpyHostToDevice, st));
-    if (!s) s = cuda_status(cudaMemcpyAsync(d_lists, L.lists.data(), sizeof(int) * L.lists.size(), cudaMemcpyHostToDevice, st));
-    if (!s) s = cuda_status(cudaMemcpyAsync(d_counts, L.counts.data(), sizeof(int) * L.counts.size(), cudaMemcpyHostToDevice, st));
     for (int f0 = 0; f0 < n && !s; f0 += chunk) {
         const int nf = std::min(chunk, n - f0);
         const uint8_t* fl = d_flops + 3 * (size_t)f0;
-        k_pf_keys<<<dim3(NPAIR, nf), 256, 0, st>>>(fl, d_cc, L.ncombo, ld, d_KT);
-        k_pf_runs<<<dim3(L.ncombo, nf), RUNS, 0, st>>>(fl, d_cc, L.ncombo, ld, d_KT, d_HL);
-        k_pf_flop_eq<<<dim3(tiles, nf), EQ_THREADS, EQ_SMEM, st>>>(fl, d_cc, L.ncombo, ld, mode, d_KT, d_HL, d_E);
-        k_pf_reduce<<<dim3(NC, nf), PAD, 0, st>>>(d_E, ld, d_lists, d_counts, d_out + (size_t)f0 * NC * NC);
+        k_pf_keys<<<dim3(NPAIR, nf), 256, 0, st>>>(fl, L->cc, ncombo, ld, d_KT);
+        k_pf_runs<<<dim3(ncombo, nf), RUNS, 0, st>>>(fl, L->cc, ncombo, ld, d_KT, d_HL);
+        k_pf_flop_eq<<<dim3(tiles, nf), EQ_THREADS, EQ_SMEM, st>>>(fl, L->cc, ncombo, ld, mode, d_KT, d_HL, d_E);
+        k_pf_reduce<<<dim3(NC, nf), PAD, 0, st>>>(d_E, ld, L->lists, L->counts, d_out + (size_t)f0 * NC * NC);
         s = cuda_status(cudaGetLastError());
     }
-    drop(d_cc); drop(d_lists); drop(d_counts);
     drop(d_KT); drop(d_HL); drop(d_E);
     return s;
 }
