@@ -6,6 +6,7 @@
 #include <climits>
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -385,7 +386,10 @@ inline void on_threads(int n, long long ns, Fn fn) {
     std::atomic<int> next{0};
     auto run = [&]() { for (int i; (i = next.fetch_add(1)) < n;) fn(i); };
     std::vector<std::thread> th;
-    for (int t = 1; t < nt; ++t) th.emplace_back(run);
+    try {
+        for (int t = 1; t < nt; ++t) th.emplace_back(run);
+    } catch (const std::system_error&) {       // no more threads to be had: those there are share the work
+    }
     run();
     for (std::thread& x : th) x.join();
 }
