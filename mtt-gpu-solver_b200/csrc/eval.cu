@@ -34,7 +34,7 @@ constexpr long long EV_QUAD_MIN = 4096;      // below this, a thread per hand: t
 // four, when most warps have one pass of them left instead of up to four.
 // 30,000,001 hands took 275 us with every suit's mask kept, tested by four
 // popcounts, and staged by bulk copies whose error word the call then read
-// back; 230 us now, and the call no longer waits.
+// back; 217 us now, and the call no longer waits.
 template <bool VEC>
 __global__ void __launch_bounds__(EV_THREADS)
 k_eval7_quad(const uint8_t* __restrict__ cards, uint32_t* __restrict__ out, long long n) {

@@ -1628,7 +1628,7 @@ __global__ void __launch_bounds__(TT) k_br_final(SolveDev a, const int* __restri
     cta_terminal<double, double, double>(term_info(sd, z), tv, 0, reach + OFF(1), zm, nullptr, X, wb,
                                          MTT_SEM_CORRECT, tid);
     // the root values side by side, so that one copy fetches a subgame's four
-    // vectors (23 us a subgame on a 1,024-subgame batch; four copies out of the
+    // vectors (24 us a subgame on a 1,024-subgame batch; four copies out of the
     // arena's regions took 33 us more)
     double* root = a.roots + 2 * sd.range_base;
     for (int h = tid; h < HS; h += TT) {
